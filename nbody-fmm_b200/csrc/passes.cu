@@ -192,7 +192,9 @@ __global__ void __launch_bounds__(CT_THREADS) k_contract(ContractArgs a) {
     cp_async_commit();
   };
 
-  if (NS == 2) prefetch(0, 0);
+  // a batch may have no source at all (the lists keep a cell whose only large pairs are with its neighbours): then
+  // its slot list is empty and holds nothing to read
+  if (NS == 2 && nslots > 0) prefetch(0, 0);
   for (int s = 0; s < nslots; ++s) {
     const int buf = NS == 2 ? (s & 1) : 0;
     if (NS == 1) {

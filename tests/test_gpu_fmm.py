@@ -301,3 +301,23 @@ def test_elongated_box_converges_and_matches_oracle(oracle):
             assert rel_l2(a, oracle.fmm(pos, m, p, 64)) < 1e-6
         errs.append(rel_l2(a, ref))
     assert errs[1] < errs[0] < 2e-5
+
+
+@pytest.mark.parametrize("p", [4, 8, 12])
+def test_m2l_batch_without_sources(oracle, p):
+    """A clump around the box centre: on every level its eight cells, one per
+    class, are large enough for M2L only with each other, and they touch, so
+    each (level, class) batch of the FP32 contraction has no source at all.
+    The workspace starts from device memory holding large integers, which the
+    empty slot lists must not be read from."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(7)
+    pos = np.concatenate([rng.random((60, 3)), 0.5 + 1e-3 * (rng.random((1600, 3)) - 0.5), [[0, 0, 0], [1, 1, 1]]])
+    mass = np.full(len(pos), 1.0 / len(pos))
+    dirty = torch.full((1 << 28,), 0x7F7F7F7F, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    del dirty
+    torch.cuda.empty_cache()
+    with fmmgpu.Context(dim=3, p=p, leaf_cap=64, direct_max=262) as c:
+        acc = c.evaluate(pos, mass)
+    assert rel_l2(acc, oracle.fmm(pos, mass, p, 64, direct_max=262)) < 1e-6
