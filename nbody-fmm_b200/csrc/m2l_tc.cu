@@ -22,13 +22,27 @@
 // split products smallest first; R += D is done by the threads in FP32
 // (round to nearest), which keeps the contraction at FP32 accuracy.
 //
-// Pipeline.  Thread 0 issues the MMAs.  The operator's BF16 images stream
-// through two shared-memory buffers by bulk asynchronous copies completing on
-// mbarriers (one split, or one split's half of the output columns when
-// P16 > 128, per copy), so the copy of the next image overlaps the MMAs of
-// the current one.  The threads prefetch the next slot's source rows into
+// Pipeline.  Eight worker warps form the A operand and add D to R, one warp
+// issues the MMAs, and one streams the operator's BF16 images through four
+// shared-memory buffers by bulk asynchronous copies completing on mbarriers
+// (part of one split's K rows per copy), so that copies run up to three ahead
+// of the MMAs.  The workers prefetch the next slot's source rows into
 // registers while the MMAs run, then split them into the A operand once the
 // MMAs have released it.
+//
+// What bounds it: at width 176 the tensor pipe (66 MMAs of N = 176, about
+// 5.8 K cycles) and, in series with it, forming A and adding D (3.5 K), about
+// 10 K cycles per slot; below that the smaller MMAs are held by their shared-
+// memory reads.  Why this split: with one thread of four worker warps issuing
+// the MMAs between its own loads a 176-wide slot took 28 K cycles, 18 K of
+// them in the issue (134 cycles per MMA, the descriptor arithmetic of a loop
+// that was not unrolled) and 4.8 K in forming A and adding D.  Hence an
+// issuing thread of its own with descriptors advanced by constants, one MMA
+// over all columns (N = w) instead of two halves (A is read once), a copying
+// warp and eight warps for the conversions: the M2L phase of the 16M mixture
+// at p = 12 with learned orders went from 35.0 to 15.8 ms.  Tried and not
+// kept: writing the second and third splits of A while the last product runs
+// (17.0 ms: the stores and the MMAs share the shared-memory bandwidth).
 //
 // Shared-memory operands use the K-major layout without swizzle: 8-row x
 // 16-byte core matrices, rows of a core matrix contiguous, 8-row groups
@@ -57,19 +71,8 @@ __device__ inline uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) 
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-__device__ inline void split3(float v, uint16_t &h, uint16_t &m, uint16_t &l) {
-  const __nv_bfloat16 bh = __float2bfloat16_rn(v);
-  const float r1 = v - __bfloat162float(bh);
-  const __nv_bfloat16 bm = __float2bfloat16_rn(r1);
-  const float r2 = r1 - __bfloat162float(bm);
-  const __nv_bfloat16 bl = __float2bfloat16_rn(r2);
-  h = __bfloat16_as_ushort(bh);
-  m = __bfloat16_as_ushort(bm);
-  l = __bfloat16_as_ushort(bl);
-}
-
-// split3 of two values at once; each 32-bit word holds (a, b) as BF16 with
-// a in the low half.
+// The three-part split of two values at once (round to nearest); each 32-bit
+// word holds (a, b) as BF16 with a in the low half.
 __device__ inline uint32_t bf2_pack(float a, float b) {
   const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t *>(&t);
@@ -83,25 +86,29 @@ __device__ inline void split3x2(float a, float b, uint32_t &h, uint32_t &m, uint
 }
 
 // Operator images: for each table slot and split s, B = T^T (n: output,
-// k: input) cut into output tiles of N0 and P16 - N0 columns, each tile
-// contiguous; element (n, k) of a tile of width nw at
-// ((k/8) * (nw/8) + n/8) * 64 + (n%8) * 8 + k%8.
-__global__ void k_tc_images(const float *tab, int K, int KP, int P16, int N0, uint16_t *img) {
+// k: input), its first W rows and columns; element (n, k) at
+// ((k/8) * (W/8) + n/8) * 64 + (n%8) * 8 + k%8, so that the first w rows (k)
+// are a contiguous prefix.  A thread takes 8 consecutive k of one n: reads
+// coalesced over n, 16-byte stores.
+__global__ void k_tc_images(const float *tab, int K, int KP, int W, uint16_t *img) {
   const int slot = blockIdx.x;
-  const size_t bsplit = (size_t)P16 * P16;
+  const size_t bsplit = (size_t)W * W;
   const float *T = tab + (size_t)slot * K * KP;
   uint16_t *out = img + (size_t)slot * 3 * bsplit;
-  for (int e = threadIdx.x; e < P16 * P16; e += blockDim.x) {
-    const int n = e / P16, k = e % P16;
-    const float v = (n < K && k < K) ? T[(size_t)k * KP + n] : 0.f;
-    uint16_t h, m, l;
-    split3(v, h, m, l);
-    const int j = n >= N0 ? 1 : 0;
-    const int nl = n - j * N0, nw = j ? P16 - N0 : N0;
-    const size_t idx = (j ? (size_t)P16 * N0 : 0) + ((size_t)(k / 8) * (nw / 8) + nl / 8) * 64 + (nl % 8) * 8 + (k % 8);
-    out[idx] = h;
-    out[bsplit + idx] = m;
-    out[2 * bsplit + idx] = l;
+  for (int e = threadIdx.x; e < W * (W / 8); e += blockDim.x) {
+    const int n = e % W, k0 = (e / W) * 8;
+    uint32_t h[4], m[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = k0 + 2 * q;
+      const float v0 = (n < K && k < K) ? T[(size_t)k * KP + n] : 0.f;
+      const float v1 = (n < K && k + 1 < K) ? T[(size_t)(k + 1) * KP + n] : 0.f;
+      split3x2(v0, v1, h[q], m[q], l[q]);
+    }
+    const size_t idx = ((size_t)(k0 / 8) * (W / 8) + n / 8) * 64 + (n % 8) * 8;
+    *(uint4 *)(out + idx) = make_uint4(h[0], h[1], h[2], h[3]);
+    *(uint4 *)(out + bsplit + idx) = make_uint4(m[0], m[1], m[2], m[3]);
+    *(uint4 *)(out + 2 * bsplit + idx) = make_uint4(l[0], l[1], l[2], l[3]);
   }
 }
 
@@ -110,23 +117,28 @@ __device__ inline void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
 
+// Whether the phase with the given parity has completed (waits a little).
+__device__ inline bool mbar_try(uint32_t addr, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}"
+      : "=r"(done)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
 // Waits for the completion of the phase with the given parity; false after
 // about 2^31 clocks (about a second).
 __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);
+  if (mbar_try(addr, parity)) return true;
   const long long t0 = clock64();
-  while (true) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P1;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (done) return true;
+  while (!mbar_try(addr, parity))
     if (clock64() - t0 > (1ll << 31)) return false;
-  }
+  return true;
 }
 
 // Bulk copy global -> shared completing on an mbarrier (no multicast).
@@ -148,9 +160,20 @@ __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
       "{\n\t"
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(tmem_d),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+}
+
+// One lane of a converged warp.
+__device__ inline bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 __device__ inline void mma_commit(uint64_t *bar) {
@@ -184,39 +207,59 @@ __device__ inline void tc_fence_after() { asm volatile("tcgen05.fence::after_thr
 // their slots as one stream, so the operator copies and the source-row
 // prefetch of the next batch overlap the MMAs of the current one.  Batch
 // metadata is double-buffered in shared memory (current, next).
+//
+// Barriers: s_a (the workers have written A and read D), s_full / s_mma (an
+// operator copy has landed in a buffer / its MMAs are done), s_done (the
+// slot's MMAs are done).  A wait that gives up makes its thread skip the rest of the
+// batch; all threads meet at the batch's end and leave together.
+static constexpr int TC_WORKERS = 256, TC_THREADS = TC_WORKERS + 64, TC_NBUF = 4;
+
+// CTAs per SM: two where shared memory and TMEM (512 columns) hold them, at
+// 96 registers a thread.  (Three of the narrow kernels' at 64 registers
+// spilled: 1.26 against 1.10 ms for the 48-wide M2L of a 4M 2D pass.)
+__host__ __device__ constexpr int tc_per_sm(int P16) { return P16 <= 96 ? 2 : 1; }
+
 template <int P16>
-__global__ void __launch_bounds__(TC_M, 1) k_tc_translate(TcArgs a, int nb, unsigned int *work) {
-  constexpr int NT = P16 > 128 ? 2 : 1;  // output tiles
-  constexpr int N0 = tc_n0(P16);
-  constexpr int N1 = P16 - N0;
+__global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcArgs a, int nb, unsigned int *work) {
+  constexpr int KH = tc_kpart(P16);  // K rows per operator copy
   constexpr int KC = P16 / 8;       // 16-byte K chunks
   constexpr int ASPLIT = TC_M * P16;
-  constexpr int BTILE = P16 * N0;
-  constexpr int TILES = 3 * NT;  // operator copies per slot
-  constexpr uint32_t NCOLS = P16 <= 128 ? 256u : 512u;
+  constexpr int BTILE = KH * P16;
+  constexpr uint32_t NCOLS = P16 <= 64 ? 128u : P16 <= 128 ? 256u : 512u;
   constexpr uint32_t RCOL = NCOLS / 2;  // running sum R; D at column 0
-  constexpr uint32_t LBO_A = (TC_M / 8) * 128;
+  constexpr uint32_t LBO_A = (TC_M / 8) * 128, LBO_B = (P16 / 8) * 128;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint16_t *As = (uint16_t *)smem;  // 3 splits
-  uint16_t *Bs = As + 3 * ASPLIT;   // 2 buffers
-  __shared__ __align__(8) uint64_t s_full[2], s_mma[2], s_done;
+  uint16_t *Bs = As + 3 * ASPLIT;   // TC_NBUF buffers
+  __shared__ __align__(8) uint64_t s_full[TC_NBUF], s_mma[TC_NBUF], s_a, s_done;
   __shared__ uint32_t s_tmem;
   __shared__ short s_slot[2][TC_MAX_SLOTS], s_op[2][TC_MAX_SLOTS];  // 16-bit: two 96-wide CTAs fit an SM
   __shared__ uint8_t s_w[2][TC_MAX_SLOTS];  // padded width of each slot's order
   __shared__ int s_n[2], s_b[2];
   __shared__ int s_grab;
 
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // a worker reads D and R at TMEM lane `trow` (a warp reaches the 32 lanes of
+  // its index mod 4; warps 0-3 take the even 16-column groups, 4-7 the odd
+  // ones) and gathers for A the 16 rows from 16 warp, as rows `grow`
+  const int trow = (warp & 3) * 32 + lane, grow = (warp & 7) * 16 + (lane & 15);
 
   // Takes the next work item with at least one slot into metadata buffer
-  // `buf` (s_n[buf] = 0 when the work is exhausted); returns this thread's
-  // target.  An item is a batch, or for M2L a run of up to chunk_slots of
-  // its present slots (item = batch * chunks + run).
+  // `buf` (s_n[buf] = 0 when the work is exhausted) and sets this thread's
+  // targets (rows trow and grow).  An item is a batch, or for M2L a run of up
+  // to chunk_slots of its present slots (item = batch * chunks + run).
   const int chunks = a.mode == TC_M2L ? (TC_MAX_SLOTS + a.chunk_slots - 1) / a.chunk_slots : 1;
-  auto load_meta = [&](int buf) -> int {
+  // Thread 0 draws the item after the one it hands out, so that nobody waits
+  // for the counter.
+  int drawn = tid == 0 ? (int)atomicAdd(work, 1u) : 0;
+  auto load_meta = [&](int buf, int &tg, int &tgg) {
+    tg = tgg = -1;
     while (true) {
-      if (tid == 0) s_grab = (int)atomicAdd(work, 1u);
+      if (tid == 0) {
+        s_grab = drawn;
+        if (drawn < nb * chunks) drawn = (int)atomicAdd(work, 1u);
+      }
       __syncthreads();
       const int item = s_grab;
       if (item >= nb * chunks) {
@@ -225,16 +268,15 @@ __global__ void __launch_bounds__(TC_M, 1) k_tc_translate(TcArgs a, int nb, unsi
           s_b[buf] = -1;
         }
         __syncthreads();
-        return -1;
+        return;
       }
       const int b = item / chunks, s0 = (item % chunks) * a.chunk_slots;
       const int4 bt = a.batches[b];
-      const int tg = tid < bt.y ? (a.tlist ? a.tlist[bt.x + tid] : bt.x + tid) : -1;
       int n = 0;
       if (a.mode == TC_M2L) {
         n = max(0, min(a.chunk_slots, a.nslots[b] - s0));
         const size_t tb = (size_t)b * TC_MAX_SLOTS + s0;
-        for (int i = tid; i < n; i += TC_M) {
+        for (int i = tid; i < n; i += TC_THREADS) {
           s_slot[buf][i] = (short)a.slot_list[tb + i];
           s_op[buf][i] = (short)a.tslot_list[tb + i];
           s_w[buf][i] = a.slot_p16 ? a.slot_p16[tb + i] : (uint8_t)P16;
@@ -247,36 +289,42 @@ __global__ void __launch_bounds__(TC_M, 1) k_tc_translate(TcArgs a, int nb, unsi
         }
         n = bt.y > 0 ? 1 : 0;
       }
+      if (n) {
+        if (trow < bt.y) tg = a.tlist ? a.tlist[bt.x + trow] : bt.x + trow;
+        if (grow < bt.y) tgg = a.tlist ? a.tlist[bt.x + grow] : bt.x + grow;
+      }
       if (tid == 0) {
         s_n[buf] = n;
         s_b[buf] = b;
-        if (n && a.mode == TC_M2L && a.tiles) atomicAdd(a.tiles, (unsigned long long)n);
-        if (n && a.mode == TC_M2L && a.widths) {
-          unsigned long long ws = 0;
-          const size_t tb = (size_t)b * TC_MAX_SLOTS + s0;
-          for (int i = 0; i < n; ++i) ws += a.slot_p16 ? a.slot_p16[tb + i] : (unsigned long long)P16;
-          atomicAdd(a.widths, ws);
-        }
       }
       __syncthreads();  // also keeps s_grab until everyone has read it
-      if (n) return tg;
+      if (warp == 8 && n && a.mode == TC_M2L && (a.tiles || a.widths)) {
+        unsigned ws = 0;
+        for (int i = lane; i < n; i += 32) ws += s_w[buf][i];
+        ws = __reduce_add_sync(0xffffffffu, ws);
+        if (lane == 0 && a.tiles) atomicAdd(a.tiles, (unsigned long long)n);
+        if (lane == 0 && a.widths) atomicAdd(a.widths, (unsigned long long)ws);
+      }
+      if (n) return;
     }
   };
 
-  int tg_cur = load_meta(0);
+  int tg_cur, tgg_cur, tg_nxt, tgg_nxt;
+  load_meta(0, tg_cur, tgg_cur);
   if (s_n[0] == 0) return;
-  int tg_nxt = load_meta(1);
+  load_meta(1, tg_nxt, tgg_nxt);
 
-  if (warp == 0) {
+  if (warp == 8) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)),
                  "r"(NCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (tid == 0) {
-    mbar_init(&s_full[0], 1);
-    mbar_init(&s_full[1], 1);
-    mbar_init(&s_mma[0], 1);
-    mbar_init(&s_mma[1], 1);
+    for (int i = 0; i < TC_NBUF; ++i) {
+      mbar_init(&s_full[i], 1);
+      mbar_init(&s_mma[i], 1);
+    }
+    mbar_init(&s_a, TC_WORKERS / 32);
     mbar_init(&s_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -284,255 +332,307 @@ __global__ void __launch_bounds__(TC_M, 1) k_tc_translate(TcArgs a, int nb, unsi
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = s_tmem;
-  const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
 
-  // Stream bookkeeping: the current batch (buffer c) starts at tile t_cur,
-  // the next (buffer c ^ 1) at t_nxt; tiles end at t_end.
-  int c = 0;
-  long long t_cur = 0, t_nxt = (long long)s_n[0] * TILES, t_end = t_nxt + (long long)s_n[1] * TILES;
-
-  // operator copy g (splits in the order 2, 1, 0; output tiles 0, 1).  A
-  // slot of padded width w < P16 needs only the first w rows (k) of each
-  // tile, a contiguous prefix, and no second tile when w <= N0; an unneeded
-  // copy completes its barrier without data.
-  const int IMG = a.img_p16 ? a.img_p16 : P16;  // operator images: N0 equals this kernel's first tile
-  auto load_tile = [&](long long g) {
-    const int buf = g < t_nxt ? c : c ^ 1;
-    const int i = (int)((g - (g < t_nxt ? t_cur : t_nxt)) / TILES), t = (int)(g % TILES);
-    const int s = 2 - t / NT, j = t % NT;
-    const int w = s_w[buf][i];
-    if ((j ? w - N0 : w) <= 0) {
-      mbar_arrive(&s_full[g & 1]);
-      return;
-    }
-    const uint32_t bytes = (uint32_t)(w * (j ? N1 : N0) * 2);
-    const uint16_t *src =
-        a.bimg + (size_t)s_op[buf][i] * 3 * IMG * IMG + (size_t)s * IMG * IMG + (j ? (size_t)IMG * N0 : 0);
-    bulk_load(Bs + (g & 1) * BTILE, src, bytes, &s_full[g & 1]);
-  };
-  // the MMAs of operator copy g for a slot of width w: B split s against A
-  // splits 2 - s .. 0, N = the tile's needed columns, w / 16 K steps
-  auto mma_tile = [&](long long g, int w) {
-    const int t = (int)(g % TILES);
-    const int s = 2 - t / NT, j = t % NT;
-    const int nw = j ? N1 : N0;
-    const int ncols = min(nw, j ? w - N0 : w);
-    if (ncols > 0) {
-      const uint32_t idesc =
-          (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ncols >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-      const uint32_t lbo_b = (uint32_t)(nw / 8) * 128;
-      const uint32_t a0 = smem_u32(As), b0 = smem_u32(Bs + (g & 1) * BTILE);
-      const int ksteps = w / 16;
-      for (int sa = 2 - s; sa >= 0; --sa)
-        for (int ks = 0; ks < ksteps; ++ks) {
-          const uint64_t ad = smem_desc(a0 + (uint32_t)(sa * ASPLIT * 2) + ks * 2 * LBO_A, LBO_A, 128);
-          const uint64_t bd = smem_desc(b0 + ks * 2 * lbo_b, lbo_b, 128);
-          const uint32_t acc = (s == 2 && sa == 0 && ks == 0) ? 0u : 1u;
-          mma_bf16(tmem + (j ? (uint32_t)N0 : 0u), ad, bd, idesc, acc);
-        }
-    }
-    mma_commit(&s_mma[g & 1]);
-  };
-
-  // source cell of target `tg` for slot i of metadata buffer `buf`, and its
-  // row.  The source index of a slot is loaded one slot ahead of its row,
-  // so that only the row load is left in the window of the MMAs.
-  float4 rv[P16 / 4];
-  auto src_of = [&](int buf, int i, int tg) -> int {
-    if (tg < 0) return -1;
-    if (a.mode == TC_M2L) return a.src_tab[((size_t)s_b[buf] * TC_MAX_SLOTS + s_slot[buf][i]) * TC_M + tid];
-    if (a.mode == TC_M2M) return tg;
-    return a.cparent[tg];
-  };
-  auto fetch = [&](int buf, int i, int src) {
-    const float4 *xr = (const float4 *)(a.X + (size_t)(src >= 0 ? src - a.cell0 : 0) * a.KS);
-    const int lim = min(a.KS, (int)s_w[buf][i]);  // the slot's order needs its first w inputs
-#pragma unroll
-    for (int q = 0; q < P16 / 4; ++q) rv[q] = (src >= 0 && 4 * q < lim) ? xr[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  // A operand of the next slot from the prefetched rows: two values per
-  // conversion (cvt.rn.bf16x2.f32), the same round-to-nearest splits as
-  // split3.  Columns K..KS-1 of a row are zero in memory and beyond KS the
-  // prefetch is zero, so no masking is needed.
-  auto write_a = [&](int w) {
-#pragma unroll
-    for (int kc = 0; kc < KC; ++kc) {
-      if (kc * 8 >= w) break;  // the MMAs of a slot of width w read only its first w columns
-      const float v[8] = {rv[2 * kc].x, rv[2 * kc].y, rv[2 * kc].z, rv[2 * kc].w,
-                          rv[2 * kc + 1].x, rv[2 * kc + 1].y, rv[2 * kc + 1].z, rv[2 * kc + 1].w};
-      uint32_t h[4], m[4], l[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) split3x2(v[2 * e], v[2 * e + 1], h[e], m[e], l[e]);
-      const size_t off = ((size_t)kc * (TC_M / 8) + tid / 8) * 64 + (tid % 8) * 8;
-      *(uint4 *)(As + off) = make_uint4(h[0], h[1], h[2], h[3]);
-      *(uint4 *)(As + ASPLIT + off) = make_uint4(m[0], m[1], m[2], m[3]);
-      *(uint4 *)(As + 2 * ASPLIT + off) = make_uint4(l[0], l[1], l[2], l[3]);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  };
-
-  long long nl = 0, nwait = 0;  // thread 0: copies issued, copies waited for
-  long long sidx = 0;           // slots done by this CTA (parity of s_done)
-  if (tid == 0) {
-    load_tile(0);
-    load_tile(1);  // every slot has three or more copies
-    nl = 2;
-  }
-  fetch(0, 0, src_of(0, 0, tg_cur));
-  int src_nx = -1;    // the source index of the next slot to fetch ...
-  bool pre = false;   // ... when it was loaded ahead
-  if (s_n[0] > 1) {
-    src_nx = src_of(0, 1, tg_cur);
-    pre = true;
-  } else if (s_n[1]) {
-    src_nx = src_of(1, 0, tg_nxt);
-    pre = true;
-  }
+  int c = 0;           // metadata buffer of the current batch
   bool ok = true;
-  while (ok) {
-    const int n = s_n[c];
-    for (int j = 0; j < n; ++j, ++sidx) {
-      write_a(s_w[c][j]);
-      tc_fence_before();
-      __syncthreads();
-      tc_fence_after();
-      // rows of the next slot, in flight during the MMAs
-      if (j + 1 < n) {
-        fetch(c, j + 1, pre ? src_nx : src_of(c, j + 1, tg_cur));
-        pre = false;
-        if (j + 2 < n) {
-          src_nx = src_of(c, j + 2, tg_cur);
-          pre = true;
-        } else if (s_n[c ^ 1]) {
-          src_nx = src_of(c ^ 1, 0, tg_nxt);
-          pre = true;
+  uint32_t sidx = 0;   // slots of the batches before the current one (parity of s_a and s_done)
+
+  if (warp == 9) {
+    // ------------------------------------------------------ operator copies
+    // Copy g (over all slots of all batches: splits in the order 2, 1, 0, of
+    // each the parts of KH of the slot's first w K rows) goes to buffer
+    // g % TC_NBUF once the MMAs of copy g - TC_NBUF are done.  Up to TC_NBUF
+    // copies of the next batch are issued before the batch ends.
+    uint32_t g = 0;
+    int ahead = 0;  // copies of the current batch issued during the one before
+    auto stream = [&](int buf, int skip, int most) -> int {  // the batch's copies [skip, most)
+      int k = 0;
+      for (int i = 0; i < s_n[buf]; ++i) {
+        const int w = s_w[buf][i], np = (w + KH - 1) / KH;
+        if (k + 3 * np <= skip) {
+          k += 3 * np;
+          continue;
         }
-      } else if (s_n[c ^ 1]) {
-        fetch(c ^ 1, 0, pre ? src_nx : src_of(c ^ 1, 0, tg_nxt));
-        pre = false;
-        if (s_n[c ^ 1] > 1) {  // the batch after next is not loaded yet
-          src_nx = src_of(c ^ 1, 1, tg_nxt);
-          pre = true;
-        }
-      }
-      if (tid == 0) {
-        for (int t = 0; t < TILES && ok; ++t) {
-          const long long g = t_cur + (long long)j * TILES + t;
-          if (!mbar_wait(&s_full[g & 1], (uint32_t)((g >> 1) & 1))) {
-            ok = false;
-            break;
+        const uint16_t *img = a.bimg + (size_t)s_op[buf][i] * 3 * P16 * P16;
+        for (int s = 2; s >= 0; --s)
+          for (int h = 0; h < np; ++h, ++k) {
+            if (k < skip) continue;
+            if (k >= most) return k;
+            const uint32_t b = g % TC_NBUF;
+            if (g >= TC_NBUF &&
+                !__all_sync(0xffffffffu, mbar_wait(&s_mma[b], ((g / TC_NBUF) - 1) & 1))) {
+              ok = false;
+              return k;
+            }
+            if (lane == 0)
+              bulk_load(Bs + b * BTILE, img + (size_t)s * P16 * P16 + (size_t)h * KH * P16,
+                        (uint32_t)min(w - h * KH, KH) * P16 * 2, &s_full[b]);
+            __syncwarp();
+            ++g;
           }
-          nwait = g + 1;
-          mma_tile(g, s_w[c][j]);
-          if (nl == g + 1 && nl < t_end && g >= 1) {  // the buffer of copy g - 1 takes copy g + 1
-            if (!mbar_wait(&s_mma[(g - 1) & 1], (uint32_t)(((g - 1) >> 1) & 1))) {
+      }
+      return k;
+    };
+    while (true) {
+      stream(c, ahead, 1 << 30);
+      ahead = ok ? stream(c ^ 1, 0, TC_NBUF) : 0;
+      const bool mine = ok;
+      ok = __syncthreads_and(ok);
+      if (!ok) {
+        if (!mine && lane == 0) atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
+        break;
+      }
+      if (s_n[c ^ 1] == 0) break;
+      c ^= 1;
+      load_meta(c ^ 1, tg_nxt, tgg_nxt);
+    }
+    if (!ok)  // the last copy into each buffer may still be in flight
+      for (uint32_t q = g > TC_NBUF ? g - TC_NBUF : 0; q < g; ++q)
+        if (!mbar_wait(&s_full[q % TC_NBUF], (q / TC_NBUF) & 1)) break;
+  } else if (warp == 8) {
+    // ---------------------------------------------------------------- MMAs
+    uint32_t g = 0;  // operator copies consumed
+    // A and B descriptors: the high words are constant, the low words hold
+    // the address and advance by constants from one K step to the next
+    const uint64_t adesc0 = smem_desc(smem_u32(As), LBO_A, 128), bdesc0 = smem_desc(smem_u32(Bs), LBO_B, 128);
+    // K steps [0, nk) of A split sa, from K row h KH, against copy q;
+    // first: D starts afresh
+    auto mma_steps = [&](int sa, int h, uint32_t q, int nk, uint32_t idesc, bool first) {
+      const uint64_t ad = adesc0 + (uint32_t)((sa * ASPLIT * 2 + h * (KH / 8) * (int)LBO_A) >> 4);
+      const uint64_t bd = bdesc0 + (((q % TC_NBUF) * (uint32_t)(BTILE * 2)) >> 4);
+#pragma unroll
+      for (int ks = 0; ks < KH / 16; ++ks)
+        if (ks < nk)
+          mma_bf16(tmem, ad + (uint32_t)(ks * 2 * (int)LBO_A >> 4), bd + (uint32_t)(ks * 2 * (int)LBO_B >> 4), idesc,
+                   first && ks == 0 ? 0u : 1u);
+    };
+    const bool lead = elect_one();
+    while (true) {
+      const int n = s_n[c];
+      // one thread waits and issues, without a warp-wide step in between
+      for (int j = 0; lead && j < n && ok; ++j) {
+        if (!mbar_wait(&s_a, (sidx + (uint32_t)j) & 1)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const int w = s_w[c][j], np = (w + KH - 1) / KH;
+        const uint32_t idesc =
+            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(w >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+#pragma unroll
+        for (int s = 2; s >= 0; --s)
+          for (int h = 0; h < np; ++h, ++g) {
+            if (!mbar_wait(&s_full[g % TC_NBUF], (g / TC_NBUF) & 1)) {
               ok = false;
               break;
             }
-            load_tile(nl++);
+            const int nk = min(w - h * KH, KH) / 16;
+            if (s == 2) {
+              mma_steps(0, h, g, nk, idesc, h == 0);
+              mma_commit(&s_mma[g % TC_NBUF]);
+            } else if (s == 1) {
+              mma_steps(1, h, g, nk, idesc, false);
+              mma_steps(0, h, g, nk, idesc, false);
+              mma_commit(&s_mma[g % TC_NBUF]);
+            } else {
+              mma_steps(2, h, g, nk, idesc, false);
+              mma_steps(1, h, g, nk, idesc, false);
+              if (h == np - 1) {  // the largest product (x1 y1) last, over all parts (np <= TC_NBUF: all resident)
+                for (int q = 0; q < np; ++q) {
+                  const uint32_t gq = g - (uint32_t)(np - 1 - q);
+                  mma_steps(0, q, gq, min(w - q * KH, KH) / 16, idesc, false);
+                  mma_commit(&s_mma[gq % TC_NBUF]);
+                }
+                mma_commit(&s_done);
+              }
+            }
           }
-        }
-        mma_commit(&s_done);  // also when stopping early, so that nobody waits in vain
       }
-      const bool dn = mbar_wait(&s_done, (uint32_t)(sidx & 1));
-      // tcgen05.ld/st are warp-collective: the whole warp goes on only if it saw the commit
-      const bool wd = __all_sync(0xffffffffu, dn);
-      if (!wd) ok = false;
-      tc_fence_after();
-      if (wd) {
-        const int w = s_w[c][j];  // D holds the slot's first w columns
+      __syncwarp();
+      sidx += (uint32_t)n;
+      const bool mine = ok;
+      ok = __syncthreads_and(ok);
+      if (!ok) {
+        if (!mine) atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
+        break;
+      }
+      if (s_n[c ^ 1] == 0) break;
+      c ^= 1;
+      load_meta(c ^ 1, tg_nxt, tgg_nxt);
+    }
+  } else {
+    // ------------------------------------------------------------- workers
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const int half = warp >> 2, r8 = lane & 7;
+    // source cell of row `grow` (target tgg) for slot i of metadata buffer
+    // `buf`.  The source index of a slot is loaded one slot ahead of its
+    // rows, so that only the row loads are left in the window of the MMAs.
+    auto src_of = [&](int buf, int i, int tgg) -> int {
+      if (tgg < 0) return -1;
+      if (a.mode == TC_M2L) return a.src_tab[((size_t)s_b[buf] * TC_MAX_SLOTS + s_slot[buf][i]) * TC_M + grow];
+      if (a.mode == TC_M2M) return tgg;
+      return a.cparent[tgg];
+    };
+    // A warp gathers its 16 rows together, in units of 8 columns of one row
+    // (32 bytes, one load): the 8 lanes of an octet take 8 rows of one column
+    // chunk and the 4 octets consecutive chunks, so that a load instruction
+    // reads 8 rows x 128 contiguous bytes, each sector once, and the 16-byte
+    // stores of an octet into a core matrix of A fill 128 contiguous bytes.
+    // (One row per thread touched 32 lines per instruction, half a sector
+    // each.)  Unit 4 u + octet of the slot's 2 (w / 8): row group (unit) /
+    // (w / 8), column chunk (unit) % (w / 8).
+    float rv[KC / 2][8];
+    auto fetch = [&](int w, int src) {
+      const int nkc = w >> 3;      // the slot's order needs its first w inputs
+      const int kmax = a.KS >> 3;  // chunks that exist in memory (KS is a multiple of 8)
+      int kc = lane >> 3, rg = 0;
+      while (kc >= nkc) kc -= nkc, ++rg;
 #pragma unroll
-        for (int c0 = 0; c0 < P16; c0 += 16) {
-          if (c0 < w) {
+      for (int u = 0; u < KC / 2; ++u) {
+        if (2 * u >= nkc) break;
+        const int sr = __shfl_sync(0xffffffffu, src, 8 * rg + r8);
+        if (sr >= 0 && kc < kmax) {
+          const float *x = a.X + (size_t)(sr - a.cell0) * a.KS + 8 * kc;
+          asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                       : "=f"(rv[u][0]), "=f"(rv[u][1]), "=f"(rv[u][2]), "=f"(rv[u][3]), "=f"(rv[u][4]),
+                         "=f"(rv[u][5]), "=f"(rv[u][6]), "=f"(rv[u][7])
+                       : "l"(x));
+        } else {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) rv[u][e] = 0.f;
+        }
+        kc += 4;
+        while (kc >= nkc) kc -= nkc, ++rg;
+      }
+    };
+    // A operand of the next slot from the prefetched rows: two values per
+    // conversion (cvt.rn.bf16x2.f32).  Columns K..KS-1 of a row are zero in
+    // memory and beyond KS the prefetch is zero, so no masking is needed.
+    auto write_a = [&](int w) {
+      const int nkc = w >> 3;  // the MMAs of a slot of width w read only its first w columns
+      int kc = lane >> 3, rg = 0;
+      while (kc >= nkc) kc -= nkc, ++rg;
+#pragma unroll
+      for (int u = 0; u < KC / 2; ++u) {
+        if (2 * u >= nkc) break;
+        uint32_t h[4], m[4], l[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split3x2(rv[u][2 * e], rv[u][2 * e + 1], h[e], m[e], l[e]);
+        const int off = (kc * (TC_M / 8) + warp * 2 + rg) * 64 + r8 * 8;
+        *(uint4 *)(As + off) = make_uint4(h[0], h[1], h[2], h[3]);
+        *(uint4 *)(As + ASPLIT + off) = make_uint4(m[0], m[1], m[2], m[3]);
+        *(uint4 *)(As + 2 * ASPLIT + off) = make_uint4(l[0], l[1], l[2], l[3]);
+        kc += 4;
+        while (kc >= nkc) kc -= nkc, ++rg;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      tc_fence_before();  // D and R of the slot before have been read
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_a);
+    };
+    fetch(s_w[0][0], src_of(0, 0, tgg_cur));
+    while (true) {
+      const int n = s_n[c];
+      // the source index of the next slot to fetch
+      int src_nx = n > 1 ? src_of(c, 1, tgg_cur) : s_n[c ^ 1] ? src_of(c ^ 1, 0, tgg_nxt) : -1;
+      int wr = 0;  // columns of R written so far
+      for (int j = 0; j < n && ok; ++j) {
+        const uint32_t si = sidx + (uint32_t)j;
+        const int w = s_w[c][j];
+        write_a(w);
+        // rows of the next slot, in flight during the MMAs
+        if (j + 1 < n) {
+          fetch(s_w[c][j + 1], src_nx);
+          src_nx = j + 2 < n ? src_of(c, j + 2, tgg_cur) : s_n[c ^ 1] ? src_of(c ^ 1, 0, tgg_nxt) : -1;
+        } else if (s_n[c ^ 1]) {
+          fetch(s_w[c ^ 1][0], src_nx);
+        }
+        // tcgen05.ld/st are warp-collective: the whole warp goes on only if it saw the commit
+        if (!__all_sync(0xffffffffu, mbar_wait(&s_done, si & 1))) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        // R += D (the slot's first w columns)
+#pragma unroll
+        for (int c0 = 0; c0 < P16; c0 += 32) {
+          const int cc = c0 + 16 * half;
+          if (cc < w) {
             uint32_t d[16];
-            tmem_ld16(tmem + lane_off + (uint32_t)c0, d);
-            if (j > 0) {
+            tmem_ld16(tmem + lane_off + (uint32_t)cc, d);
+            if (cc < wr) {
               uint32_t r[16];
-              tmem_ld16(tmem + lane_off + RCOL + (uint32_t)c0, r);
+              tmem_ld16(tmem + lane_off + RCOL + (uint32_t)cc, r);
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
               for (int e = 0; e < 16; ++e) d[e] = __float_as_uint(__uint_as_float(d[e]) + __uint_as_float(r[e]));
             } else {
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             }
-            tmem_st16(tmem + lane_off + RCOL + (uint32_t)c0, d);
-          } else if (j == 0) {
-            const uint32_t z[16] = {};
-            tmem_st16(tmem + lane_off + RCOL + (uint32_t)c0, z);
+            tmem_st16(tmem + lane_off + RCOL + (uint32_t)cc, d);
           }
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        wr = max(wr, w);
       }
-      // all MMAs of this slot are done: the buffer of its last copy takes the next one
-      const long long g_end = t_cur + (long long)(j + 1) * TILES;
-      if (tid == 0 && ok && nl < t_end && nl == g_end + 1) load_tile(nl++);
-      tc_fence_before();
-      ok = __syncthreads_and(ok);
-      if (!ok) break;
-    }
-    if (!ok) break;
-    // epilogue: R into the targets' expansions (fire-and-forget vector
-    // reductions; M2M rows of several batches meet in one parent)
-    tc_fence_after();
-    {
-      const int dst = a.mode == TC_M2M ? (tg_cur >= 0 ? a.cparent[tg_cur] : -1) : tg_cur;
-      float *y = a.Y + (size_t)(dst >= 0 ? dst - a.cell0 : 0) * a.KS;
+      sidx += (uint32_t)n;
+      // epilogue: R into the targets' expansions (fire-and-forget vector
+      // reductions; M2M rows of several batches meet in one parent)
+      if (ok) {
+        const int dst = a.mode == TC_M2M ? (tg_cur >= 0 ? a.cparent[tg_cur] : -1) : tg_cur;
+        float *y = a.Y + (size_t)(dst >= 0 ? dst - a.cell0 : 0) * a.KS;
 #pragma unroll
-      for (int c0 = 0; c0 < P16; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem + lane_off + RCOL + (uint32_t)c0, r);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (dst >= 0) {
+        for (int c0 = 0; c0 < P16; c0 += 32) {
+          const int cc = c0 + 16 * half;
+          if (cc < wr) {
+            uint32_t r[16];
+            tmem_ld16(tmem + lane_off + RCOL + (uint32_t)cc, r);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (dst >= 0) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (c0 + 4 * q < a.KS)
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(y + c0 + 4 * q), "r"(r[4 * q]),
-                           "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
-                           : "memory");
+              for (int q = 0; q < 4; ++q)
+                if (cc + 4 * q < a.KS)
+                  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(y + cc + 4 * q), "r"(r[4 * q]),
+                               "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3])
+                               : "memory");
+            }
+          }
         }
       }
+      // advance: the next batch becomes current; take the one after it
+      const bool mine = ok;
+      ok = __syncthreads_and(ok);
+      if (!mine && lane == 0) atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
+      if (!ok || s_n[c ^ 1] == 0) break;
+      c ^= 1;
+      tg_cur = tg_nxt;
+      tgg_cur = tgg_nxt;
+      load_meta(c ^ 1, tg_nxt, tgg_nxt);
     }
-    tc_fence_before();
-    // advance: the next batch becomes current; take the one after it
-    if (s_n[c ^ 1] == 0) break;
-    c ^= 1;
-    tg_cur = tg_nxt;
-    t_cur = t_nxt;
-    t_nxt = t_end;
-    tg_nxt = load_meta(c ^ 1);  // syncs: everyone has finished the epilogue's TMEM reads
-    t_end = t_nxt + (long long)s_n[c ^ 1] * TILES;
   }
 
-  if (!ok && tid == 0) {
-    atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
-    for (long long g = nwait; g < nl; ++g)  // copies still in flight
-      if (!mbar_wait(&s_full[g & 1], (uint32_t)((g >> 1) & 1))) break;
-  }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS));
+  if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS));
 }
 
 // ------------------------------------------------------------------ host
 static size_t tc_dyn_smem(int P16) {
-  return (size_t)3 * TC_M * P16 * 2 + (size_t)2 * P16 * tc_n0(P16) * 2;
+  return (size_t)3 * TC_M * P16 * 2 + (size_t)TC_NBUF * P16 * tc_kpart(P16) * 2;
 }
 
-size_t tc_smem_bytes(int P16) { return tc_dyn_smem(P16); }
-
-int tc_build_images(const float *tab, int n_slots, int K, int KP, int P16, uint16_t *img, cudaStream_t st,
+int tc_build_images(const float *tab, int n_slots, int K, int KP, int W, uint16_t *img, cudaStream_t st,
                     int64_t &launches) {
-  k_tc_images<<<n_slots, 256, 0, st>>>(tab, K, KP, P16, tc_n0(P16), img);
+  k_tc_images<<<n_slots, 256, 0, st>>>(tab, K, KP, W, img);
   launches += 1;
   return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
 template <int P16>
 static int tc_launch_p(const TcArgs &a, int nb, unsigned int *work, cudaStream_t st) {
-  // at most two CTAs per SM (each holds 256 TMEM columns), one when a CTA
-  // holds 512
+  // at most as many CTAs per SM as TMEM has room for
   size_t sh = tc_dyn_smem(P16);
-  sh = std::max(sh, P16 <= 128 ? (size_t)80 * 1024 : (size_t)120 * 1024);
+  sh = std::max(sh, P16 <= 64 ? (size_t)60 * 1024 : P16 <= 128 ? (size_t)80 * 1024 : (size_t)120 * 1024);
   // the shared-memory opt-in is per function and device
   static std::mutex mu;
   static size_t attr[64] = {};
@@ -552,7 +652,7 @@ static int tc_launch_p(const TcArgs &a, int nb, unsigned int *work, cudaStream_t
           cudaFuncSetAttribute(k_tc_translate<P16>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                cudaSharedmemCarveoutMaxShared) != cudaSuccess)
         return FMM_ERR_CUDA;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dev[dev], k_tc_translate<P16>, TC_M, sh) !=
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_dev[dev], k_tc_translate<P16>, TC_THREADS, sh) !=
               cudaSuccess ||
           per_sm_dev[dev] < 1)
         return FMM_ERR_CUDA;
@@ -560,20 +660,21 @@ static int tc_launch_p(const TcArgs &a, int nb, unsigned int *work, cudaStream_t
     }
     per_sm = per_sm_dev[dev];
   }
-  // a CTA of the kernels up to 128 wide holds 256 TMEM columns and under
-  // half the shared memory, so two share an SM: launch two per SM whatever
-  // the occupancy query says (the CTAs take work from a counter, so a CTA
-  // that cannot start at once only finds less work)
-  if (P16 <= 128) per_sm = std::max(per_sm, 2);
-  // M2L with fewer than four batches per CTA: runs of 24 slots as work items,
-  // so that the CTAs finish together
+  // the narrow kernels' CTAs share an SM whatever the occupancy query says
+  // (they take work from a counter, so a CTA that cannot start at once only
+  // finds less work)
+  per_sm = std::max(per_sm, tc_per_sm(P16));
+  // M2L with fewer than four batches per CTA: runs of at most 24 slots as
+  // work items, so that the CTAs finish together; fewer slots (down to 4)
+  // while there are not four items per CTA
   TcArgs b = a;
   b.chunk_slots = TC_MAX_SLOTS;
-  if (a.mode == TC_M2L && nb < 4 * per_sm * nsm) b.chunk_slots = 24;
+  if (a.mode == TC_M2L && nb < 4 * per_sm * nsm)
+    b.chunk_slots = std::max(4, std::min(24, (int)((int64_t)nb * TC_MAX_SLOTS / (4 * per_sm * nsm))));
   if (a.mode == TC_M2L && a.run_slots > 0) b.chunk_slots = std::min(a.run_slots, TC_MAX_SLOTS);
   const int chunks = a.mode == TC_M2L ? (TC_MAX_SLOTS + b.chunk_slots - 1) / b.chunk_slots : 1;
   const int grid = std::min(nb * chunks, per_sm * nsm);
-  k_tc_translate<P16><<<grid, TC_M, sh, st>>>(b, nb, work);
+  k_tc_translate<P16><<<grid, TC_THREADS, sh, st>>>(b, nb, work);
   return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 

@@ -26,10 +26,8 @@ struct TcArgs {
   int op_base;              // M2M / L2L: operator-table slot of child class 0
   const float *X;           // source expansions, KS floats per cell
   float *Y;                 // target expansions (accumulated into)
-  const uint16_t *bimg;     // BF16 split operator images, 3 * P16^2 per table slot
-  int cell0, K, KS, P16;    // P16 = K rounded up to 16
-  int img_p16;              // padded width the operator images were built for (0: P16); a narrower
-                            // kernel reads the first output tile of wider images (same first-tile width)
+  const uint16_t *bimg;     // BF16 split operator images of width P16: 3 * P16^2 per table slot
+  int cell0, K, KS, P16;    // P16: width of the kernel, K rounded up to 16 (narrow M2L tiles: less)
   unsigned int *err;
   unsigned long long *tiles;  // M2L: number of (batch, slot) tiles contracted (nullable)
   unsigned long long *widths; // M2L: sum of the tiles' padded widths (nullable)
@@ -38,11 +36,15 @@ struct TcArgs {
                             // split into items whose sums all add into the targets)
 };
 
-// Width of the first output tile: one tile up to 128 columns, else two.
-__host__ __device__ constexpr int tc_n0(int P16) { return P16 <= 128 ? P16 : ((P16 / 2 + 15) & ~15); }
+// K rows of one operator copy: a whole split up to 48, half of it up to 128,
+// else a third (four copies and the three A splits fill the shared memory of
+// one CTA at 176, and of two at 96).
+__host__ __device__ constexpr int tc_kpart(int P16) {
+  return P16 <= 48 ? P16 : P16 <= 128 ? ((P16 / 16 + 1) / 2) * 16 : ((P16 / 16 + 2) / 3) * 16;
+}
 
-size_t tc_smem_bytes(int P16);
-int tc_build_images(const float *tab, int n_slots, int K, int KP, int P16, uint16_t *img, cudaStream_t st,
+// The images of the operators' first W rows and columns (W a multiple of 16).
+int tc_build_images(const float *tab, int n_slots, int K, int KP, int W, uint16_t *img, cudaStream_t st,
                     int64_t &launches);
 // Launches one translation pass over nb batches; `work` is a zeroed device
 // counter the persistent CTAs take batches from.

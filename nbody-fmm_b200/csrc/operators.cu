@@ -259,7 +259,7 @@ int build_op_tables(OpTables &ops, int dim, int p, int depth, const PassGeom &g,
                     bool want64) {
   int K = dim == 3 ? (p + 1) * (p + 1) : 2 * p + 1;
   int KP = 32 * ((K + 31) / 32);
-  int KS = (K + 3) & ~3;
+  int KS = (K + 7) & ~7;  // rows of M and L start on 32-byte sectors (the 256-bit row loads of k_tc_translate)
   ops.dim = dim;
   ops.p = p;
   ops.K = K;
