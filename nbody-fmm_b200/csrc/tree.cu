@@ -6,12 +6,16 @@
 // leaf coordinate at depth d, (unsigned)((x - a) / ((b - a) / 2^d)), equals
 // floor(2^d * q) with q = (x - a) / (b - a) in FP64, because dividing by a
 // power of two commutes with IEEE rounding; so the key at depth d is the key
-// at D shifted right by dim*(D-d).  One radix sort of the D-keys then gives
-// the maximum leaf occupancy of any depth as a maximum run length.  The
-// reference's leaves with their particles in input order (tree.cpp:62-66)
-// are the runs of that order with each run put back in input order (a rank
-// count inside the leaf), or for leaves of more than 512 particles a second
-// stable sort of the depth-d keys in input order.
+// at D shifted right by dim*(D-d).  One radix sort of the D-keys then holds
+// the cells of every depth as runs: particle i starts a cell at each depth
+// above the number of levels its key shares with the key before it.  One
+// pass over the sorted keys counts the cells and the largest cell of every
+// depth, so that the depth loop and the sizes of all levels need one read of
+// the host, and one more writes the cells of all levels.  The reference's
+// leaves with their particles in input order (tree.cpp:62-66) are the leaf
+// runs with each run put back in input order (a rank count inside the leaf),
+// or for leaves of more than 512 particles a second stable sort of the
+// depth-d keys in input order.
 #include <algorithm>
 #include <vector>
 
@@ -77,22 +81,33 @@ __global__ void k_scan_blocks(uint32_t *sums, int nb, uint32_t *total_out) {
   if (threadIdx.x == 0 && total_out) *total_out = carry;
 }
 
-__global__ void k_scan_apply(const uint32_t *in, uint32_t *out, int64_t n, const uint32_t *block_offs) {
+// Without block offsets (block_offs null) every block adds up the sums of the
+// blocks before it itself, and the last one writes the total.
+__global__ void k_scan_apply(const uint32_t *in, uint32_t *out, int64_t n, const uint32_t *block_offs,
+                             const uint32_t *sums, uint32_t *total_out) {
   __shared__ uint32_t s_warp[SCAN_BLOCK / 32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+  uint32_t off, total;
+  if (block_offs) {
+    off = block_offs[blockIdx.x];
+  } else {
+    uint32_t t = 0;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_BLOCK) t += sums[k];
+    block_excl_scan(t, s_warp, off);
+  }
   uint32_t v[SCAN_ITEMS], s = 0;
   for (int i = 0; i < SCAN_ITEMS; ++i) {
     int64_t k = base + i;
     v[i] = k < n ? in[k] : 0;
     s += v[i];
   }
-  uint32_t total;
-  uint32_t e = block_excl_scan(s, s_warp, total) + block_offs[blockIdx.x];
+  uint32_t e = block_excl_scan(s, s_warp, total) + off;
   for (int i = 0; i < SCAN_ITEMS; ++i) {
     int64_t k = base + i;
     if (k < n) out[k] = e;
     e += v[i];
   }
+  if (!block_offs && total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = off + total;
 }
 
 // Exclusive prefix sum of n uint32 (in may alias out); *total_dev = sum.
@@ -102,10 +117,13 @@ void exclusive_scan(Workspace &ws, const uint32_t *in, uint32_t *out, int64_t n,
   uint32_t *sums = ws.scan_tmp(nb);
   // k_scan_reduce uses a strided tile layout and k_scan_apply a blocked one;
   // both cover the same SCAN_TILE elements per block, so the sums agree.
+  // Up to 2048 blocks (4M elements) adding the sums up in every block is
+  // cheaper than a launch for it.
+  const bool two = nb <= 2048;
   k_scan_reduce<<<nb, SCAN_BLOCK, 0, st>>>(in, n, sums);
-  k_scan_blocks<<<1, SCAN_BLOCK, 0, st>>>(sums, nb, total_dev);
-  k_scan_apply<<<nb, SCAN_BLOCK, 0, st>>>(in, out, n, sums);
-  ws.launches += 3;
+  if (!two) k_scan_blocks<<<1, SCAN_BLOCK, 0, st>>>(sums, nb, total_dev);
+  k_scan_apply<<<nb, SCAN_BLOCK, 0, st>>>(in, out, n, two ? nullptr : sums, sums, total_dev);
+  ws.launches += two ? 2 : 3;
 }
 
 // ------------------------------------------------------------ radix sort
@@ -115,8 +133,12 @@ static constexpr int RS_TILE = RS_BLOCK * RS_ROUNDS;
 // Largest leaf whose order k_leaf_order redoes in place (each particle counts
 // the smaller input indices of its leaf); larger leaves take the full sort.
 static constexpr int LEAF_ORDER_MAX = 512;
+// Up to this many tiles (65,536 items) the scatter adds up the tiles'
+// histograms itself, two launches per digit instead of four.
+static constexpr int RS_FUSED_TILES = 32;
 
-__global__ void k_radix_hist(const uint64_t *keys, int64_t n, int shift, uint32_t *hist, int nb) {
+// hist: [digit][tile], or [tile][256] (by_tile).
+__global__ void k_radix_hist(const uint64_t *keys, int64_t n, int shift, uint32_t *hist, int nb, bool by_tile) {
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -126,16 +148,19 @@ __global__ void k_radix_hist(const uint64_t *keys, int64_t n, int shift, uint32_
     if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
   }
   __syncthreads();
-  hist[(int64_t)threadIdx.x * nb + blockIdx.x] = h[threadIdx.x];
+  if (by_tile) hist[(int64_t)blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
+  else hist[(int64_t)threadIdx.x * nb + blockIdx.x] = h[threadIdx.x];
 }
 
 // Stable scatter of one tile of RS_TILE items: items are ranked in (round,
 // warp, lane) order, which is their input order inside the tile, and placed
 // in shared memory in digit order; then consecutive threads write each
 // digit's run to its consecutive places in the output (coalesced stores).
+// offs: the exclusive scan of the [digit][tile] histograms, or with by_tile
+// the [tile][256] histograms themselves, which thread d adds up for digit d.
 __global__ void __launch_bounds__(RS_BLOCK) k_radix_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
                                                             uint32_t *vout, int64_t n, int shift, const uint32_t *offs,
-                                                            int nb) {
+                                                            int nb, bool by_tile) {
   __shared__ uint64_t s_key[RS_TILE];
   __shared__ uint32_t s_val[RS_TILE];
   __shared__ uint32_t s_goff[256], s_tstart[256], s_run[256], s_warp[RS_BLOCK / 32];
@@ -144,7 +169,17 @@ __global__ void __launch_bounds__(RS_BLOCK) k_radix_scatter(const uint64_t *kin,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t base = (int64_t)blockIdx.x * RS_TILE;
   const int tile_n = (int)min((int64_t)RS_TILE, n - base);
-  s_goff[tid] = offs[(int64_t)tid * nb + blockIdx.x];  // the digit's first place in the output
+  if (by_tile) {
+    uint32_t all = 0, before = 0, total;
+    for (int b = 0; b < nb; ++b) {
+      const uint32_t v = offs[(int64_t)b * 256 + tid];
+      if (b == (int)blockIdx.x) before = all;
+      all += v;
+    }
+    s_goff[tid] = block_excl_scan(all, s_warp, total) + before;
+  } else {
+    s_goff[tid] = offs[(int64_t)tid * nb + blockIdx.x];  // the digit's first place in the output
+  }
   s_run[tid] = 0;
   s_tstart[tid] = 0;  // the tile's digit histogram first
   __syncthreads();
@@ -206,10 +241,11 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
   if (n <= 1 || bits <= 0) return;
   int nb = (int)((n + RS_TILE - 1) / RS_TILE);
   uint32_t *hist = ws.radix_hist(nb);
+  const bool by_tile = nb <= RS_FUSED_TILES;
   for (int shift = 0; shift < bits; shift += 8) {
-    k_radix_hist<<<nb, RS_BLOCK, 0, st>>>(keys, n, shift, hist, nb);
-    exclusive_scan(ws, hist, hist, (int64_t)256 * nb, nullptr, st);
-    k_radix_scatter<<<nb, RS_BLOCK, 0, st>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, nb);
+    k_radix_hist<<<nb, RS_BLOCK, 0, st>>>(keys, n, shift, hist, nb, by_tile);
+    if (!by_tile) exclusive_scan(ws, hist, hist, (int64_t)256 * nb, nullptr, st);
+    k_radix_scatter<<<nb, RS_BLOCK, 0, st>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, nb, by_tile);
     ws.launches += 2;
     std::swap(keys, keys_alt);
     std::swap(vals, vals_alt);
@@ -217,49 +253,71 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
 }
 
 // ------------------------------------------------------------ tree kernels
-__global__ void k_aabb_init(unsigned long long *box) {
-  if (threadIdx.x < 3) {
-    box[threadIdx.x] = ~0ull;     // min
-    box[3 + threadIdx.x] = 0ull;  // max
-  }
-}
-
 // AABB (tree.cpp:20-30) plus a finiteness check of positions and masses.
-__global__ void k_aabb(const double *pos, const double *mass, int64_t n, int dim, unsigned long long *box,
-                       unsigned int *err) {
-  unsigned long long lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0, 0, 0};
+// Every block writes its box to part[block][6]; the last one to finish (a
+// ticket per block; *ticket returns to zero) reduces them into geom = {min,
+// max}.  (Atomic minima and maxima of every warp on the same six words took
+// 50 us on 2^20 particles, most of a 25 MB read's 5 us.)
+__global__ void __launch_bounds__(256) k_aabb(const double *pos, const double *mass, int64_t n, int dim,
+                                              unsigned long long *part, unsigned int *ticket, double *geom,
+                                              unsigned int *err) {
+  __shared__ unsigned long long s_box[8][6];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long v[6] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull};
   bool bad = false;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    for (int d = 0; d < dim; ++d) {
-      double x = pos[i * dim + d];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      if (d >= dim) break;
+      const double x = pos[i * dim + d];
       bad |= !isfinite(x);
-      unsigned long long u = dbl_to_ordered(x);
-      lo[d] = u < lo[d] ? u : lo[d];
-      hi[d] = u > hi[d] ? u : hi[d];
+      const unsigned long long u = dbl_to_ordered(x);
+      v[d] = u < v[d] ? u : v[d];
+      v[3 + d] = u > v[3 + d] ? u : v[3 + d];
     }
     bad |= !isfinite(mass[i]);
   }
-  for (int d = 0; d < dim; ++d) {
-    for (int o = 16; o; o >>= 1) {
-      unsigned long long a = __shfl_xor_sync(0xffffffffu, lo[d], o), b = __shfl_xor_sync(0xffffffffu, hi[d], o);
-      lo[d] = a < lo[d] ? a : lo[d];
-      hi[d] = b > hi[d] ? b : hi[d];
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(err, FMM_DEV_ERR_NONFINITE_INPUT);
+  // the block's box: thread d < 6 ends with component d
+  auto reduce = [&]() {
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, v[d], o);
+        v[d] = d < 3 ? (t < v[d] ? t : v[d]) : (t > v[d] ? t : v[d]);
+      }
+      if (lane == 0) s_box[warp][d] = v[d];
     }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(&box[d], lo[d]);
-      atomicMax(&box[3 + d], hi[d]);
+    __syncthreads();
+    unsigned long long r = 0;
+    if (threadIdx.x < 6) {
+      const int d = threadIdx.x;
+      r = s_box[0][d];
+      for (int w = 1; w < 8; ++w) r = d < 3 ? min(r, s_box[w][d]) : max(r, s_box[w][d]);
     }
-  }
-  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, FMM_DEV_ERR_NONFINITE_INPUT);
-}
-
-__global__ void k_box_decode(const unsigned long long *box, double *geom, int dim) {
-  if (threadIdx.x == 0) {
-    for (int d = 0; d < 3; ++d) {
-      geom[d] = d < dim ? ordered_to_dbl(box[d]) : 0.0;
-      geom[3 + d] = d < dim ? ordered_to_dbl(box[3 + d]) : 0.0;
+    return r;
+  };
+  unsigned long long r = reduce();
+  if (threadIdx.x < 6) part[(size_t)blockIdx.x * 6 + threadIdx.x] = r;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+#pragma unroll
+  for (int d = 0; d < 6; ++d) v[d] = d < 3 ? ~0ull : 0ull;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      const unsigned long long t = __ldcg(part + (size_t)b * 6 + d);
+      v[d] = d < 3 ? min(v[d], t) : max(v[d], t);
     }
-  }
+  r = reduce();
+  if (threadIdx.x < 6) geom[threadIdx.x] = threadIdx.x % 3 < dim ? ordered_to_dbl(r) : 0.0;
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
 // Key of each particle at the maximum depth Dmax; values = input index.
@@ -300,90 +358,164 @@ __global__ void k_leafkeys_input(const double *pos, int64_t n, int dim, int Dmax
   vals[i] = (uint32_t)i;
 }
 
-__global__ void k_run_flags(const uint64_t *keys, int64_t n, int shift, uint32_t *flags) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t k = shift >= 64 ? 0 : keys[i] >> shift;
-  uint64_t kp = (i == 0 || shift >= 64) ? 0 : keys[i - 1] >> shift;
-  flags[i] = (i == 0 || k != kp) ? 1u : 0u;
+// Levels 0 .. cp on which sorted keys a <= b share their cell (cp = Dmax: the
+// same key): level d compares the keys shifted right by dim (Dmax - d).
+__device__ inline int common_level(uint64_t a, uint64_t b, int dim, int Dmax) {
+  const uint64_t x = a ^ b;
+  return x ? Dmax - 1 - (63 - __clzll((long long)x)) / dim : Dmax;
 }
 
-__global__ void k_run_starts(const uint32_t *flags, const uint32_t *idx, int64_t n, uint32_t *starts) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (flags[i]) starts[idx[i]] = (uint32_t)i;
-}
+static constexpr int LV_BLOCK = 256, LV_ROUNDS = 4, LV_TILE = LV_BLOCK * LV_ROUNDS, LV_MAX = FMM_MAX_DEPTH + 1;
 
-__global__ void k_run_max(const uint32_t *starts, const uint32_t *nruns, int64_t n, uint32_t *maxlen) {
-  uint32_t nr = *nruns;
-  uint32_t m = 0;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nr; j += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t e = (j + 1 < nr) ? starts[j + 1] : (uint32_t)n;
-    uint32_t l = e - starts[j];
-    m = l > m ? l : m;
+// One pass over the sorted Dmax keys for all depths at once.  Particle i
+// starts a cell on every level d > cp(i - 1, i) (all levels for i = 0).
+//   blockcnt[d * nb + tile]: cells of level d that start in the tile;
+//   lev[d]: their sum, lev[LV_MAX + d]: the largest cell of level d (zeroed
+//   by the caller).
+// The cell that particle i starts on level d ends where the key differs on
+// level d; from the deepest level up its end only moves on, so one walk
+// (doubling steps, then halving) gives the sizes on all levels.  Levels on
+// which the next particle starts a cell too have size 1.
+__global__ void __launch_bounds__(LV_BLOCK) k_levels(const uint64_t *keys, int64_t n, int dim, int Dmax, int nb,
+                                                     uint32_t *blockcnt, uint32_t *lev) {
+  __shared__ uint32_t s_cnt[LV_MAX + 1], s_max[LV_MAX];
+  for (int d = threadIdx.x; d <= LV_MAX; d += LV_BLOCK) {
+    s_cnt[d] = 0;
+    if (d < LV_MAX) s_max[d] = 1;
   }
-  for (int o = 16; o; o >>= 1) {
-    uint32_t y = __shfl_xor_sync(0xffffffffu, m, o);
-    m = y > m ? y : m;
+  __syncthreads();
+  for (int r = 0; r < LV_ROUNDS; ++r) {
+    const int64_t i = (int64_t)blockIdx.x * LV_TILE + r * LV_BLOCK + threadIdx.x;
+    const uint64_t k = i < n ? keys[i] : 0;
+    // the particle starts a cell on the levels first .. Dmax (first = Dmax + 1: on none)
+    const int first = i >= n ? Dmax + 1 : i == 0 ? 0 : common_level(keys[i - 1], k, dim, Dmax) + 1;
+    const unsigned peers = __match_any_sync(0xffffffffu, first);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&s_cnt[first], (uint32_t)__popc(peers));
+    int64_t j = i + 1;  // the keys in [i, j) share level d
+    for (int d = j < n ? common_level(k, keys[j], dim, Dmax) : -1; d >= first; --d) {
+      const int sh = dim * (Dmax - d);
+      auto same = [&](int64_t q) { return q < n && (sh >= 64 || (keys[q] >> sh) == (k >> sh)); };
+      int64_t step = 1;
+      while (same(j + step - 1)) {
+        j += step;
+        step *= 2;
+      }
+      for (step /= 2; step > 0; step /= 2)
+        if (same(j + step - 1)) j += step;
+      const uint32_t len = (uint32_t)(j - i);
+      if (len > s_max[d]) atomicMax(&s_max[d], len);
+    }
+    __syncwarp();
   }
-  if ((threadIdx.x & 31) == 0) atomicMax(maxlen, m);
+  __syncthreads();
+  if (threadIdx.x <= Dmax) {
+    const int d = threadIdx.x;
+    uint32_t c = 0;
+    for (int f = 0; f <= d; ++f) c += s_cnt[f];
+    blockcnt[(size_t)d * nb + blockIdx.x] = c;
+    if (c) atomicAdd(&lev[d], c);
+    // (a word read a moment early only costs an atomic that changes nothing)
+    if (s_max[d] > *(volatile uint32_t *)&lev[LV_MAX + d]) atomicMax(&lev[LV_MAX + d], s_max[d]);
+  }
 }
 
-// The final particle order from the Dmax order.  A leaf is a run of equal
-// depth-D keys (the Dmax key shifted right by `shift`); inside it the final
-// order is the input order, i.e. the particles sorted by their input index
-// (vals), so each particle's place is its rank among its leaf's indices.
-// Runs come from the depth loop's last pass: exclusive scan idx of the run
-// flags, run starts, nruns runs.  The result equals the stable sort of the
-// depth-D keys from input order.
-__global__ void k_leaf_order(const uint64_t *keys, const uint32_t *vals, const uint32_t *flags, const uint32_t *idx,
-                             const uint32_t *starts, uint32_t nruns, int64_t n, int shift, uint64_t *lk,
+// Exclusive scan of each level's tile counts, in place: one block per level.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_level_scan(uint32_t *blockcnt, int nb) {
+  __shared__ uint32_t s_warp[SCAN_BLOCK / 32];
+  uint32_t *row = blockcnt + (size_t)blockIdx.x * nb;
+  uint32_t carry = 0;
+  for (int b0 = 0; b0 < nb; b0 += SCAN_TILE) {
+    uint32_t v[SCAN_ITEMS], s = 0, tot;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) {
+      const int k = b0 + (int)threadIdx.x * SCAN_ITEMS + i;
+      v[i] = k < nb ? row[k] : 0;
+      s += v[i];
+    }
+    uint32_t e = carry + block_excl_scan(s, s_warp, tot);
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) {
+      const int k = b0 + (int)threadIdx.x * SCAN_ITEMS + i;
+      if (k < nb) row[k] = e;
+      e += v[i];
+    }
+    carry += tot;
+  }
+}
+
+struct LevelOffsets {
+  int off[LV_MAX + 1];  // first cell of each level 0 .. D, then the end
+};
+
+// The cells of all levels 0 .. D from the sorted Dmax keys and the scanned
+// tile counts: cell r of a level is the r-th particle that starts one there
+// (a ballot per level and 32 particles).  Writes keys, particle ranges,
+// parents and children (filled with -1 before) and every particle's leaf.
+__global__ void __launch_bounds__(LV_BLOCK) k_make_cells(const uint64_t *keys, int64_t n, int dim, int Dmax, int D,
+                                                         int nb, const uint32_t *blockoff, LevelOffsets lo,
+                                                         uint64_t *ckey, int *cpbeg, int *cpend, int *cparent,
+                                                         int *cchild, int *leaf_of) {
+  __shared__ uint32_t s_wc[LV_MAX][LV_BLOCK / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // a warp takes 32 LV_ROUNDS consecutive particles
+  const int64_t base = (int64_t)blockIdx.x * LV_TILE + warp * 32 * LV_ROUNDS;
+  uint64_t key[LV_ROUNDS];
+  int first[LV_ROUNDS];
+#pragma unroll
+  for (int r = 0; r < LV_ROUNDS; ++r) {
+    const int64_t i = base + r * 32 + lane;
+    key[r] = i < n ? keys[i] : 0;
+    first[r] = i >= n ? LV_MAX + 1 : i == 0 ? 0 : common_level(keys[i - 1], key[r], dim, Dmax) + 1;
+  }
+  for (int d = 0; d <= D; ++d) {
+    int c = 0;
+#pragma unroll
+    for (int r = 0; r < LV_ROUNDS; ++r) c += __popc(__ballot_sync(0xffffffffu, first[r] <= d));
+    if (lane == 0) s_wc[d][warp] = (uint32_t)c;
+  }
+  __syncthreads();
+  int up[LV_ROUNDS];  // the particle's cell one level up
+#pragma unroll
+  for (int r = 0; r < LV_ROUNDS; ++r) up[r] = -1;
+  for (int d = 0; d <= D; ++d) {
+    int c = lo.off[d] + (int)blockoff[(size_t)d * nb + blockIdx.x] - 1;
+    for (int w = 0; w < warp; ++w) c += (int)s_wc[d][w];
+    const int sh = dim * (Dmax - d);
+#pragma unroll
+    for (int r = 0; r < LV_ROUNDS; ++r) {
+      const int64_t i = base + r * 32 + lane;
+      const bool head = first[r] <= d;
+      const unsigned m = __ballot_sync(0xffffffffu, head);
+      const int cell = c + __popc(m & (0xffffffffu >> (31 - lane)));
+      c += __popc(m);
+      if (head) {
+        const uint64_t k = sh >= 64 ? 0ull : key[r] >> sh;
+        ckey[cell] = k;
+        cpbeg[cell] = (int)i;
+        if (cell > lo.off[d]) cpend[cell - 1] = (int)i;
+        cparent[cell] = up[r];
+        if (d > 0) cchild[((int64_t)up[r] << dim) + (int)(k & ((1u << dim) - 1u))] = cell;
+      }
+      if (i == n - 1) cpend[lo.off[d + 1] - 1] = (int)n;
+      if (d == D && i < n) leaf_of[i] = cell;
+      up[r] = cell;
+    }
+  }
+}
+
+// The final particle order from the Dmax order: inside a leaf the input
+// order, i.e. the particles sorted by their input index (vals), so each
+// particle's place is its rank among its leaf's indices.  The result equals
+// the stable sort of the depth-D keys from input order.
+__global__ void k_leaf_order(const uint32_t *vals, const int *leaf_of, const int *cpbeg, const int *cpend, int64_t n,
                              uint32_t *pv) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t L = idx[i] + flags[i] - 1u;  // this particle's run
-  const int64_t s = starts[L], e = L + 1u < nruns ? (int64_t)starts[L + 1u] : n;
+  const int L = leaf_of[i], s = cpbeg[L], e = cpend[L];
   const uint32_t v = vals[i];
-  int64_t r = 0;
-  for (int64_t j = s; j < e; ++j) r += vals[j] < v ? 1 : 0;
+  int r = 0;
+  for (int j = s; j < e; ++j) r += vals[j] < v ? 1 : 0;
   pv[s + r] = v;
-  lk[s + r] = shift >= 64 ? 0ull : keys[i] >> shift;
-}
-
-// Leaves: one per run of equal leaf keys in the sorted order.
-__global__ void k_make_leaves(const uint64_t *lk_sorted, const uint32_t *flags, const uint32_t *idx, int64_t n,
-                              int leaf_base, uint64_t *cell_key, int *cell_pbeg, int *cell_pend, int *leaf_of) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int li = (int)idx[i] - (flags[i] ? 0 : 1);
-  leaf_of[i] = leaf_base + li;
-  if (flags[i]) {
-    cell_key[leaf_base + li] = lk_sorted[i];
-    cell_pbeg[leaf_base + li] = (int)i;
-  }
-  if (i == n - 1 || flags[i + 1]) cell_pend[leaf_base + li] = (int)(i + 1);
-}
-
-__global__ void k_parent_flags(const uint64_t *ckey, int cbase, int nchild, int dim, uint32_t *flags) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nchild) return;
-  flags[j] = (j == 0 || (ckey[cbase + j] >> dim) != (ckey[cbase + j - 1] >> dim)) ? 1u : 0u;
-}
-
-__global__ void k_make_parents(uint64_t *ckey, int *cpbeg, int *cpend, int *cparent, int *cchild, int cbase,
-                               int nchild, int pbase, int dim, const uint32_t *flags, const uint32_t *idx) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nchild) return;
-  const int nc = 1 << dim;
-  int pi = pbase + (int)idx[j] - (flags[j] ? 0 : 1);
-  uint64_t k = ckey[cbase + j];
-  cparent[cbase + j] = pi;
-  cchild[(int64_t)pi * nc + (int)(k & (nc - 1))] = cbase + j;
-  if (flags[j]) {
-    ckey[pi] = k >> dim;
-    cpbeg[pi] = cpbeg[cbase + j];
-  }
-  if (j == nchild - 1 || flags[j + 1]) cpend[pi] = cpend[cbase + j];
 }
 
 // Adaptive targets, per cell g (flag[g - cell0]): bit 0, a target: the root,
@@ -479,11 +611,6 @@ __global__ void k_root_colleague(int *ccoll, int root, int dim) {
   }
 }
 
-__global__ void k_fill_i32(int *p, int64_t n, int v) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = v;
-}
-
 // Gathers particles into leaf order: the offset from the leaf's geometric
 // centre split into FP32 hi + lo parts (x - c = hi + lo to ~48 bits), and the
 // FP32 mass, used by P2M, L2P (hi only) and P2P (hi and lo).
@@ -536,113 +663,83 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   const int Dmax = ((64 / dim) >> dim) << dim;  // tree.cpp:38
   const int TPB = 256;
   const int nbN = cdiv(n, TPB);
-  ws.reserve_particles(n);
+  const int nblv = cdiv(n, LV_TILE);
+  if (!ws.reserve_particles(n) || !ws.blev.reserve((size_t)nblv * (Dmax + 1))) return FMM_ERR_OUT_OF_MEMORY;
+  uint32_t *lev = ws.scalars;  // cells, then the largest cell, of every level
   CUDA_TRY(cudaMemsetAsync(ws.dev_err, 0, sizeof(unsigned int), st));
-  // AABB
-  k_aabb_init<<<1, 32, 0, st>>>(ws.box_u64);
-  k_aabb<<<std::min(nbN, 148 * 8), TPB, 0, st>>>(d_pos, d_mass, n, dim, ws.box_u64, ws.dev_err);
-  k_box_decode<<<1, 32, 0, st>>>(ws.box_u64, ws.geom, dim);
+  CUDA_TRY(cudaMemsetAsync(lev, 0, 2 * LV_MAX * sizeof(uint32_t), st));
+  k_aabb<<<std::min(nbN, WS_AABB_BLOCKS), TPB, 0, st>>>(d_pos, d_mass, n, dim, ws.box_u64, ws.ticket, ws.geom,
+                                                       ws.dev_err);
   k_keys<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, ws.geom, ws.keyA, ws.valA);
-  ws.launches += 4;
-  CUDA_TRY(cudaMemcpyAsync(t.lo, ws.geom, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  unsigned int herr = 0;
-  CUDA_TRY(cudaMemcpyAsync(&herr, ws.dev_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaStreamSynchronize(st));
-  if (herr & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
-  for (int d = 0; d < 3; ++d) t.hi[d] = t.lo[3 + d];
-
+  ws.launches += 2;
   // sort all particles by their Dmax key
   uint64_t *kA = ws.keyA, *kB = ws.keyB;
   uint32_t *vA = ws.valA, *vB = ws.valB;
   radix_sort(ws, kA, vA, kB, vB, n, dim * Dmax, st);
+  k_levels<<<nblv, LV_BLOCK, 0, st>>>(kA, n, dim, Dmax, nblv, ws.blev.ptr, lev);
+  ws.launches += 1;
+  // the box, the finiteness check (keys of non-finite positions are clamped
+  // into range, so what ran above is harmless) and the levels' sizes
+  uint32_t hlev[2 * LV_MAX];
+  unsigned int herr = 0;
+  CUDA_TRY(cudaMemcpyAsync(t.lo, ws.geom, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(&herr, ws.dev_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(hlev, lev, sizeof(hlev), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaStreamSynchronize(st));
+  if (herr & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
+  for (int d = 0; d < 3; ++d) t.hi[d] = t.lo[3 + d];
 
   // depth loop, tree.cpp:43-69
   unsigned int max_n = (unsigned int)n;
-  unsigned int depth = 0, nruns = 0;
-  uint32_t *flags = ws.u32A, *idx = ws.u32B, *starts = ws.u32C;
+  unsigned int depth = 0;
   do {
     uint64_t n_leafs = (uint64_t)(max_n - 1) / (unsigned)threshold + 1;
     depth += bit_width_u64(n_leafs) / dim + 1;
     if (depth > (unsigned)Dmax) depth = Dmax;
-    int shift = dim * (Dmax - (int)depth);
-    k_run_flags<<<nbN, TPB, 0, st>>>(kA, n, shift, flags);
-    exclusive_scan(ws, flags, idx, n, ws.scalars, st);
-    k_run_starts<<<nbN, TPB, 0, st>>>(flags, idx, n, starts);
-    CUDA_TRY(cudaMemsetAsync(ws.scalars + 1, 0, sizeof(uint32_t), st));
-    k_run_max<<<std::min(nbN, 148 * 8), TPB, 0, st>>>(starts, ws.scalars, n, ws.scalars + 1);
-    ws.launches += 3;
-    uint32_t h[2];
-    CUDA_TRY(cudaMemcpyAsync(h, ws.scalars, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    max_n = h[1];
-    nruns = h[0];
+    max_n = hlev[LV_MAX + depth];
   } while (depth < (unsigned)Dmax && max_n > (unsigned)threshold);
   t.depth = (int)depth;
   const int D = t.depth;
 
-  // final order: stable sort of the depth-D leaf keys, starting from input
-  // order, so each leaf keeps its particles in input order (tree.cpp:62-66).
-  // The depth-D key is the Dmax key shifted right, so the Dmax order already
-  // groups the leaves; with leaves of at most LEAF_ORDER_MAX particles only
-  // the order inside each leaf is redone (k_leaf_order), else the leaf keys
-  // are sorted afresh from input order.
-  uint64_t *lk = ws.keyC, *lkAlt = ws.keyA;
-  uint32_t *pv = ws.valC, *pvAlt = ws.valA;
+  // the cells of all levels, contiguous from the root
+  const int nc = 1 << dim, ns = dim == 3 ? 27 : 9;
+  LevelOffsets lo;
+  t.level_count.assign(D + 1, 0);
+  t.level_off.assign(D + 2, 0);
+  t.level_max.assign(D + 1, 0);
+  int64_t cells = 0;
+  for (int d = 0; d <= D; ++d) {
+    lo.off[d] = t.level_off[d] = (int)cells;
+    t.level_count[d] = (int)hlev[d];
+    t.level_max[d] = (int)hlev[LV_MAX + d];
+    cells += hlev[d];
+    if (cells > (int64_t)INT32_MAX) return FMM_ERR_OUT_OF_MEMORY;
+  }
+  lo.off[D + 1] = t.level_off[D + 1] = (int)cells;
+  t.cell0 = 0;
+  t.n_cells = (int)cells;
+  if (!ws.reserve_cells(cells, nc, ns)) return FMM_ERR_OUT_OF_MEMORY;
+  CUDA_TRY(cudaMemsetAsync(ws.cell_child, 0xff, sizeof(int) * (size_t)cells * nc, st));
+  k_level_scan<<<D + 1, SCAN_BLOCK, 0, st>>>(ws.blev.ptr, nblv);
+  k_make_cells<<<nblv, LV_BLOCK, 0, st>>>(kA, n, dim, Dmax, D, nblv, ws.blev.ptr, lo, ws.cell_key, ws.cell_pbeg,
+                                          ws.cell_pend, ws.cell_parent, ws.cell_child, ws.leaf_of);
+  ws.launches += 2;
+  // final order: each leaf's particles in input order (tree.cpp:62-66).  The
+  // Dmax order already groups the leaves; with leaves of at most
+  // LEAF_ORDER_MAX particles only the order inside each leaf is redone, else
+  // the leaf keys are sorted afresh from input order.
+  uint32_t *pv = ws.valC;
   if (max_n <= (unsigned)LEAF_ORDER_MAX) {
-    k_leaf_order<<<nbN, TPB, 0, st>>>(kA, vA, flags, idx, starts, nruns, n, dim * (Dmax - D), lk, pv);
+    k_leaf_order<<<nbN, TPB, 0, st>>>(vA, ws.leaf_of, ws.cell_pbeg, ws.cell_pend, n, pv);
     ws.launches += 1;
   } else {
+    uint64_t *lk = ws.keyC, *lkAlt = ws.keyA;
+    uint32_t *pvAlt = ws.valA;
     k_leafkeys_input<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, D, ws.geom, ws.keyC, ws.valC);
     ws.launches += 1;
     radix_sort(ws, lk, pv, lkAlt, pvAlt, n, dim * D, st);
   }
-  t.d_leafkey_sorted = lk;
   t.d_perm = pv;
-
-  // leaves
-  k_run_flags<<<nbN, TPB, 0, st>>>(lk, n, 0, flags);
-  exclusive_scan(ws, flags, idx, n, ws.scalars, st);
-  ws.launches += 1;
-  uint32_t nleaves = 0;
-  CUDA_TRY(cudaMemcpyAsync(&nleaves, ws.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaStreamSynchronize(st));
-  t.level_count.assign(D + 1, 0);
-  t.level_off.assign(D + 2, 0);
-  t.level_count[D] = (int)nleaves;
-  const int nc = 1 << dim, ns = dim == 3 ? 27 : 9;
-  int64_t cap = (int64_t)(D + 1) * nleaves;
-  ws.reserve_cells(cap, nc, ns);
-  // levels are laid out bottom-up from the end of the cell arrays so that
-  // they end up contiguous and ordered from the root: [level 0, ..., level D]
-  int base = (int)(cap - nleaves);
-  k_make_leaves<<<nbN, TPB, 0, st>>>(lk, flags, idx, n, base, ws.cell_key, ws.cell_pbeg, ws.cell_pend, ws.leaf_of);
-  ws.launches += 1;
-  std::vector<int> lbase(D + 1);
-  lbase[D] = base;
-  for (int d = D - 1; d >= 0; --d) {
-    int nch = t.level_count[d + 1];
-    int cb = lbase[d + 1];
-    k_parent_flags<<<cdiv(nch, TPB), TPB, 0, st>>>(ws.cell_key, cb, nch, dim, flags);
-    exclusive_scan(ws, flags, idx, nch, ws.scalars, st);
-    uint32_t np = 0;
-    CUDA_TRY(cudaMemcpyAsync(&np, ws.scalars, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    int pb = cb - (int)np;
-    k_fill_i32<<<cdiv((int64_t)np * nc, TPB), TPB, 0, st>>>(ws.cell_child + (int64_t)pb * nc, (int64_t)np * nc, -1);
-    k_make_parents<<<cdiv(nch, TPB), TPB, 0, st>>>(ws.cell_key, ws.cell_pbeg, ws.cell_pend, ws.cell_parent,
-                                                    ws.cell_child, cb, nch, pb, dim, flags, idx);
-    ws.launches += 3;
-    t.level_count[d] = (int)np;
-    lbase[d] = pb;
-  }
-  // cell indices stay absolute: level d occupies [lbase[d], lbase[d] + count)
-  for (int d = 0; d <= D; ++d) t.level_off[d] = lbase[d];
-  t.level_off[D + 1] = (int)cap;
-  t.cell0 = lbase[0];
-  t.n_cells = (int)(cap - lbase[0]);
-  // leaf children are -1
-  k_fill_i32<<<cdiv((int64_t)nleaves * nc, TPB), TPB, 0, st>>>(ws.cell_child + (int64_t)lbase[D] * nc,
-                                                                (int64_t)nleaves * nc, -1);
   // adaptive targets (3D trees of depth >= 3, as the force pass runs them):
   // the flags now, so that only target cells get colleague rows
   const uint8_t *aflag = nullptr;
@@ -655,15 +752,15 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
     aflag = ws.aflag;
   }
   // colleagues, top-down
-  k_root_colleague<<<1, 32, 0, st>>>(ws.cell_coll, lbase[0], dim);
-  ws.launches += 2;
+  k_root_colleague<<<1, 32, 0, st>>>(ws.cell_coll, 0, dim);
+  ws.launches += 1;
   for (int d = 1; d <= D; ++d) {
     if (aflag)  // adaptive targets are 3D only
       k_colleagues_targets<3><<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(
-          ws.cell_key, ws.cell_parent, ws.cell_child, ws.cell_coll, lbase[d], t.level_count[d], aflag, t.cell0);
+          ws.cell_key, ws.cell_parent, ws.cell_child, ws.cell_coll, t.level_off[d], t.level_count[d], aflag, t.cell0);
     else
       k_colleagues<<<cdiv(t.level_count[d], 8), 8 * ns, 0, st>>>(ws.cell_key, ws.cell_parent, ws.cell_child,
-                                                                  ws.cell_coll, lbase[d], t.level_count[d], dim,
+                                                                  ws.cell_coll, t.level_off[d], t.level_count[d], dim,
                                                                   nullptr, t.cell0);
     ws.launches += 1;
   }

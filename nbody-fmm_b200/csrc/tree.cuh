@@ -46,10 +46,14 @@ struct DevBuf {
   }
 };
 
+// blocks of the bounding-box kernel
+static constexpr int WS_AABB_BLOCKS = 148 * 4;
+
 struct Workspace {
   // per particle
   DevBuf<uint64_t> bkeyA, bkeyB, bkeyC;
-  DevBuf<uint32_t> bvalA, bvalB, bvalC, bu32A, bu32B, bu32C;
+  DevBuf<uint32_t> bvalA, bvalB, bvalC;
+  DevBuf<uint32_t> blev;     // cells per level and tile of the sorted keys
   DevBuf<int> bleaf_of;
   DevBuf<float4> bpart;      // leaf-relative FP32 offset (hi part) + mass, leaf order
   DevBuf<float4> bpart_lo;   // low part of the offset
@@ -69,7 +73,7 @@ struct Workspace {
                                       // pairs, [4] sum over M2L pairs of the target's particle count
 
   uint64_t *keyA = nullptr, *keyB = nullptr, *keyC = nullptr;
-  uint32_t *valA = nullptr, *valB = nullptr, *valC = nullptr, *u32A = nullptr, *u32B = nullptr, *u32C = nullptr;
+  uint32_t *valA = nullptr, *valB = nullptr, *valC = nullptr;
   int *leaf_of = nullptr;
   float4 *part = nullptr, *part_lo = nullptr, *far = nullptr;
   uint64_t *cell_key = nullptr;
@@ -79,13 +83,18 @@ struct Workspace {
   unsigned long long *box_u64 = nullptr;
   double *geom = nullptr;
   uint32_t *scalars = nullptr;
+  unsigned int *ticket = nullptr;  // of the bounding-box kernel, zero between launches
   unsigned int *dev_err = nullptr;
   unsigned long long *counters = nullptr;
   int64_t launches = 0;
   bool ok = true;
 
   bool init_small() {
-    ok &= bbox.reserve(8) && bgeom.reserve(8) && bscalars.reserve(8) && berr.reserve(4) && bcount.reserve(8);
+    ok &= bbox.reserve(6 * WS_AABB_BLOCKS) && bgeom.reserve(8) && bscalars.reserve(2 * (FMM_MAX_DEPTH + 1) + 1) &&
+          berr.reserve(4) && bcount.reserve(8);
+    if (!ok) return false;
+    ticket = bscalars.ptr + 2 * (FMM_MAX_DEPTH + 1);
+    ok &= cudaMemset(ticket, 0, sizeof(unsigned int)) == cudaSuccess;
     counters = bcount.ptr;
     box_u64 = bbox.ptr;
     geom = bgeom.ptr;
@@ -96,11 +105,10 @@ struct Workspace {
   bool reserve_particles(int64_t n) {
     size_t m = (size_t)(n > 0 ? n : 1);
     ok &= bkeyA.reserve(m) && bkeyB.reserve(m) && bkeyC.reserve(m) && bvalA.reserve(m) && bvalB.reserve(m) &&
-          bvalC.reserve(m) && bu32A.reserve(m) && bu32B.reserve(m) && bu32C.reserve(m) && bleaf_of.reserve(m) &&
+          bvalC.reserve(m) && bleaf_of.reserve(m) &&
           bpart.reserve(m) && bpart_lo.reserve(m) && bfar.reserve(m);
     keyA = bkeyA.ptr; keyB = bkeyB.ptr; keyC = bkeyC.ptr;
     valA = bvalA.ptr; valB = bvalB.ptr; valC = bvalC.ptr;
-    u32A = bu32A.ptr; u32B = bu32B.ptr; u32C = bu32C.ptr;
     leaf_of = bleaf_of.ptr;
     part = bpart.ptr;
     part_lo = bpart_lo.ptr;
@@ -136,7 +144,7 @@ struct Workspace {
   void release_all() {
     bkeyA.release(); bkeyB.release(); bkeyC.release();
     bvalA.release(); bvalB.release(); bvalC.release();
-    bu32A.release(); bu32B.release(); bu32C.release();
+    blev.release();
     bleaf_of.release(); bpart.release(); bpart_lo.release(); bfar.release();
     bcell_key.release(); bcell_pbeg.release(); bcell_pend.release(); bcell_parent.release();
     bcell_child.release(); bcell_coll.release(); baflag.release(); balist.release();
@@ -155,11 +163,11 @@ struct TreeState {
   double lo[6] = {0, 0, 0, 0, 0, 0};  // lo[0..2] box min (lo[3..5] scratch)
   double hi[3] = {0, 0, 0};
   std::vector<int> level_count, level_off;
+  std::vector<int> level_max;  // particles of the largest cell of each level
   int cell0 = 0;      // index of the root
   int n_cells = 0;
   int adaptive_leaf = 0;  // adaptive targets: the threshold ws.aflag / ws.alist were computed for (0: none, and
                           // every cell has its colleague row; else only the target cells have one)
-  uint64_t *d_leafkey_sorted = nullptr;
   uint32_t *d_perm = nullptr;  // leaf order -> input index
 };
 
