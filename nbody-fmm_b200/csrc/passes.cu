@@ -996,9 +996,11 @@ static constexpr int DF_MAX_LEVELS = 33;
 
 struct DirectArgs {
   // levels of the launch, coarse first: warps [w0[k], w0[k+1]) take the
-  // cells first[k] + (warp - w0[k]), or with a target list (k_direct_far's
-  // LIST) the cells tlist[first[k] + (warp - w0[k])]
-  int nlev;
+  // cells first[k] + (warp - w0[k]) / parts[k], or with a target list
+  // (k_direct_far's LIST) the cells tlist[first[k] + (warp - w0[k]) / parts[k]];
+  // the parts of a cell take its targets `chunk` at a time in turn
+  int nlev, chunk;
+  int parts[DF_MAX_LEVELS];
   int first[DF_MAX_LEVELS], w0[DF_MAX_LEVELS + 1];
   const float4 *off[DF_MAX_LEVELS];  // particle offsets from their level-d ancestor's centre
   float h[DF_MAX_LEVELS][3];         // level-d cell size
@@ -1019,6 +1021,11 @@ struct DirectArgs {
 // Small T (NT <= 7 targets): every lane holds all targets and takes every
 // 32nd particle of the concatenated sources; larger T: register-blocked
 // target groups over sources staged through shared memory.
+//
+// With offsets that are not well separated (a box that is not near a cube)
+// whole pairs of coarse cells are summed, and with one warp per cell the
+// kernel waited for a few warps with thousands of targets: there a cell's
+// targets are spread over parts[k] warps.
 //
 // Per kept source cell si the warp keeps s_pref[si] (its first position in
 // the concatenation; every cell non-empty) and s_cell[si] = (shift c_S - c_T,
@@ -1146,7 +1153,52 @@ __device__ inline void blocked_shape(int nt, int R, int &Gl, float &cost) {
   cost = (float)(rounds * R) / (float)Gl;
 }
 
-template <int DIM, bool POT, bool LIST = false>
+// The targets [tb, tb + nt) of one cell against its listed sources.
+template <int DIM, bool POT>
+__device__ __forceinline__ void direct_targets(const DirectArgs &a, const float4 *off, int tb, int nt,
+                                               const float4 *s_cell, const int *s_pref, int nsrc, int lane,
+                                               float4 *stage) {
+  switch (nt) {
+    case 1: direct_small<1, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 2: direct_small<2, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 3: direct_small<3, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 4: direct_small<4, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 5: direct_small<5, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 6: direct_small<6, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    case 7: direct_small<7, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
+    default: break;
+  }
+  // larger T: the register blocking R in 1..4 that minimises the busiest lane's work (largest R on ties)
+  int bestR = 1, bestG = 1;
+  float best = 1e30f;
+#pragma unroll
+  for (int R = 1; R <= 4; ++R) {
+    int G;
+    float c;
+    blocked_shape(nt, R, G, c);
+    if (c <= best) {  // ties: the larger R reuses each staged source for more targets
+      best = c;
+      bestR = R;
+      bestG = G;
+    }
+  }
+  switch (bestR) {
+    case 1: direct_blocked<1, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
+    case 2: direct_blocked<2, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
+    case 3: direct_blocked<3, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
+    default: direct_blocked<4, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
+  }
+}
+
+// The same for a part of a large cell's targets, out of line (the kernel's own
+// copy keeps its registers).
+template <int DIM, bool POT>
+__device__ __noinline__ void direct_split(const DirectArgs &a, const float4 *off, int tb, int nt, const float4 *s_cell,
+                                          const int *s_pref, int nsrc, int lane, float4 *stage) {
+  direct_targets<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, stage);
+}
+
+template <int DIM, bool POT, bool LIST, bool SPLIT>
 __global__ void __launch_bounds__(256, 4) k_direct_far(DirectArgs a) {
   constexpr int NS = DIM == 3 ? 27 : 9, NC = 1 << DIM, NCAND = NS * NC, NR = (NCAND + 31) / 32;
   __shared__ float4 s_cell_all[8][189];
@@ -1158,9 +1210,16 @@ __global__ void __launch_bounds__(256, 4) k_direct_far(DirectArgs a) {
   if (wl >= a.w0[a.nlev]) return;
   int lv = a.nlev - 1;  // deep levels, which hold most of the warps, first
   while (wl < a.w0[lv]) --lv;
-  const int T = LIST ? a.tlist[a.first[lv] + (wl - a.w0[lv])] : a.first[lv] + (wl - a.w0[lv]);
-  const int tb = a.pbeg[T], nt = a.pend[T] - tb;
+  int ci = wl - a.w0[lv], part = 0;
+  const int parts = SPLIT ? a.parts[lv] : 1;
+  if (SPLIT && parts > 1) {
+    part = ci % parts;
+    ci /= parts;
+  }
+  const int T = LIST ? a.tlist[a.first[lv] + ci] : a.first[lv] + ci;
+  int tb = a.pbeg[T], nt = a.pend[T] - tb;
   if ((long long)nt > a.direct_max && !a.any_fdirect) return;
+  if (SPLIT && part > 0 && (long long)part * a.chunk >= nt) return;
   const float4 *off = a.off[lv];
   float4 *s_cell = s_cell_all[wib];
   int *s_pref = s_pref_all[wib];
@@ -1228,37 +1287,16 @@ __global__ void __launch_bounds__(256, 4) k_direct_far(DirectArgs a) {
   }
   __syncwarp();
   if (nsrc == 0) return;
-  if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
-  switch (nt) {
-    case 1: direct_small<1, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 2: direct_small<2, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 3: direct_small<3, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 4: direct_small<4, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 5: direct_small<5, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 6: direct_small<6, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    case 7: direct_small<7, DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane); return;
-    default: break;
+  if (!SPLIT || parts == 1) {
+    if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
+    direct_targets<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, s_stage_all[wib]);
+    return;
   }
-  // larger T: the register blocking R in 1..4 that minimises the busiest lane's work (largest R on ties)
-  int bestR = 1, bestG = 1;
-  float best = 1e30f;
-#pragma unroll
-  for (int R = 1; R <= 4; ++R) {
-    int G;
-    float c;
-    blocked_shape(nt, R, G, c);
-    if (c <= best) {  // ties: the larger R reuses each staged source for more targets
-      best = c;
-      bestR = R;
-      bestG = G;
-    }
-  }
-  float4 *stage = s_stage_all[wib];
-  switch (bestR) {
-    case 1: direct_blocked<1, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
-    case 2: direct_blocked<2, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
-    case 3: direct_blocked<3, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
-    default: direct_blocked<4, DIM, POT>(a, off, tb, nt, bestG, s_cell, s_pref, nsrc, lane, stage); break;
+  const int tend = tb + nt;
+  for (tb += part * a.chunk; tb < tend; tb += parts * a.chunk) {
+    nt = min(a.chunk, tend - tb);
+    if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
+    direct_split<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, s_stage_all[wib]);
   }
 }
 
@@ -2261,6 +2299,9 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     // the list (the level's cells in order, gaps after the targets)
     da.tlist = adaptive ? eb.ftl.ptr : nullptr;
     da.nlev = 0;
+    // targets per warp where cells are split: few enough that n of them give
+    // a few thousand warps, up to the 128 of four targets per lane
+    da.chunk = n < (1 << 17) ? 32 : n < (1 << 19) ? 64 : 128;
     int64_t nw = 0;
     for (int d = 2; d <= D; ++d) {
       const int k = da.nlev++;
@@ -2271,22 +2312,25 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
       da.h[k][0] = (float)(g.ext[0] * invd);
       da.h[k][1] = (float)(g.ext[1] * invd);
       da.h[k][2] = (float)(g.ext[2] * invd);
-      nw += adaptive ? (int64_t)ntgt[d] : (int64_t)t.level_count[d];
+      const int64_t nc = adaptive ? (int64_t)ntgt[d] : (int64_t)t.level_count[d];
+      const int64_t most = std::max<int64_t>(1, (1 << 25) / std::max<int64_t>(nc, 1));
+      da.parts[k] = any_fdirect ? (int)std::min<int64_t>(cdiv(t.level_max[d], da.chunk), most) : 1;
+      nw += nc * da.parts[k];
     }
     da.w0[da.nlev] = (int)nw;
     const int64_t grid = cdiv(nw * 32, TPB);
-    if (adaptive) {
-      if (grid > 0) {
-        if (want_pot) k_direct_far<3, true, true><<<grid, TPB, 0, st>>>(da);
-        else k_direct_far<3, false, true><<<grid, TPB, 0, st>>>(da);
-      }
-    } else if (dim == 3) {
-      if (want_pot) k_direct_far<3, true><<<grid, TPB, 0, st>>>(da);
-      else k_direct_far<3, false><<<grid, TPB, 0, st>>>(da);
-    } else {
-      if (want_pot) k_direct_far<2, true><<<grid, TPB, 0, st>>>(da);
-      else k_direct_far<2, false><<<grid, TPB, 0, st>>>(da);
-    }
+    auto pick = [&](auto plain, auto split) { return any_fdirect ? split : plain; };
+    void (*kern)(DirectArgs);
+    if (adaptive)
+      kern = want_pot ? pick(k_direct_far<3, true, true, false>, k_direct_far<3, true, true, true>)
+                      : pick(k_direct_far<3, false, true, false>, k_direct_far<3, false, true, true>);
+    else if (dim == 3)
+      kern = want_pot ? pick(k_direct_far<3, true, false, false>, k_direct_far<3, true, false, true>)
+                      : pick(k_direct_far<3, false, false, false>, k_direct_far<3, false, false, true>);
+    else
+      kern = want_pot ? pick(k_direct_far<2, true, false, false>, k_direct_far<2, true, false, true>)
+                      : pick(k_direct_far<2, false, false, false>, k_direct_far<2, false, false, true>);
+    if (grid > 0) kern<<<(unsigned)grid, TPB, 0, st>>>(da);
     ws.launches += 1;
   }
   if (ev) cudaEventRecord(ev[6], st);
