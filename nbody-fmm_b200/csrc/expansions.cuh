@@ -51,17 +51,15 @@ struct HostPinned {
 
 struct ExpBuffers {
   DevBuf<float> M, L;  // n_cells * KS each (indexed by absolute cell - cell0)
-  DevBuf<int> tlist;      // class-grouped cells of levels >= 2 (L2L targets)
-  DevBuf<int> tlist_m2l;  // the same restricted to cells with possible M2L pairs
-  DevBuf<uint64_t> ckey, ckey_alt, ckey_m2l;  // (level, class) sort keys of those cells
-  DevBuf<uint32_t> cval, cval2;
+  DevBuf<int> tlist;      // class-grouped cells of levels >= 2: all (without the shortcuts), then those with
+                          // possible M2L pairs
+  DevBuf<uint8_t> lkey;   // (level, class) list keys of those cells, two lists
   DevBuf<int4> batches;
   DevBuf<uint32_t> cls_count;
   DevBuf<float4> lvl_off;  // particle offsets from their level-d ancestor's centre, levels 2..D-1
   DevBuf<uint8_t> lact;    // shortcuts, per cell: [0, ncell) M2L contributions, [ncell, 2 ncell) needs L,
                            // [2 ncell, 3 ncell) M2L source, [3 ncell, 4 ncell) how M is formed
-  DevBuf<uint64_t> ukey;   // shortcuts: sort keys (two sorts, key and alternate each)
-  DevBuf<uint32_t> uval;
+  DevBuf<int> rows;        // shortcuts: class-grouped cells that need L2L, then the M2M rows
   DevBuf<int> p2m_list;    // shortcuts: the cells whose multipole comes straight from their particles, then their count
   DevBuf<int4> batches2;   // shortcuts: batches of the cells that need L2L, then of the M2M rows
   HostPinned<int4> hbatches, hbatches2;  // their host staging

@@ -158,14 +158,10 @@ int fmm_destroy(fmm_ctx *c) {
   c->eb.M.release();
   c->eb.L.release();
   c->eb.tlist.release();
+  c->eb.lkey.release();
+  c->eb.rows.release();
   c->eb.batches.release();
   c->eb.cls_count.release();
-  c->eb.ckey.release();
-  c->eb.ckey_alt.release();
-  c->eb.cval.release();
-  c->eb.cval2.release();
-  c->eb.ckey_m2l.release();
-  c->eb.tlist_m2l.release();
   c->eb.lvl_off.release();
   c->eb.m2l_src.release();
   c->eb.m2l_list.release();
@@ -180,7 +176,6 @@ int fmm_destroy(fmm_ctx *c) {
   c->eb.batches2.release();
   c->eb.esrc.release();
   c->eb.elev.release();
-  c->eb.ukey.release();
   c->eb.p2m_list.release();
   c->eb.ftl.release();
   c->eb.xs.release();
@@ -188,7 +183,6 @@ int fmm_destroy(fmm_ctx *c) {
   c->eb.citems.release();
   c->eb.hbatches.release();
   c->eb.hbatches2.release();
-  c->eb.uval.release();
   c->eb.m2l_split_w.release();
   c->eb.m2l_w.release();
   c->eb.cf.release();

@@ -1301,48 +1301,78 @@ __global__ void __launch_bounds__(256, 4) k_direct_far(DirectArgs a) {
 }
 
 // ------------------------------------------------------------------ lists
-// Sort keys (level, class) of the cells of one level: key_all for L2L (every
-// cell), key_m2l for M2L with 255 for cells that cannot have an M2L pair under
-// the direct-pair rule (every child S of the parent's colleagues has
-// n_T * n_S <= direct_max; adjacency is ignored, so the test only errs
-// towards keeping a cell), and with adaptive targets (aflag set) for cells
-// that are no target.
-__global__ void k_class_keys(const uint64_t *ckey, const int *cpbeg, const int *cpend, const int *cparent,
-                             const int *ccoll, const int *cchild, long long direct_max, int first, int count, int level,
-                             int dim, uint64_t *keys_all, uint64_t *keys_m2l, uint32_t *vals, int out_off,
-                             const uint8_t *aflag, int cell0) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  int g = first + i;
-  const uint64_t k = ((uint64_t)level << dim) | (ckey[g] & ((1u << dim) - 1));
-  keys_all[out_off + i] = k;
-  vals[out_off + i] = (uint32_t)g;
-  bool m2l = !aflag || (aflag[g - cell0] & 1);  // with adaptive targets only targets (and their rows) count
-  if (m2l && direct_max > 0) {
-    const int nc = 1 << dim, ns = dim == 3 ? 27 : 9;
-    const long long nt = cpend[g] - cpbeg[g];
-    const int *pc = ccoll + (int64_t)cparent[g] * ns;
-    m2l = false;
-    for (int s = 0; s < ns && !m2l; ++s) {
-      const int Q = pc[s];
-      if (Q < 0 || nt * (cpend[Q] - cpbeg[Q]) <= direct_max) continue;
-      for (int c = 0; c < nc && !m2l; ++c) {
-        const int q = cchild[(int64_t)Q * nc + c];
-        if (q >= 0 && nt * (cpend[q] - cpbeg[q]) > direct_max) m2l = true;
-      }
-    }
-  }
-  keys_m2l[out_off + i] = m2l ? k : 255u;
+// The level of cell g in [off[lo], off[D + 1]).
+__device__ inline int cell_level(const LevelOffsets &lv, int lo, int D, int g) {
+  while (lo < D && g >= lv.off[lo + 1]) ++lo;
+  return lo;
 }
 
-__global__ void k_class_hist(const uint64_t *keys, int n, uint32_t *hist) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    atomicAdd(&h[keys[i] & 255u], 1u);
-  __syncthreads();
-  if (h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
+// List keys (level << dim | class) of the cells of levels 2 .. D: key_all for
+// L2L (every cell; null: not wanted), key_m2l for M2L with 255 for cells that
+// cannot have an M2L pair under the direct-pair rule (every child S of the
+// parent's colleagues has n_T * n_S <= direct_max; adjacency is ignored, so
+// the test only errs towards keeping a cell), and with adaptive targets
+// (aflag set) for cells that are no target.
+//
+// A warp takes CW cells: one lane each for the flags and keys, then eight
+// lanes per cell that has to be looked at, four cells at a time, over the
+// parent's colleagues (one thread each waited for up to 216 loads one after
+// another: 130 us of a 4096-particle pass, where there is little else to
+// run).  CW = 32 for many cells, of which most need no look (44 M cells of a
+// 16M mixture: 2.4 ms with four cells per warp), 4 to spread few cells over
+// more warps.
+template <int DIM, int CW>
+__global__ void k_class_keys(const uint64_t *ckey, const int *cpbeg, const int *cpend, const int *cparent,
+                             const int *ccoll, const int *cchild, long long direct_max, LevelOffsets lv, int D,
+                             uint8_t *keys_all, uint8_t *keys_m2l, const uint8_t *aflag, int cell0) {
+  constexpr int NC = 1 << DIM, NS = DIM == 3 ? 27 : 9;
+  const int lane = threadIdx.x & 31, sub = lane & 7, oct = lane >> 3;
+  const int first = lv.off[2];
+  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * CW + lane;
+  const int g = first + i;
+  const bool in = lane < CW && g < lv.off[D + 1];
+  const bool target = in && (!aflag || (aflag[g - cell0] & 1));
+  unsigned look = direct_max > 0 ? __ballot_sync(0xffffffffu, target) : 0u;
+  unsigned m2l = direct_max > 0 ? 0u : __ballot_sync(0xffffffffu, target);
+  int nt_me = 0, par_me = 0;
+  if (target && direct_max > 0) {
+    nt_me = cpend[g] - cpbeg[g];
+    par_me = cparent[g];
+  }
+  while (look) {  // the next four cells, one per octet
+    unsigned rest = look;
+    for (int q = 0; q < oct; ++q) rest &= rest - 1;
+    const int b = __ffs(rest) - 1;  // -1: none left for this octet
+    const long long nt = __shfl_sync(0xffffffffu, nt_me, b & 31);
+    const int par = __shfl_sync(0xffffffffu, par_me, b & 31);
+    const int *pc = ccoll + (int64_t)par * NS;
+    bool open = b >= 0, hit = false;
+    for (int s0 = 0; s0 < NS; s0 += 8) {
+      if (!__any_sync(0xffffffffu, open)) break;
+      const int s = s0 + sub;
+      bool found = false;
+      const int Q = open && s < NS ? pc[s] : -1;
+      if (Q >= 0 && nt * (cpend[Q] - cpbeg[Q]) > direct_max) {
+        int q[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) q[c] = cchild[(int64_t)Q * NC + c];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) found |= q[c] >= 0 && nt * (cpend[q[c]] - cpbeg[q[c]]) > direct_max;
+      }
+      if (__ballot_sync(0xffffffffu, found) & (0xffu << (8 * oct))) {
+        hit = true;
+        open = false;
+      }
+    }
+    m2l |= __reduce_or_sync(0xffffffffu, hit ? 1u << b : 0u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) look &= look - 1;  // (zero stays zero)
+  }
+  if (in) {
+    const uint8_t k = (uint8_t)((cell_level(lv, 2, D, g) << DIM) | (int)(ckey[g] & (NC - 1)));
+    if (keys_all) keys_all[i] = k;
+    keys_m2l[i] = (m2l >> lane) & 1 ? k : (uint8_t)255;
+  }
 }
 
 // ------------------------------------------------------------ M shortcut
@@ -1408,19 +1438,20 @@ __global__ void k_zero_rows(const uint8_t *fx, uint8_t wx, float *X, const uint8
   }
 }
 
-// Sort keys of the M2M rows of one level: with child_rows (tensor-core
-// M2M, rows are children) the children of mode-2 cells by (level, class),
-// else (CUDA-core M2M, rows are parents) the mode-2 cells by (level, 0);
-// 255 for the rest.
-__global__ void k_m2m_keys(const uint64_t *ckey, const uint8_t *mode, const int *parent, int first, int count,
-                           int level, int dim, int cell0, int child_rows, uint64_t *keys, uint32_t *vals, int out_off) {
+// List keys of the cells of levels 2 .. D, two lists of n: the cells that
+// need L2L (levels >= 3) by (level, class); the M2M rows, with child_rows
+// (tensor-core M2M, rows are children) the children of mode-2 cells by
+// (level, class), else (CUDA-core M2M, rows are parents) the mode-2 cells by
+// (level, 0).  255: in no list.
+__global__ void k_row_keys(const uint64_t *ckey, const uint8_t *needs, const uint8_t *mode, const int *parent,
+                           LevelOffsets lv, int D, int dim, int cell0, int child_rows, int n, uint8_t *keys) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int g = first + i;
-  const bool on = child_rows ? mode[parent[g] - cell0] == 2 : mode[g - cell0] == 2;
-  const uint64_t cls = child_rows ? (ckey[g] & ((1u << dim) - 1)) : 0u;
-  keys[out_off + i] = on ? (((uint64_t)level << dim) | cls) : 255u;
-  vals[out_off + i] = (uint32_t)g;
+  if (i >= n) return;
+  const int g = lv.off[2] + i, d = cell_level(lv, 2, D, g);
+  const int cls = (int)(ckey[g] & ((1u << dim) - 1));
+  keys[i] = d >= 3 && needs[g - cell0] ? (uint8_t)((d << dim) | cls) : (uint8_t)255;
+  const bool row = child_rows ? d >= 3 && mode[parent[g] - cell0] == 2 : mode[g - cell0] == 2;
+  keys[(int64_t)n + i] = row ? (uint8_t)((d << dim) | (child_rows ? cls : 0)) : (uint8_t)255;
 }
 
 struct P2MListArgs {
@@ -1630,16 +1661,6 @@ __global__ void k_leaf_esrc(int leaf_first, int nleaves, int D, int first2, cons
   elev[i] = (uint8_t)(c >= first2 ? lev : 0);
 }
 
-// Sort keys of the cells of one level that need L2L: (level, class), else 255.
-__global__ void k_l2l_keys(const uint64_t *ckey, const uint8_t *needs, int first, int count, int level, int dim,
-                           int cell0, uint64_t *keys, uint32_t *vals, int out_off) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int g = first + i;
-  keys[out_off + i] = needs[g - cell0] ? (((uint64_t)level << dim) | (ckey[g] & ((1u << dim) - 1))) : 255u;
-  vals[out_off + i] = (uint32_t)g;
-}
-
 // ------------------------------------------------------------ separation
 // Offset o = (dx+3) + 7(dy+3) + 49(dz+3) (cells of the box with extents ex):
 // the two cells' radii summed over the distance of their centres exceeds
@@ -1794,35 +1815,28 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   int ntl = 0;
   const int *tl = nullptr, *tl_m2l = nullptr;
   size_t nhb = 0;
+  LevelOffsets lvo{};
+  for (int d = 0; d <= D + 1; ++d) lvo.off[d] = t.level_off[d];
   if (D >= 2) {
     ntl = t.level_off[D] + t.level_count[D] - t.level_off[2];
-    if (!eb.tlist.reserve(ntl) || !eb.tlist_m2l.reserve(ntl) || !eb.cls_count.reserve(512) ||
-        !eb.ckey.reserve(ntl) || !eb.ckey_alt.reserve(ntl) || !eb.ckey_m2l.reserve(ntl) || !eb.cval.reserve(ntl) ||
-        !eb.cval2.reserve(ntl))
+    // lists: every cell (without the shortcuts), then the M2L targets
+    const int nlist = shortcut ? 1 : 2;
+    if (!eb.tlist.reserve((size_t)nlist * ntl) || !eb.lkey.reserve((size_t)2 * ntl) || !eb.cls_count.reserve(512))
       return FMM_ERR_OUT_OF_MEMORY;
-    for (int d = 2; d <= D; ++d)
-      k_class_keys<<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(
-          ws.cell_key, ws.cell_pbeg, ws.cell_pend, ws.cell_parent, ws.cell_coll, ws.cell_child, direct_max,
-          t.level_off[d], t.level_count[d], d, dim, eb.ckey.ptr, eb.ckey_m2l.ptr, eb.cval.ptr,
-          t.level_off[d] - t.level_off[2], adaptive ? ws.aflag : nullptr, cell0);
-    ws.launches += D - 1;
-    CUDA_TRY(cudaMemsetAsync(eb.cls_count.ptr, 0, 512 * sizeof(uint32_t), st));
-    uint64_t *kk = eb.ckey.ptr, *kk2 = eb.ckey_alt.ptr;
-    uint32_t *mv = eb.cval.ptr, *mv2 = (uint32_t *)eb.tlist_m2l.ptr;
-    if (!shortcut) {
-      CUDA_TRY(cudaMemcpyAsync(eb.cval2.ptr, eb.cval.ptr, sizeof(uint32_t) * ntl, cudaMemcpyDeviceToDevice, st));
-      uint32_t *vv = eb.cval.ptr, *vv2 = (uint32_t *)eb.tlist.ptr;
-      radix_sort(ws, kk, vv, kk2, vv2, ntl, 8, st);  // sorted (keys, cells) end in (kk, vv)
-      tl = (const int *)vv;
-      k_class_hist<<<std::min(cdiv(ntl, TPB), 148 * 4), TPB, 0, st>>>(kk, ntl, eb.cls_count.ptr);
-      ws.launches += 1;
-      mv = eb.cval2.ptr;
-    }
-    uint64_t *mk = eb.ckey_m2l.ptr, *mk2 = (kk == eb.ckey.ptr) ? eb.ckey_alt.ptr : eb.ckey.ptr;
-    radix_sort(ws, mk, mv, mk2, mv2, ntl, 8, st);
-    tl_m2l = (const int *)mv;
-    k_class_hist<<<std::min(cdiv(ntl, TPB), 148 * 4), TPB, 0, st>>>(mk, ntl, eb.cls_count.ptr + 256);
+    uint8_t *k_all = shortcut ? nullptr : eb.lkey.ptr, *k_m2l = eb.lkey.ptr + (shortcut ? 0 : ntl);
+    const int cw = ntl < (1 << 20) ? 4 : 32;
+    auto ck_kern = dim == 3 ? (cw == 4 ? k_class_keys<3, 4> : k_class_keys<3, 32>)
+                            : (cw == 4 ? k_class_keys<2, 4> : k_class_keys<2, 32>);
+    ck_kern<<<cdiv(cdiv(ntl, cw) * (int64_t)32, TPB), TPB, 0, st>>>(ws.cell_key, ws.cell_pbeg, ws.cell_pend, ws.cell_parent,
+                                                         ws.cell_coll, ws.cell_child, direct_max, lvo, D, k_all, k_m2l,
+                                                         adaptive ? ws.aflag : nullptr, cell0);
     ws.launches += 1;
+    // (the counts of the M2L list are read from 256 on)
+    CUDA_TRY(cudaMemsetAsync(eb.cls_count.ptr, 0, 512 * sizeof(uint32_t), st));
+    bucket_lists(ws, eb.lkey.ptr, nlist, ntl, lvo.off[2], eb.tlist.ptr, eb.cls_count.ptr + (shortcut ? 256 : 0), st);
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
+    tl = eb.tlist.ptr;
+    tl_m2l = eb.tlist.ptr + (shortcut ? 0 : ntl);
     uint32_t hc[512];
     CUDA_TRY(cudaMemcpyAsync(hc, eb.cls_count.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -1932,7 +1946,8 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
       ws.launches += 1;
     }
     if (nbm > 0) {
-      k_m2l_sources<<<nbm, 256, 0, st>>>(cm, tchunk, eb.m2l_src.ptr, eb.m2l_list.ptr, eb.m2l_nslots.ptr,
+      // few batches: more threads for each, so that the chains of loads overlap
+      k_m2l_sources<<<nbm, nbm < 2 * 148 ? 1024 : 256, 0, st>>>(cm, tchunk, eb.m2l_src.ptr, eb.m2l_list.ptr, eb.m2l_nslots.ptr,
                                          tc ? eb.m2l_tslot.ptr : nullptr, tc ? ws.counters : nullptr,
                                          geometric ? eb.order_p16.ptr : nullptr, geometric ? eb.m2l_w.ptr : nullptr,
                                          ws.counters + 4, lact, msrc, cell0);
@@ -1965,29 +1980,14 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     ws.launches += 2;
     // L2L rows: levels 3..D; M2M rows: children at levels 3..D (tensor
     // cores) or the mode-2 parents at levels 2..D-1
-    const int l3 = t.level_off[3], nl3 = t.level_off[D] + t.level_count[D] - l3;
     const int m_lo = tc ? 3 : 2, m_hi = tc ? D : D - 1;
-    const int m_first = t.level_off[m_lo], nm = t.level_off[m_hi] + t.level_count[m_hi] - m_first;
-    if (!eb.ukey.reserve(4 * (size_t)ntl) || !eb.uval.reserve(4 * (size_t)ntl)) return FMM_ERR_OUT_OF_MEMORY;
-    for (int d = 3; d <= D; ++d)
-      k_l2l_keys<<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(ws.cell_key, needs, t.level_off[d], t.level_count[d], d,
-                                                              dim, cell0, eb.ukey.ptr, eb.uval.ptr, t.level_off[d] - l3);
-    for (int d = m_lo; d <= m_hi; ++d)
-      k_m2m_keys<<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(ws.cell_key, mmode, ws.cell_parent, t.level_off[d],
-                                                              t.level_count[d], d, dim, cell0, tc ? 1 : 0,
-                                                              eb.ukey.ptr + 2 * (size_t)ntl,
-                                                              eb.uval.ptr + 2 * (size_t)ntl, t.level_off[d] - m_first);
-    ws.launches += (D - 2) + (m_hi - m_lo + 1);
-    uint64_t *kk = eb.ukey.ptr, *kk2 = eb.ukey.ptr + ntl;
-    uint32_t *vv = eb.uval.ptr, *vv2 = eb.uval.ptr + ntl;
-    radix_sort(ws, kk, vv, kk2, vv2, nl3, 8, st);
-    uint64_t *mk = eb.ukey.ptr + 2 * (size_t)ntl, *mk2 = eb.ukey.ptr + 3 * (size_t)ntl;
-    uint32_t *mv = eb.uval.ptr + 2 * (size_t)ntl, *mv2 = eb.uval.ptr + 3 * (size_t)ntl;
-    radix_sort(ws, mk, mv, mk2, mv2, nm, 8, st);
+    if (!eb.rows.reserve(2 * (size_t)ntl)) return FMM_ERR_OUT_OF_MEMORY;
+    k_row_keys<<<cdiv(ntl, TPB), TPB, 0, st>>>(ws.cell_key, needs, mmode, ws.cell_parent, lvo, D, dim, cell0,
+                                               tc ? 1 : 0, ntl, eb.lkey.ptr);
+    ws.launches += 1;
     CUDA_TRY(cudaMemsetAsync(eb.cls_count.ptr, 0, 512 * sizeof(uint32_t), st));
-    k_class_hist<<<std::max(1, std::min(cdiv(nl3, TPB), 148 * 4)), TPB, 0, st>>>(kk, nl3, eb.cls_count.ptr);
-    k_class_hist<<<std::max(1, std::min(cdiv(nm, TPB), 148 * 4)), TPB, 0, st>>>(mk, nm, eb.cls_count.ptr + 256);
-    ws.launches += 2;
+    bucket_lists(ws, eb.lkey.ptr, 2, ntl, first2, eb.rows.ptr, eb.cls_count.ptr, st);
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
     uint32_t hc[512];
     CUDA_TRY(cudaMemcpyAsync(hc, eb.cls_count.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
@@ -2023,8 +2023,8 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     if (!eb.batches2.reserve(nb2 + 1)) return FMM_ERR_OUT_OF_MEMORY;
     if (nb2)
       CUDA_TRY(cudaMemcpyAsync(eb.batches2.ptr, hb2, nb2 * sizeof(int4), cudaMemcpyHostToDevice, st));
-    tl2 = (const int *)vv;
-    tlm = (const int *)mv;
+    tl2 = eb.rows.ptr;
+    tlm = eb.rows.ptr + ntl;
     b2 = eb.batches2.ptr;
     if (!eb.esrc.reserve((size_t)t.level_count[D]) || !eb.elev.reserve((size_t)t.level_count[D]))
       return FMM_ERR_OUT_OF_MEMORY;

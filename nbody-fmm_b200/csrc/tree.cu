@@ -252,6 +252,102 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
   }
 }
 
+// ------------------------------------------------------------ bucket lists
+// List y's block sums: items per (bucket, tile); key 255 is in no bucket.
+__global__ void __launch_bounds__(RS_BLOCK) k_bucket_hist(const uint8_t *keys, int64_t n, uint32_t *hist, int nb,
+                                                          bool by_tile, uint32_t *counts) {
+  __shared__ uint32_t h[256];
+  const int y = blockIdx.y, tid = threadIdx.x;
+  h[tid] = 0;
+  __syncthreads();
+  const int64_t base = (int64_t)blockIdx.x * RS_TILE;
+  for (int r = 0; r < RS_ROUNDS; ++r) {
+    const int64_t i = base + (int64_t)r * RS_BLOCK + tid;
+    const uint32_t d = i < n ? keys[(int64_t)y * n + i] : 255u;
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    if (d != 255u && (tid & 31) == __ffs(peers) - 1) atomicAdd(&h[d], (uint32_t)__popc(peers));
+  }
+  __syncthreads();
+  if (by_tile) hist[((int64_t)y * nb + blockIdx.x) * 256 + tid] = h[tid];
+  else hist[((int64_t)y * 256 + tid) * nb + blockIdx.x] = h[tid];
+  if (h[tid]) atomicAdd(&counts[y * 256 + tid], h[tid]);
+}
+
+// Stable scatter: the items of each tile in input order to their bucket's
+// places, ranked by (round, warp, lane).  offs: the exclusive scan of the
+// [list][bucket][tile] sums, or with by_tile the [list][tile][256] sums.
+__global__ void __launch_bounds__(RS_BLOCK) k_bucket_scatter(const uint8_t *keys, int64_t n, const uint32_t *offs,
+                                                             int nb, bool by_tile, int first, int *out) {
+  __shared__ uint32_t s_at[256], s_warp[RS_BLOCK / 32];
+  __shared__ uint32_t s_cnt[RS_BLOCK / 32][256];
+  const int y = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (by_tile) {
+    uint32_t all = 0, before = 0, total;
+    for (int b = 0; b < nb; ++b) {
+      const uint32_t v = offs[((int64_t)y * nb + b) * 256 + tid];
+      if (b == (int)blockIdx.x) before = all;
+      all += v;
+    }
+    s_at[tid] = block_excl_scan(all, s_warp, total) + before;
+  } else {
+    s_at[tid] = offs[((int64_t)y * 256 + tid) * nb + blockIdx.x] - offs[(int64_t)y * 256 * nb];
+  }
+  out += (int64_t)y * n;
+  // a warp takes 32 RS_ROUNDS consecutive items: one count of its items per
+  // bucket, then the places of its rounds one after another
+  const int64_t base = (int64_t)blockIdx.x * RS_TILE + (int64_t)warp * 32 * RS_ROUNDS;
+  uint32_t dig[RS_ROUNDS];
+  uint32_t any = 0;
+  for (int b = lane; b < 256; b += 32) s_cnt[warp][b] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < RS_ROUNDS; ++r) {
+    const int64_t i = base + r * 32 + lane;
+    dig[r] = i < n ? keys[(int64_t)y * n + i] : 255u;
+    any |= dig[r] != 255u;
+    const uint32_t peers = __match_any_sync(0xffffffffu, dig[r]);
+    if (dig[r] != 255u && lane == __ffs(peers) - 1) s_cnt[warp][dig[r]] += (uint32_t)__popc(peers);
+    __syncwarp();
+  }
+  if (!__syncthreads_or((int)any)) return;
+  uint32_t run = s_at[tid];
+  for (int w = 0; w < RS_BLOCK / 32; ++w) {
+    const uint32_t c = s_cnt[w][tid];
+    s_cnt[w][tid] = run;  // where the warp's items of this bucket start
+    run += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < RS_ROUNDS; ++r) {
+    const uint32_t d = dig[r];
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
+    const uint32_t at = d != 255u ? s_cnt[warp][d] : 0u;
+    __syncwarp();
+    if (d != 255u) {
+      out[at + __popc(peers & ((1u << lane) - 1u))] = first + (int)(base + r * 32 + lane);
+      if (lane == __ffs(peers) - 1) s_cnt[warp][d] = at + (uint32_t)__popc(peers);
+    }
+    __syncwarp();
+  }
+}
+
+// Lists of the cells first .. first + n by their 8-bit key, nlist lists from
+// nlist x n keys: list y is out[y n ..), bucket after bucket (255 left out),
+// ascending inside a bucket; counts[y * 256 + b] (zeroed by the caller) the
+// size of its bucket b.  The keys are bytes and most cells are in no bucket,
+// so this reads a byte per cell where a sort of (key, cell) pairs moved 32.
+void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int first, int *out, uint32_t *counts,
+                  cudaStream_t st) {
+  const int nb = (int)std::max<int64_t>(1, (n + RS_TILE - 1) / RS_TILE);
+  const bool by_tile = nb <= RS_FUSED_TILES;
+  uint32_t *hist = ws.radix_hist(nlist * nb);
+  const dim3 grid(nb, nlist);
+  k_bucket_hist<<<grid, RS_BLOCK, 0, st>>>(keys, n, hist, nb, by_tile, counts);
+  if (!by_tile) exclusive_scan(ws, hist, hist, (int64_t)256 * nb * nlist, nullptr, st);
+  k_bucket_scatter<<<grid, RS_BLOCK, 0, st>>>(keys, n, hist, nb, by_tile, first, out);
+  ws.launches += 2;
+}
+
 // ------------------------------------------------------------ tree kernels
 // AABB (tree.cpp:20-30) plus a finiteness check of positions and masses.
 // Every block writes its box to part[block][6]; the last one to finish (a
@@ -442,10 +538,6 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_level_scan(uint32_t *blockcnt, i
     carry += tot;
   }
 }
-
-struct LevelOffsets {
-  int off[LV_MAX + 1];  // first cell of each level 0 .. D, then the end
-};
 
 // The cells of all levels 0 .. D from the sorted Dmax keys and the scanned
 // tile counts: cell r of a level is the r-th particle that starts one there

@@ -152,6 +152,10 @@ struct Workspace {
   }
 };
 
+struct LevelOffsets {
+  int off[FMM_MAX_DEPTH + 2];  // first cell of each level 0 .. D, then the end
+};
+
 // Result of a tree build.  Cell indices are absolute into the Workspace cell
 // arrays; level d holds cells [level_off[d], level_off[d] + level_count[d]),
 // levels are contiguous from the root, and every cell covers the contiguous
@@ -175,6 +179,8 @@ void exclusive_scan(Workspace &ws, const uint32_t *in, uint32_t *out, int64_t n,
                     cudaStream_t st);
 void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
                 int bits, cudaStream_t st);
+void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int first, int *out, uint32_t *counts,
+                  cudaStream_t st);
 int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d_mass, int64_t n, int dim,
                int threshold, cudaStream_t st, int adaptive_leaf = 0);
 // Adaptive-target flags of every cell of a built tree into flag[0 .. n_cells)
