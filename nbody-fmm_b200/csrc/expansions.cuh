@@ -16,6 +16,7 @@ struct OpTables {
   int n_m2l = 0, off_m2m = 0, off_l2l = 0, n_slots = 0;
   DevBuf<float> tab;        // n_slots * K * KP
   DevBuf<double> scratch;   // FP64 staging
+  uint16_t *img = nullptr, *img96 = nullptr;  // tensor cores: the images of this pass
   DevBuf<double> tab64;     // FP64 copy of the 3D M2L operators (training-pair probe only)
 };
 
@@ -87,8 +88,12 @@ struct PassGeom {
   double lo[3], ext[3], emax;
 };
 
+// Builds the operators of a pass into ops (FP32 matrices; want64: FP64 M2L
+// matrices too), or with `images` set (tensor cores) as BF16 split images in
+// that buffer, with96: also those of the M2L operators' first 96 rows and
+// columns.
 int build_op_tables(OpTables &ops, int dim, int p, int depth, const PassGeom &g, cudaStream_t st, int64_t &launches,
-                    bool want64 = false);
+                    bool want64, DevBuf<uint16_t> *images, bool with96);
 
 // Learned-order settings of a pass, and the training-pair collection hook.
 struct OrderOpts {

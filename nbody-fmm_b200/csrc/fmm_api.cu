@@ -233,7 +233,12 @@ static int pass(fmm_ctx *c, int64_t n, const double *d_pos, const double *d_mass
     g.ext[d] = d < dim ? c->tree.hi[d] - c->tree.lo[d] : 0.0;
     g.emax = std::max(g.emax, g.ext[d]);
   }
-  rc = build_op_tables(c->ops, dim, c->cfg.p, c->tree.depth, g, st, c->ws.launches, want64);
+  // variable orders at a full width of 176 (p = 12): narrow M2L tiles take a 96-wide kernel
+  const bool tc = c->cfg.m2l_mode == FMM_M2L_TC;
+  const bool var_order = oo.mode == FMM_ORDER_GEOMETRIC || (dim == 3 && oo.mode == FMM_ORDER_LEARNED && oo.params);
+  const int K = dim == 3 ? (c->cfg.p + 1) * (c->cfg.p + 1) : 2 * c->cfg.p + 1;
+  rc = build_op_tables(c->ops, dim, c->cfg.p, c->tree.depth, g, st, c->ws.launches, want64,
+                       tc ? &c->eb.tc_img : nullptr, tc && var_order && K > 160);
   if (rc) return rc;
   const double jr = c->stats.judge_rel_l2;
   const int64_t fb = c->stats.order_fallbacks;

@@ -50,8 +50,6 @@
 // mbarrier gives up after about a second; the kernel then flags the device
 // error word, drains its copies (again with a limit), releases its TMEM and
 // returns.
-#include <cuda_bf16.h>
-
 #include <algorithm>
 #include <mutex>
 
@@ -71,44 +69,17 @@ __device__ inline uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) 
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// The three-part split of two values at once (round to nearest); each 32-bit
-// word holds (a, b) as BF16 with a in the low half.
-__device__ inline uint32_t bf2_pack(float a, float b) {
-  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t *>(&t);
-}
-__device__ inline void split3x2(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
-  h = bf2_pack(a, b);
-  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
-  m = bf2_pack(ra, rb);
-  const float sa = ra - __uint_as_float(m << 16), sb = rb - __uint_as_float(m & 0xffff0000u);
-  l = bf2_pack(sa, sb);
-}
-
-// Operator images: for each table slot and split s, B = T^T (n: output,
-// k: input), its first W rows and columns; element (n, k) at
-// ((k/8) * (W/8) + n/8) * 64 + (n%8) * 8 + k%8, so that the first w rows (k)
-// are a contiguous prefix.  A thread takes 8 consecutive k of one n: reads
-// coalesced over n, 16-byte stores.
+// A thread takes 8 consecutive k of one n: reads coalesced over n, 16-byte
+// stores.
 __global__ void k_tc_images(const float *tab, int K, int KP, int W, uint16_t *img) {
-  const int slot = blockIdx.x;
-  const size_t bsplit = (size_t)W * W;
-  const float *T = tab + (size_t)slot * K * KP;
-  uint16_t *out = img + (size_t)slot * 3 * bsplit;
+  const float *T = tab + (size_t)blockIdx.x * K * KP;
+  uint16_t *out = img + (size_t)blockIdx.x * 3 * W * W;
   for (int e = threadIdx.x; e < W * (W / 8); e += blockDim.x) {
     const int n = e % W, k0 = (e / W) * 8;
-    uint32_t h[4], m[4], l[4];
+    float v[8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int k = k0 + 2 * q;
-      const float v0 = (n < K && k < K) ? T[(size_t)k * KP + n] : 0.f;
-      const float v1 = (n < K && k + 1 < K) ? T[(size_t)(k + 1) * KP + n] : 0.f;
-      split3x2(v0, v1, h[q], m[q], l[q]);
-    }
-    const size_t idx = ((size_t)(k0 / 8) * (W / 8) + n / 8) * 64 + (n % 8) * 8;
-    *(uint4 *)(out + idx) = make_uint4(h[0], h[1], h[2], h[3]);
-    *(uint4 *)(out + bsplit + idx) = make_uint4(m[0], m[1], m[2], m[3]);
-    *(uint4 *)(out + 2 * bsplit + idx) = make_uint4(l[0], l[1], l[2], l[3]);
+    for (int q = 0; q < 8; ++q) v[q] = (n < K && k0 + q < K) ? T[(size_t)(k0 + q) * KP + n] : 0.f;
+    tc_store_image(out, W, n, k0, v);
   }
 }
 

@@ -1,5 +1,7 @@
 // Translations (M2L, M2M, L2L) on the 5th-generation tensor cores (tcgen05).
 #pragma once
+#include <cuda_bf16.h>
+
 #include "tree.cuh"
 
 namespace fmm {
@@ -43,7 +45,35 @@ __host__ __device__ constexpr int tc_kpart(int P16) {
   return P16 <= 48 ? P16 : P16 <= 128 ? ((P16 / 16 + 1) / 2) * 16 : ((P16 / 16 + 2) / 3) * 16;
 }
 
-// The images of the operators' first W rows and columns (W a multiple of 16).
+// The three-part BF16 split of two values at once (round to nearest); each
+// 32-bit word holds (a, b) with a in the low half.
+__device__ inline uint32_t bf2_pack(float a, float b) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&t);
+}
+__device__ inline void split3x2(float a, float b, uint32_t &h, uint32_t &m, uint32_t &l) {
+  h = bf2_pack(a, b);
+  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);
+  m = bf2_pack(ra, rb);
+  const float sa = ra - __uint_as_float(m << 16), sb = rb - __uint_as_float(m & 0xffff0000u);
+  l = bf2_pack(sa, sb);
+}
+
+// Operator image of width W: for each split s, B = T^T (n: output, k: input)
+// of the first W rows and columns, W^2 values; element (n, k) at
+// ((k/8) * (W/8) + n/8) * 64 + (n%8) * 8 + k%8, so that the first w rows (k)
+// are a contiguous prefix.  Stores the inputs k0 .. k0 + 7 of output n.
+__device__ inline void tc_store_image(uint16_t *img, int W, int n, int k0, const float *v) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) split3x2(v[2 * q], v[2 * q + 1], h[q], m[q], l[q]);
+  const size_t bsplit = (size_t)W * W, at = ((size_t)(k0 / 8) * (W / 8) + n / 8) * 64 + (n % 8) * 8;
+  *(uint4 *)(img + at) = make_uint4(h[0], h[1], h[2], h[3]);
+  *(uint4 *)(img + bsplit + at) = make_uint4(m[0], m[1], m[2], m[3]);
+  *(uint4 *)(img + 2 * bsplit + at) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// The images of width W of FP32 matrices tab (K x KP each).
 int tc_build_images(const float *tab, int n_slots, int K, int KP, int W, uint16_t *img, cudaStream_t st,
                     int64_t &launches);
 // Launches one translation pass over nb batches; `work` is a zeroed device

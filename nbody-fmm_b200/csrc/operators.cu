@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "expansions.cuh"
+#include "m2l_tc.cuh"
 
 namespace fmm {
 
@@ -40,14 +41,19 @@ __device__ inline cd hget(const cd *X, int n, int m) {
   return (m & 1) ? cd{-v.re, -v.im} : v;
 }
 
+// The harmonics of degree up to p by a block: degree after degree, thread m
+// takes order m (a single thread's chain of 325 entries at p = 12 was most of
+// the operators' build time on small systems).
 __device__ void regular_s(int p, const double *r, cd *R) {
-  double x = r[0], y = r[1], z = r[2], r2 = x * x + y * y + z * z;
-  R[0] = {1.0, 0.0};
+  const double x = r[0], y = r[1], z = r[2], r2 = x * x + y * y + z * z;
+  const int m = threadIdx.x;
+  if (m == 0) R[0] = {1.0, 0.0};
   for (int l = 1; l <= p; ++l) {
-    cd d = R[hid(l - 1, l - 1)];
-    cd v = cmul({-x, -y}, d);
-    R[hid(l, l)] = cscale(v, 1.0 / (2.0 * l));
-    for (int m = 0; m < l; ++m) {
+    __syncthreads();
+    if (m == l) {
+      cd v = cmul({-x, -y}, R[hid(l - 1, l - 1)]);
+      R[hid(l, l)] = cscale(v, 1.0 / (2.0 * l));
+    } else if (m < l) {
       cd a = cscale(R[hid(l - 1, m)], (2.0 * l - 1.0) * z);
       if (m <= l - 2) a = csub(a, cscale(R[hid(l - 2, m)], r2));
       R[hid(l, m)] = cscale(a, 1.0 / (double)(l * l - m * m));
@@ -56,12 +62,14 @@ __device__ void regular_s(int p, const double *r, cd *R) {
 }
 
 __device__ void irregular_s(int p, const double *r, cd *S) {
-  double x = r[0], y = r[1], z = r[2], r2 = x * x + y * y + z * z, ir2 = 1.0 / r2;
-  S[0] = {1.0 / sqrt(r2), 0.0};
+  const double x = r[0], y = r[1], z = r[2], r2 = x * x + y * y + z * z, ir2 = 1.0 / r2;
+  const int m = threadIdx.x;
+  if (m == 0) S[0] = {1.0 / sqrt(r2), 0.0};
   for (int l = 1; l <= p; ++l) {
-    cd d = S[hid(l - 1, l - 1)];
-    S[hid(l, l)] = cscale(cmul({x, y}, d), -(2.0 * l - 1.0) * ir2);
-    for (int m = 0; m < l; ++m) {
+    __syncthreads();
+    if (m == l) {
+      S[hid(l, l)] = cscale(cmul({x, y}, S[hid(l - 1, l - 1)]), -(2.0 * l - 1.0) * ir2);
+    } else if (m < l) {
       cd a = cscale(S[hid(l - 1, m)], (2.0 * l - 1.0) * z);
       if (m <= l - 2) a = csub(a, cscale(S[hid(l - 2, m)], (double)((l - 1 - m) * (l - 1 + m))));
       S[hid(l, m)] = cscale(a, ir2);
@@ -101,10 +109,17 @@ __device__ inline cd op_coef(int kind, const cd *H, int k, int l, int n, int mp)
   }
 }
 
-// One block per slot.  Builds K x KP (input-major) FP32 matrix.
-__global__ void k_build_ops3d(float *tab, double *tab64, int p, int K, int KP, int n_m2l, double ax, double ay,
-                              double az) {
+// One block per slot.  Builds the operator as whichever of these is not null:
+// tab, K x KP (input-major) FP32; tab64, the same in FP64 (M2L slots); img,
+// its BF16 split image of width W; img96 (M2L slots), the image of its first
+// 96 rows and columns (k_tc_images' layout).  A thread computes 8 consecutive
+// inputs of one output, so that the matrices are stored coalesced and the
+// images 16 bytes at a time, and the FP32 matrices are not written where only
+// the images are read (46 MB each way at p = 12).
+__global__ void __launch_bounds__(256) k_build_ops3d(float *tab, double *tab64, uint16_t *img, int W, uint16_t *img96,
+                                                     int p, int K, int KP, int n_m2l, double ax, double ay, double az) {
   extern __shared__ cd H[];
+  __shared__ int s_dec[(FMM_MAX_P + 1) * (FMM_MAX_P + 1)];  // n | m << 8 | imaginary << 16 of each real index
   const int slot = blockIdx.x;
   int kind;
   double r[3];
@@ -128,33 +143,51 @@ __global__ void k_build_ops3d(float *tab, double *tab64, int p, int K, int KP, i
     r[1] = (2 * ((c >> 1) & 1) - 1) * ay * 0.25;
     r[2] = (2 * ((c >> 2) & 1) - 1) * az * 0.25;
   }
-  if (threadIdx.x == 0 && !zero) {
+  for (int i = threadIdx.x; i < K; i += blockDim.x) {
+    int n, m, im;
+    dec_idx(i, n, m, im);
+    s_dec[i] = n | m << 8 | im << 16;
+  }
+  if (!zero) {
     if (kind == 0) irregular_s(2 * p, r, H);
     else regular_s(p, r, H);
   }
   __syncthreads();
-  float *T = tab + (size_t)slot * K * KP;
-  for (int e = threadIdx.x; e < K * KP; e += blockDim.x) {
-    int in = e / KP, out = e % KP;
-    double val = 0.0;
-    if (!zero && out < K) {
-      int k, l, po, n, mp, pi;
-      dec_idx(out, k, l, po);
-      dec_idx(in, n, mp, pi);
-      if (mp == 0) {
-        cd A = op_coef(kind, H, k, l, n, 0);
-        val = po ? A.im : A.re;
-      } else {
-        cd A = op_coef(kind, H, k, l, n, mp);
-        cd B = op_coef(kind, H, k, l, n, -mp);
-        if (mp & 1) B = {-B.re, -B.im};
-        cd S = cadd(A, B), Dd = csub(A, B);
-        if (pi == 0) val = po ? S.im : S.re;
-        else val = po ? Dd.re : -Dd.im;
+  const size_t bsplit = (size_t)W * W;
+  uint16_t *im_w = img ? img + (size_t)slot * 3 * bsplit : nullptr;
+  uint16_t *im_96 = img96 && slot < n_m2l ? img96 + (size_t)slot * 3 * 96 * 96 : nullptr;
+  const bool f64 = tab64 && slot < n_m2l;
+  const int nout = max(tab || f64 ? KP : 0, img ? W : 0), nin = img ? W : (K + 7) & ~7;
+  for (int e = threadIdx.x; e < nout * (nin >> 3); e += blockDim.x) {
+    const int out = e % nout, in0 = (e / nout) * 8;
+    const int od = out < K ? s_dec[out] : 0, k = od & 255, l = (od >> 8) & 255, po = od >> 16;
+    float v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int in = in0 + q;
+      double val = 0.0;
+      if (!zero && out < K && in < K) {
+        const int id = s_dec[in], n = id & 255, mp = (id >> 8) & 255, pi = id >> 16;
+        if (mp == 0) {
+          cd A = op_coef(kind, H, k, l, n, 0);
+          val = po ? A.im : A.re;
+        } else {
+          cd A = op_coef(kind, H, k, l, n, mp);
+          cd B = op_coef(kind, H, k, l, n, -mp);
+          if (mp & 1) B = {-B.re, -B.im};
+          cd S = cadd(A, B), Dd = csub(A, B);
+          if (pi == 0) val = po ? S.im : S.re;
+          else val = po ? Dd.re : -Dd.im;
+        }
+      }
+      v[q] = (float)val;
+      if (in < K && out < KP) {
+        if (tab) tab[((size_t)slot * K + in) * KP + out] = v[q];
+        if (f64) tab64[((size_t)slot * K + in) * KP + out] = val;
       }
     }
-    T[e] = (float)val;
-    if (tab64 && slot < n_m2l) tab64[(size_t)slot * K * KP + e] = val;
+    if (im_w && out < W) tc_store_image(im_w, W, out, in0, v);
+    if (im_96 && out < 96 && in0 < 96) tc_store_image(im_96, 96, out, in0, v);
   }
 }
 
@@ -256,7 +289,7 @@ __global__ void k_build_ops2d(float *tab, int p, int K, int KP, int n_m2l, doubl
 }
 
 int build_op_tables(OpTables &ops, int dim, int p, int depth, const PassGeom &g, cudaStream_t st, int64_t &launches,
-                    bool want64) {
+                    bool want64, DevBuf<uint16_t> *images, bool with96) {
   int K = dim == 3 ? (p + 1) * (p + 1) : 2 * p + 1;
   int KP = 32 * ((K + 31) / 32);
   int KS = (K + 7) & ~7;  // rows of M and L start on 32-byte sectors (the 256-bit row loads of k_tc_translate)
@@ -269,7 +302,18 @@ int build_op_tables(OpTables &ops, int dim, int p, int depth, const PassGeom &g,
   ops.off_m2m = ops.n_m2l;
   ops.off_l2l = ops.n_m2l + (1 << dim);
   ops.n_slots = ops.n_m2l + 2 * (1 << dim);
-  if (!ops.tab.reserve((size_t)ops.n_slots * K * KP)) return FMM_ERR_OUT_OF_MEMORY;
+  ops.img = ops.img96 = nullptr;
+  if (depth < 2) return FMM_OK;  // no translations
+  const int W = (K + 15) & ~15;
+  if (images) {
+    const size_t nimg = (size_t)ops.n_slots * 3 * W * W;
+    if (!images->reserve(nimg + (with96 ? (size_t)ops.n_m2l * 3 * 96 * 96 : 0))) return FMM_ERR_OUT_OF_MEMORY;
+    ops.img = images->ptr;
+    ops.img96 = with96 ? images->ptr + nimg : nullptr;
+  }
+  // the tensor cores read the images only; the 2D images are formed from the matrices
+  const bool mats = !images || dim == 2;
+  if (mats && !ops.tab.reserve((size_t)ops.n_slots * K * KP)) return FMM_ERR_OUT_OF_MEMORY;
   double emax = g.emax > 0 ? g.emax : 1.0;
   double a[3] = {g.ext[0] / emax, g.ext[1] / emax, dim == 3 ? g.ext[2] / emax : 0.0};
   if (dim == 3) {
@@ -279,12 +323,14 @@ int build_op_tables(OpTables &ops, int dim, int p, int depth, const PassGeom &g,
       if (!ops.tab64.reserve((size_t)ops.n_m2l * K * KP)) return FMM_ERR_OUT_OF_MEMORY;
       t64 = ops.tab64.ptr;
     }
-    k_build_ops3d<<<ops.n_slots, 256, sh, st>>>(ops.tab.ptr, t64, p, K, KP, ops.n_m2l, a[0], a[1], a[2]);
+    k_build_ops3d<<<ops.n_slots, 256, sh, st>>>(mats ? ops.tab.ptr : nullptr, t64, ops.img, W, ops.img96, p, K, KP,
+                                               ops.n_m2l, a[0], a[1], a[2]);
   } else {
     k_build_ops2d<<<ops.n_slots, 256, 0, st>>>(ops.tab.ptr, p, K, KP, ops.n_m2l, a[0], a[1], std::log(emax));
   }
   launches += 1;
-  return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+  if (cudaGetLastError() != cudaSuccess) return FMM_ERR_CUDA;
+  return images && dim == 2 ? tc_build_images(ops.tab.ptr, ops.n_slots, K, KP, W, ops.img, st, launches) : FMM_OK;
 }
 
 }  // namespace fmm

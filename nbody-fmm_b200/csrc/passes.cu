@@ -1763,24 +1763,12 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   const int P16 = (ops.K + 15) & ~15;
   const bool tc = m2l_mode == FMM_M2L_TC && P16 <= TC_MAX_P16;
   const int tchunk = tc ? 128 : CT_TGT;
-  // with variable orders at P16 = 176, M2L tiles up to 96 wide run in a kernel of their own
-  const bool split96 = tc && P16 == 176 && (order.mode == FMM_ORDER_GEOMETRIC ||
-                                            (dim == 3 && order.mode == FMM_ORDER_LEARNED && order.params));
+  const bool split96 = ops.img96 != nullptr;  // M2L tiles up to 96 wide run in a kernel of their own
   int tc_k = 0;  // tensor-core launches so far (work counter index)
-  uint16_t *img96 = nullptr;  // the M2L operators' first 96 rows and columns
   if (tc && D >= 2) {
-    const size_t nimg = (size_t)ops.n_slots * 3 * P16 * P16;
-    if (!eb.tc_img.reserve(nimg + (split96 ? (size_t)ops.n_m2l * 3 * 96 * 96 : 0)) ||
-        !eb.tc_work.reserve(TC_MAX_LAUNCHES))
-      return FMM_ERR_OUT_OF_MEMORY;
+    if (!eb.tc_work.reserve(TC_MAX_LAUNCHES)) return FMM_ERR_OUT_OF_MEMORY;
     if (2 * D + 2 > TC_MAX_LAUNCHES) return FMM_ERR_UNSUPPORTED;
     CUDA_TRY(cudaMemsetAsync(eb.tc_work.ptr, 0, TC_MAX_LAUNCHES * sizeof(unsigned int), st));
-    int rc = tc_build_images(ops.tab.ptr, ops.n_slots, ops.K, ops.KP, P16, eb.tc_img.ptr, st, ws.launches);
-    if (!rc && split96) {
-      img96 = eb.tc_img.ptr + nimg;
-      rc = tc_build_images(ops.tab.ptr, ops.n_m2l, ops.K, ops.KP, 96, img96, st, ws.launches);
-    }
-    if (rc) return rc;
   }
   const double emax = g.emax > 0 ? g.emax : 1.0;
   const double sD = std::ldexp(emax, -D);
@@ -1901,7 +1889,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   ta.cchild = ws.cell_child;
   ta.cparent = ws.cell_parent;
   ta.nchild = 1 << dim;
-  ta.bimg = eb.tc_img.ptr;
+  ta.bimg = ops.img;
   ta.cell0 = cell0;
   ta.K = ops.K;
   ta.KS = KS;
@@ -2188,7 +2176,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
         if (!rc) {
           TcArgs lo = t2;
           lo.P16 = 96;
-          lo.bimg = img96;
+          lo.bimg = ops.img96;
           lo.slot_list = lo_s;
           lo.tslot_list = lo_t;
           lo.slot_p16 = lo_w;
