@@ -2,76 +2,114 @@
 // and the drop-in for NaiveUpdate::update (naive_update.cpp:9-35).
 // Targets are split over blocks and sources over a second grid dimension;
 // partial sums meet through FP64 atomics.
+#include <algorithm>
+
 #include "direct.cuh"
 
 namespace fmm {
 
-static constexpr int DS_THREADS = 256;
+static constexpr int DS_THREADS = 256, DS_R = 2, DS_TARGETS = DS_THREADS * DS_R;
 
-__global__ void k_direct(const double *pos, const double *mass, int64_t n, const int64_t *targets, int64_t nt,
-                         int dim, double eps2, int soft_mode, int64_t chunk, double G, double *acc, double *pot) {
-  __shared__ double4 sp[DS_THREADS];
-  const int64_t ti = (int64_t)blockIdx.x * DS_THREADS + threadIdx.x;
-  const bool act = ti < nt;
-  const int64_t i = act ? (targets ? targets[ti] : ti) : 0;
-  double xi = 0, yi = 0, zi = 0;
-  if (act) {
-    xi = pos[i * dim];
-    yi = pos[i * dim + 1];
-    zi = dim == 3 ? pos[i * dim + 2] : 0.0;
-  }
-  double ax = 0, ay = 0, az = 0, ph = 0;
-  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-  for (int64_t jb = j0; jb < j1; jb += DS_THREADS) {
-    int64_t j = jb + threadIdx.x;
-    if (j < j1) {
-      sp[threadIdx.x] = make_double4(pos[j * dim], pos[j * dim + 1], dim == 3 ? pos[j * dim + 2] : 0.0, mass[j]);
+// One pair: f = the factor of -d in the force, pw = the potential term.
+//
+// Bound by the FP64 pipe (two issue cycles per warp instruction), so the
+// divisions and square roots count: NaiveUpdate's m / ((r^2 + 1e-4) r) is one
+// reciprocal square root, of r^2 (r^2 + 1e-4)^2, while that product stays
+// well inside the FP64 range (r^2 in [2^-300, 2^300), tested on the exponent
+// bits; outside, the two divisions and the square root), and nothing is
+// computed for a potential that is not asked for.
+template <int DIM, int SOFT, bool POT>
+__device__ __forceinline__ void direct_pair(double r2, double w, double eps2, double &f, double &pw) {
+  if (DIM == 3) {
+    if (SOFT == FMM_SOFT_NAIVE_REF) {
+      const double s = r2 + 1.0e-4;
+      const unsigned ex = (unsigned)__double2hiint(r2) >> 20;
+      if (ex - 723u < 600u) {
+        f = w * rsqrt(r2 * s * s);
+        if (POT) pw = f * s;
+      } else {
+        const double r = sqrt(r2);
+        f = w / (s * r);
+        if (POT) pw = w / r;
+      }
     } else {
-      sp[threadIdx.x] = make_double4(0, 0, 0, 0);
+      const double ir = rsqrt(r2 + eps2);
+      pw = w * ir;
+      f = pw * ir * ir;
     }
-    __syncthreads();
-    const int cnt = (int)min((int64_t)DS_THREADS, j1 - jb);
-    if (act) {
-      for (int k = 0; k < cnt; ++k) {
-        if (jb + k == i) continue;
-        double4 q = sp[k];
-        double dx = xi - q.x, dy = yi - q.y, dz = zi - q.z;
-        double r2 = dx * dx + dy * dy + dz * dz;
-        double f, pw;
-        if (dim == 3) {
-          if (soft_mode == FMM_SOFT_NAIVE_REF) {
-            double r = sqrt(r2);
-            f = q.w / ((r2 + 1.0e-4) * r);
-            pw = q.w / r;
-          } else {
-            double ir = rsqrt(r2 + eps2);
-            pw = q.w * ir;
-            f = pw * ir * ir;
-          }
-        } else {
-          double rr = soft_mode == FMM_SOFT_NAIVE_REF ? r2 + 1.0e-4 : r2 + eps2;
-          f = q.w / rr;
-          pw = -0.5 * q.w * log(rr);
-        }
-        ax -= f * dx;
-        ay -= f * dy;
-        az -= f * dz;
-        ph += pw;
+  } else {
+    const double rr = SOFT == FMM_SOFT_NAIVE_REF ? r2 + 1.0e-4 : r2 + eps2;
+    f = w / rr;
+    if (POT) pw = -0.5 * w * log(rr);
+  }
+}
+
+// A thread sums DS_R targets (DS_THREADS apart) over the block's share of the
+// sources, staged DS_THREADS at a time: two independent chains to fill the
+// FP64 pipe's latency, one shared load for both.  The test for j == i runs
+// only in the stages that hold one of the warp's own targets.
+template <int DIM, int SOFT, bool POT>
+__global__ void __launch_bounds__(DS_THREADS) k_direct(const double *pos, const double *mass, int64_t n,
+                                                       const int64_t *targets, int64_t nt, double eps2, int64_t chunk,
+                                                       double G, double *acc, double *pot) {
+  __shared__ double4 sp[DS_THREADS];
+  double x[DS_R][3], a[DS_R][3], ph[DS_R];
+  int64_t me[DS_R];
+#pragma unroll
+  for (int r = 0; r < DS_R; ++r) {
+    const int64_t ti = (int64_t)blockIdx.x * DS_TARGETS + r * DS_THREADS + threadIdx.x;
+    me[r] = ti < nt ? (targets ? targets[ti] : ti) : -1;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x[r][k] = me[r] >= 0 && k < DIM ? pos[me[r] * DIM + k] : 0.0;
+      a[r][k] = 0.0;
+    }
+    ph[r] = 0.0;
+  }
+  const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = min(n, j0 + chunk);
+  auto sum = [&](int cnt, int64_t jb, bool own) {
+#pragma unroll 2
+    for (int k = 0; k < cnt; ++k) {
+      const double4 q = sp[k];
+#pragma unroll
+      for (int r = 0; r < DS_R; ++r) {
+        if (own && jb + k == me[r]) continue;
+        const double dx = x[r][0] - q.x, dy = x[r][1] - q.y, dz = DIM == 3 ? x[r][2] - q.z : 0.0;
+        const double r2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
+        double f, pw = 0.0;
+        direct_pair<DIM, SOFT, POT>(r2, q.w, eps2, f, pw);
+        a[r][0] -= f * dx;
+        a[r][1] -= f * dy;
+        if (DIM == 3) a[r][2] -= f * dz;
+        if (POT) ph[r] += pw;
       }
     }
+  };
+  for (int64_t jb = j0; jb < j1; jb += DS_THREADS) {
+    const int64_t j = jb + threadIdx.x;
+    if (j < j1)
+      sp[threadIdx.x] = make_double4(pos[j * DIM], pos[j * DIM + 1], DIM == 3 ? pos[j * DIM + 2] : 0.0, mass[j]);
+    __syncthreads();
+    const int cnt = (int)min((int64_t)DS_THREADS, j1 - jb);
+    bool mine = false;
+#pragma unroll
+    for (int r = 0; r < DS_R; ++r) mine |= me[r] >= jb && me[r] < jb + DS_THREADS;
+    if (__any_sync(0xffffffffu, mine)) sum(cnt, jb, true);
+    else sum(cnt, jb, false);
     __syncthreads();
   }
-  if (act) {
-    if (gridDim.y == 1) {
-      acc[ti * dim] = G * ax;
-      acc[ti * dim + 1] = G * ay;
-      if (dim == 3) acc[ti * dim + 2] = G * az;
-      if (pot) pot[ti] = G * ph;
-    } else {
-      atomicAdd(&acc[ti * dim], G * ax);
-      atomicAdd(&acc[ti * dim + 1], G * ay);
-      if (dim == 3) atomicAdd(&acc[ti * dim + 2], G * az);
-      if (pot) atomicAdd(&pot[ti], G * ph);
+#pragma unroll
+  for (int r = 0; r < DS_R; ++r) {
+    const int64_t ti = (int64_t)blockIdx.x * DS_TARGETS + r * DS_THREADS + threadIdx.x;
+    if (ti >= nt) continue;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) {
+      if (gridDim.y == 1) acc[ti * DIM + k] = G * a[r][k];
+      else atomicAdd(&acc[ti * DIM + k], G * a[r][k]);
+    }
+    if (POT) {
+      if (gridDim.y == 1) pot[ti] = G * ph[r];
+      else atomicAdd(&pot[ti], G * ph[r]);
     }
   }
 }
@@ -79,16 +117,28 @@ __global__ void k_direct(const double *pos, const double *mass, int64_t n, const
 int direct_sum(const double *d_pos, const double *d_mass, int64_t n, const int64_t *d_targets, int64_t nt, int dim,
                double eps2, int soft_mode, double G, double *d_acc, double *d_pot, cudaStream_t st, int64_t &launches) {
   if (nt <= 0 || n <= 0) return FMM_OK;
-  int bx = (int)((nt + DS_THREADS - 1) / DS_THREADS);
-  // enough source chunks to give ~4 blocks per SM
-  int by = (int)std::max<int64_t>(1, std::min<int64_t>((148 * 4 + bx - 1) / bx, (n + 4095) / 4096));
-  int64_t chunk = (n + by - 1) / by;
+  const int64_t bx = (nt + DS_TARGETS - 1) / DS_TARGETS;
+  // source shares for about eight blocks per SM (three run at a time), of at least two stages
+  const int64_t by = std::max<int64_t>(
+      1, std::min<int64_t>({(148 * 8 + bx - 1) / bx, (n + 2 * DS_THREADS - 1) / (2 * DS_THREADS), 65535}));
+  const int64_t chunk = (n + by - 1) / by;
   if (by > 1) {
     cudaMemsetAsync(d_acc, 0, sizeof(double) * nt * dim, st);
     if (d_pot) cudaMemsetAsync(d_pot, 0, sizeof(double) * nt, st);
   }
-  dim3 grid(bx, by);
-  k_direct<<<grid, DS_THREADS, 0, st>>>(d_pos, d_mass, n, d_targets, nt, dim, eps2, soft_mode, chunk, G, d_acc, d_pot);
+  const dim3 grid((unsigned)bx, (unsigned)by);
+  auto run = [&](auto kern) {
+    kern<<<grid, DS_THREADS, 0, st>>>(d_pos, d_mass, n, d_targets, nt, eps2, chunk, G, d_acc, d_pot);
+  };
+  const bool naive = soft_mode == FMM_SOFT_NAIVE_REF;
+  constexpr int P = FMM_SOFT_PLUMMER, N = FMM_SOFT_NAIVE_REF;
+  if (dim == 3) {
+    if (d_pot) naive ? run(k_direct<3, N, true>) : run(k_direct<3, P, true>);
+    else naive ? run(k_direct<3, N, false>) : run(k_direct<3, P, false>);
+  } else {
+    if (d_pot) naive ? run(k_direct<2, N, true>) : run(k_direct<2, P, true>);
+    else naive ? run(k_direct<2, N, false>) : run(k_direct<2, P, false>);
+  }
   launches += 1;
   return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
