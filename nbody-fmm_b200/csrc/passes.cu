@@ -642,82 +642,207 @@ struct P2PArgs {
   unsigned long long *pair_count;
 };
 
-// One warp per target leaf; the leaf's particles are spread over the lanes
-// (several lanes per particle for small leaves, each taking a share of the
-// sources).  Sources: the leaf itself (j != i) and its existing neighbours
-// (leaf.cpp:118-142).  The direct far field (interaction-list pairs summed
-// particle by particle) has been added into `far` by k_direct_far before
-// this kernel runs; this kernel adds the near field and writes the output.
+// The cell holding position f = f0 + lane of a chunk of 32 concatenated
+// positions, given the cell si0 holding f0; moves si0 to the cell holding
+// f0 + 32.  s_pref[c] is the first position of cell c (every cell non-empty),
+// s_pref[nsrc] the end; lanes past the end get the last cell (the caller masks
+// them).  One shared load per lane, the cell starts inside the chunk as the
+// bits of a warp-wide OR, and a population count (at most 32 cells overlap 32
+// consecutive positions).
+__device__ inline int chunk_cell(const int *s_pref, int nsrc, int f0, int &si0, int lane) {
+  const int c = si0 + lane;
+  const int rel = c < nsrc ? s_pref[c] - f0 : 32;  // lane 0: <= 0
+  const unsigned bit = rel < 32 ? 1u << max(rel, 0) : 0u;
+  const unsigned starts = __reduce_or_sync(0xffffffffu, bit);
+  const int si = si0 + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
+  const int last = __shfl_sync(0xffffffffu, si, 31);
+  si0 = s_pref[last + 1] <= f0 + 32 ? last + 1 : last;
+  return si;
+}
+
+// Lanes per target group for R targets per lane (largest power of two with
+// ceil(nt / R) * Gl <= 32) and the work of the busiest lane per source:
+// rounds x (R pairs of about 19 instructions with the hi + lo differences,
+// and 4 for the two staged loads and the loop) / Gl.
+__device__ inline void colleague_shape(int nt, int R, int &Gl, float &cost) {
+  const int groups = (nt + R - 1) / R;
+  Gl = 1;
+  while (Gl * 2 * groups <= 32) Gl *= 2;
+  const int rounds = (groups + 32 / Gl - 1) / (32 / Gl);
+  cost = (float)rounds * (float)(19 * R + 4) / (float)Gl;
+}
+
+// The register blocking R in 1..4 with the least work on the busiest lane
+// (larger R on ties), and its lanes per target group.
+__device__ inline int best_shape(int nt, int &Gl) {
+  if (nt <= 4) {  // one group of all lanes
+    Gl = 32;
+    return nt;
+  }
+  int bestR = 1;
+  float best = 1e30f;
+#pragma unroll
+  for (int R = 1; R <= 4; ++R) {
+    int G;
+    float c;
+    colleague_shape(nt, R, G, c);
+    if (c <= best) {
+      best = c;
+      bestR = R;
+      Gl = G;
+    }
+  }
+  return bestR;
+}
+
+// A leaf's concatenated neighbours in shared memory: s_pref as in chunk_cell,
+// s_cell[k] = (slot, index delta): the particle at position f is f + delta.
+struct NearList {
+  const int *pref;
+  const int2 *cell;
+  int n, total;
+};
+
+// One warp's targets [tb, tb + nt) of a leaf, R to a lane in groups of Gl
+// lanes that share the sources (every Gl-th of each chunk of 32 staged through
+// shared memory, shifted into the target leaf's frame), then the output.
+template <int R, int DIM, bool POT>
+__device__ bool near_targets(const P2PArgs &a, int tb, int nt, int Gl, const NearList &nl, const float2 *h,
+                             float4 *s_hi, float4 *s_lo, int lane) {
+  const int groups = (nt + R - 1) / R, gpr = 32 / Gl;
+  bool bad = false;
+  for (int g0 = 0; g0 < groups; g0 += gpr) {
+    const int gi = g0 + lane / Gl, sub = lane % Gl;
+    const bool live = gi < groups;
+    float thx[R], tlx[R], thy[R], tly[R], thz[R], tlz[R], ax[R], ay[R], az[R], ph[R];
+    int me[R];  // the target's particle index (the first target's for the lanes' padding)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int ti = gi * R + r;
+      me[r] = tb + (live && ti < nt ? ti : 0);
+      const float4 t = a.part[me[r]], tl = a.part_lo[me[r]];
+      thx[r] = t.x;
+      thy[r] = t.y;
+      thz[r] = t.z;
+      tlx[r] = tl.x;
+      tly[r] = tl.y;
+      tlz[r] = tl.z;
+      ax[r] = ay[r] = az[r] = ph[r] = 0.f;
+    }
+    int si0 = 0;
+    for (int f0 = 0; f0 < nl.total; f0 += 32) {
+      const int f = f0 + lane;
+      const int si = chunk_cell(nl.pref, nl.n, f0, si0, lane);
+      if (f < nl.total) {
+        const int2 c = nl.cell[si];
+        const int j = f + c.y;
+        const float4 q = a.part[j], ql = a.part_lo[j];
+        // + c_s - c_t, a hi + lo multiple of the leaf size per axis
+        const float mx = (float)(c.x % 3 - 1), my = (float)((c.x / 3) % 3 - 1), mz = (float)(c.x / 9 - 1);
+        float sx, sy, sz = 0.f, ex, ey, ez = 0.f;
+        two_sum(q.x, mx * h[0].x, sx, ex);
+        two_sum(q.y, my * h[1].x, sy, ey);
+        if (DIM == 3) two_sum(q.z, mz * h[2].x, sz, ez);
+        s_hi[lane] = make_float4(sx, sy, sz, q.w);
+        s_lo[lane] = make_float4(ex + fmaf(mx, h[0].y, ql.x), ey + fmaf(my, h[1].y, ql.y),
+                                 DIM == 3 ? ez + fmaf(mz, h[2].y, ql.z) : 0.f, __int_as_float(j));
+      }
+      __syncwarp();
+      const int cnt = min(32, nl.total - f0);
+      for (int k = sub; k < cnt; k += Gl) {
+        const float4 q = s_hi[k], ql = s_lo[k];
+        const int j = __float_as_int(ql.w);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (j == me[r]) continue;
+          const float rx = (thx[r] - q.x) + (tlx[r] - ql.x);
+          const float ry = (thy[r] - q.y) + (tly[r] - ql.y);
+          const float rz = DIM == 3 ? (thz[r] - q.z) + (tlz[r] - ql.z) : 0.f;
+          pair_acc<DIM, true, POT>(rx, ry, rz, q.w, a.eps2, ax[r], ay[r], az[r], ph[r]);
+        }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      for (int o = 1; o < Gl; o <<= 1) {
+        ax[r] += __shfl_xor_sync(0xffffffffu, ax[r], o);
+        ay[r] += __shfl_xor_sync(0xffffffffu, ay[r], o);
+        if (DIM == 3) az[r] += __shfl_xor_sync(0xffffffffu, az[r], o);
+        if (POT) ph[r] += __shfl_xor_sync(0xffffffffu, ph[r], o);
+      }
+      const int ti = gi * R + r;
+      if (sub == 0 && live && ti < nt) {
+        const float4 fa = a.far[me[r]];
+        const uint32_t o = a.perm[me[r]];
+        const double vx = a.G * ((double)fa.x + ax[r]), vy = a.G * ((double)fa.y + ay[r]),
+                     vz = DIM == 3 ? a.G * ((double)fa.z + az[r]) : 0.0;
+        a.acc[DIM * (size_t)o] = vx;
+        a.acc[DIM * (size_t)o + 1] = vy;
+        if (DIM == 3) a.acc[3 * (size_t)o + 2] = vz;
+        if (POT) a.pot[o] = a.G * ((double)fa.w + ph[r]);
+        bad |= !(isfinite(vx) && isfinite(vy) && isfinite(vz));
+      }
+    }
+  }
+  return bad;
+}
+
+// One warp per target leaf.  Sources: the leaf itself (j != i) and its
+// existing neighbours (leaf.cpp:118-142), concatenated, so that a warp's lanes
+// stay busy whatever the neighbours' sizes: with 1 to 2 particles per leaf (a
+// Plummer sphere's uniform-depth tree) a loop over the 27 neighbours left 30
+// of 32 lanes idle.  The direct far field (interaction-list pairs summed
+// particle by particle) has been added into `far` by k_direct_far before this
+// kernel runs; this kernel adds the near field and writes the output.
 //
-// Near-field precision: x_i - x_j = (t_i - shift) - s_j with t_i, s_j the
+// Near-field precision: x_i - x_j = t_i - (s_j + shift) with t_i, s_j the
 // offsets from the two leaf centres and shift = c_s - c_t an exact multiple
-// of the leaf size.  Offsets are hi + lo FP32 pairs, the shift is hi + lo
-// from FP64, and (t_hi - shift_hi) is formed error-free (TwoSum), so each
-// difference is rounded once, relative to itself, whatever the separation.
+// of the leaf size.  Offsets and shift are hi + lo FP32 pairs and s_hi +
+// shift_hi is formed error-free (TwoSum), so each difference is rounded once,
+// relative to itself, whatever the separation.
 template <int DIM, bool POT>
-__global__ void k_p2p(P2PArgs a) {
+__global__ void __launch_bounds__(256, 4) k_p2p(P2PArgs a) {
   constexpr int NS = DIM == 3 ? 27 : 9;
-  const int lane = threadIdx.x & 31;
+  __shared__ float4 s_hi_all[8][32], s_lo_all[8][32];
+  __shared__ int2 s_cell_all[8][NS];
+  __shared__ int s_pref_all[8][NS + 1];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int wl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (wl >= a.nleaves) return;
   const int g = a.leaf_first + wl;
   const int tb = a.pbeg[g], nt = a.pend[g] - tb;
-  const int tp = nt < 32 ? nt : 32;
+  const int C = lane < NS ? a.coll[(int64_t)g * NS + lane] : -1;
+  const int cb = C >= 0 ? a.pbeg[C] : 0, cn = C >= 0 ? a.pend[C] - cb : 0;
+  int x = cn;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, cn > 0);
+  if (cn > 0) {
+    const int at = __popc(m & ((1u << lane) - 1u));
+    s_cell_all[wib][at] = make_int2(lane, cb - (x - cn));
+    s_pref_all[wib][at + 1] = x;
+  }
+  if (lane == 0) s_pref_all[wib][0] = 0;
+  __syncwarp();
+  const int total = __shfl_sync(0xffffffffu, x, 31);
+  const NearList nl{s_pref_all[wib], s_cell_all[wib], __popc(m), total};
+  const float2 h[3] = {make_float2((float)a.hx, (float)(a.hx - (double)(float)a.hx)),
+                       make_float2((float)a.hy, (float)(a.hy - (double)(float)a.hy)),
+                       make_float2((float)a.hz, (float)(a.hz - (double)(float)a.hz))};
   int Gl = 1;
-  while (Gl * 2 * tp <= 32) Gl *= 2;
-  const int tpp = 32 / Gl;
-  const int *cl = a.coll + (int64_t)g * NS;
-  bool bad = false;
-  long long npairs = 0;
-  for (int t0 = 0; t0 < nt; t0 += tpp) {
-    const int ti = t0 + lane / Gl, sub = lane % Gl;
-    const bool act = ti < nt;
-    const int me_i = tb + (act ? ti : 0);
-    const float4 me = a.part[me_i], mel = a.part_lo[me_i];
-    float ax = 0.f, ay = 0.f, az = 0.f, ph = 0.f;
-    for (int s = 0; s < NS; ++s) {
-      const int S = cl[s];
-      if (S < 0) continue;
-      // shift = c_s - c_t in hi + lo
-      const double sx = (s % 3 - 1) * a.hx, sy = ((s / 3) % 3 - 1) * a.hy, sz = DIM == 3 ? (s / 9 - 1) * a.hz : 0.0;
-      const float shx = (float)sx, shy = (float)sy, shz = (float)sz;
-      float tx, ty, tz, ex, ey, ez;
-      two_sum(me.x, -shx, tx, ex);
-      two_sum(me.y, -shy, ty, ey);
-      two_sum(me.z, -shz, tz, ez);
-      ex += mel.x - (float)(sx - (double)shx);
-      ey += mel.y - (float)(sy - (double)shy);
-      ez += mel.z - (float)(sz - (double)shz);
-      const int se = a.pend[S];
-      if (t0 == 0 && lane == 0) npairs += (long long)nt * (se - a.pbeg[S]) - (S == g ? nt : 0);
-      for (int j = a.pbeg[S] + sub; j < se; j += Gl) {
-        if (j == me_i) continue;
-        const float4 q = a.part[j], ql = a.part_lo[j];
-        const float rx = (tx - q.x) + (ex - ql.x);
-        const float ry = (ty - q.y) + (ey - ql.y);
-        const float rz = (tz - q.z) + (ez - ql.z);
-        pair_acc<DIM, true, POT>(rx, ry, rz, q.w, a.eps2, ax, ay, az, ph);
-      }
-    }
-    for (int o = 1; o < Gl; o <<= 1) {
-      ax += __shfl_xor_sync(0xffffffffu, ax, o);
-      ay += __shfl_xor_sync(0xffffffffu, ay, o);
-      az += __shfl_xor_sync(0xffffffffu, az, o);
-      ph += __shfl_xor_sync(0xffffffffu, ph, o);
-    }
-    if (act && sub == 0) {
-      const float4 f = a.far[me_i];
-      const uint32_t o = a.perm[me_i];
-      double vx = a.G * ((double)f.x + ax), vy = a.G * ((double)f.y + ay), vz = a.G * ((double)f.z + az);
-      a.acc[DIM * (size_t)o] = vx;
-      a.acc[DIM * (size_t)o + 1] = vy;
-      if (DIM == 3) a.acc[3 * (size_t)o + 2] = vz;
-      if (a.pot) a.pot[o] = a.G * ((double)f.w + ph);
-      bad |= !(isfinite(vx) && isfinite(vy) && isfinite(vz));
-    }
+  bool bad;
+  switch (best_shape(nt, Gl)) {
+    case 1: bad = near_targets<1, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+    case 2: bad = near_targets<2, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+    case 3: bad = near_targets<3, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+    default: bad = near_targets<4, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
   }
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.err, FMM_DEV_ERR_NONFINITE_OUTPUT);
-  if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)npairs);
+  if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * (total - 1)));
 }
 
 // Adaptive targets: the colleague sums of the adaptive leaves.  An adaptive
@@ -779,18 +904,6 @@ struct CollChunk {
   int f0, f1, bbeg, bend, ncoll;
   double ox, oy, oz;
 };
-
-// Lanes per target group for R targets per lane (largest power of two with
-// ceil(nt / R) * Gl <= 32) and the work of the busiest lane per source:
-// rounds x (R pairs of about 19 instructions with the hi + lo differences,
-// and 4 for the two staged loads and the loop) / Gl.
-__device__ inline void colleague_shape(int nt, int R, int &Gl, float &cost) {
-  const int groups = (nt + R - 1) / R;
-  Gl = 1;
-  while (Gl * 2 * groups <= 32) Gl *= 2;
-  const int rounds = (groups + 32 / Gl - 1) / (32 / Gl);
-  cost = (float)rounds * (float)(19 * R + 4) / (float)Gl;
-}
 
 // The targets of B, R to a lane, in target groups of Gl lanes that share the
 // sources (every Gl-th of each chunk of 32 staged through shared memory).
@@ -920,20 +1033,8 @@ __global__ void __launch_bounds__(256, 4) k_colleague_sum(P2PArgs a, const int *
     const int bl = __ffs(__ballot_sync(0xffffffffu, C == B)) - 1;
     const int bend = __shfl_sync(0xffffffffu, x, bl), bbeg = bend - __shfl_sync(0xffffffffu, nc, bl);
     const double ox = xs[DIM * (size_t)tb], oy = xs[DIM * (size_t)tb + 1], oz = DIM == 3 ? xs[DIM * (size_t)tb + 2] : 0.0;
-    // the register blocking R in 1..4 with the least work on the busiest lane (larger R on ties)
-    int bestR = 1, bestG = 1;
-    float best = 1e30f;
-#pragma unroll
-    for (int R = 1; R <= 4; ++R) {
-      int G;
-      float c;
-      colleague_shape(nt, R, G, c);
-      if (c <= best) {
-        best = c;
-        bestR = R;
-        bestG = G;
-      }
-    }
+    int bestG = 1;
+    const int bestR = best_shape(nt, bestG);
     const CollChunk cc{f0, f1, bbeg, bend, ncoll, ox, oy, oz};
     switch (bestR) {
       case 1: colleague_targets<1, DIM, POT>(a, xs, far, tb, nt, bestG, cc, s_pref, s_cell, s_hi, s_lo, lane); break;
@@ -1031,22 +1132,6 @@ struct DirectArgs {
 // the concatenation; every cell non-empty) and s_cell[si] = (shift c_S - c_T,
 // index delta): the particle at concatenated position f of cell si is
 // off[f + delta].
-
-// For the chunk f0 .. f0 + 31, given the cell si0 holding f0, returns the
-// cell holding f0 + lane (lanes past the end get the last cell; the caller
-// masks them) and moves si0 to the cell holding f0 + 32: one shared load per
-// lane, the cell starts inside the chunk as the bits of a warp-wide OR, and a
-// population count (at most 32 cells overlap 32 consecutive positions).
-__device__ inline int chunk_cell(const int *s_pref, int nsrc, int f0, int &si0, int lane) {
-  const int c = si0 + lane;
-  const int rel = c < nsrc ? s_pref[c] - f0 : 32;  // lane 0: <= 0
-  const unsigned bit = rel < 32 ? 1u << max(rel, 0) : 0u;
-  const unsigned starts = __reduce_or_sync(0xffffffffu, bit);
-  const int si = si0 + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
-  const int last = __shfl_sync(0xffffffffu, si, 31);
-  si0 = s_pref[last + 1] <= f0 + 32 ? last + 1 : last;
-  return si;
-}
 
 // The source particle at concatenated position f of cell si, shifted into
 // the target's frame.
