@@ -1,0 +1,96 @@
+"""Sizes at which the tree, list and direct-sum kernels change tile, launch
+shape or code path, against the oracle: trees bit-exact, FP64 direct sums
+within 1e-12, FP32 force passes within 1e-6 (the bars of test_gpu_fmm.py)."""
+import numpy as np
+import pytest
+from conftest import rel_l2
+
+import fmmgpu
+from fmmgpu import workloads
+
+pytestmark = pytest.mark.gpu
+
+
+# tiles of 1024 sorted keys (levels, cells) and 2048 items (sorts and lists), and 65,536 items, up to which the sort
+# adds its tile histograms up itself
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 1023, 1024, 1025, 2047, 2049, 65535, 65537])
+def test_tree_at_tile_edges(oracle, n, dim):
+    gen = workloads.plummer if dim == 3 else workloads.disk_clumps_2d
+    pos = gen(n, seed=31)[0]
+    want = oracle.tree(pos, 16)
+    with fmmgpu.Context(dim=dim, leaf_cap=16) as c:
+        got = c.tree(pos, with_pairs=False)
+    assert got["depth"] == want["depth"]
+    for k in ("leaf_keys", "leaf_start", "perm"):
+        np.testing.assert_array_equal(got[k], want[k])
+    for a, b in zip(got["level_keys"], want["level_keys"]):
+        np.testing.assert_array_equal(a, b)
+
+
+def test_tree_with_many_equal_keys(oracle):
+    """More than 512 particles with one key at the maximum depth (the leaf
+    order by a sort) next to single ones, and runs across tiles."""
+    rng = np.random.default_rng(5)
+    pos = np.concatenate([rng.random((40, 3)), np.repeat(rng.random((2, 3)), [700, 2300], axis=0), rng.random((60, 3))])
+    rng.shuffle(pos)
+    want = oracle.tree(pos, 64)
+    with fmmgpu.Context(dim=3, leaf_cap=64) as c:
+        got = c.tree(pos, with_pairs=False)
+    for k in ("leaf_keys", "leaf_start", "perm"):
+        np.testing.assert_array_equal(got[k], want[k])
+
+
+# boxes far from a cube: whole cell pairs are summed directly, large cells by several warps (32, 64 or 128 targets each)
+# (adaptive targets need a tree of depth 3: from 6000 particles)
+@pytest.mark.parametrize("n,adaptive", [(700, 0), (6000, 0), (20000, 0), (6000, 32), (20000, 32)])
+@pytest.mark.parametrize("stretch", [(1.0, 0.7, 1.0), (1.0, 0.45, 0.6)])
+def test_elongated_box(oracle, n, adaptive, stretch):
+    pos, m = workloads.uniform_cube(n, seed=41)
+    pos = pos * np.array(stretch)
+    with fmmgpu.Context(dim=3, p=6, leaf_cap=32, direct_max=128, m2l_mode=fmmgpu.FMM_M2L_TC,
+                        adaptive_leaf=adaptive) as c:
+        acc, pot = c.evaluate(pos, m, want_pot=True)
+    if adaptive:
+        want = oracle.fmm_adaptive(pos, m, 6, 32, aleaf=adaptive, direct_max=128, w_direct_max=10 ** 18, want_pot=True)
+    else:
+        want = oracle.fmm(pos, m, 6, 32, direct_max=128, want_pot=True)
+    assert rel_l2(acc, want[0]) < 1e-6
+    assert rel_l2(pot, want[1]) < 1e-6
+
+
+def _direct(pos, m, targets, soft, eps2):
+    """The sum in FP64, term by term as the kernel's two forms."""
+    dim = pos.shape[1]
+    acc, pot = np.zeros((len(targets), dim)), np.zeros(len(targets))
+    for k, i in enumerate(targets):
+        d = pos[i] - pos
+        r2 = (d * d).sum(1)
+        keep = np.arange(len(pos)) != i
+        d, r2, w = d[keep], r2[keep], m[keep]
+        if dim == 3 and soft == fmmgpu.FMM_SOFT_NAIVE_REF:
+            f, p = w / ((r2 + 1e-4) * np.sqrt(r2)), w / np.sqrt(r2)
+        elif dim == 3:
+            f, p = w / (r2 + eps2) ** 1.5, w / np.sqrt(r2 + eps2)
+        else:
+            rr = r2 + (1e-4 if soft == fmmgpu.FMM_SOFT_NAIVE_REF else eps2)
+            f, p = w / rr, -0.5 * w * np.log(rr)
+        acc[k], pot[k] = -(f[:, None] * d).sum(0), p.sum()
+    return acc, pot
+
+
+# 256 sources per stage, 512 targets per block; distances inside and far outside the range of the one-rsqrt form
+@pytest.mark.parametrize("soft", [fmmgpu.FMM_SOFT_PLUMMER, fmmgpu.FMM_SOFT_NAIVE_REF])
+@pytest.mark.parametrize("n,dim,scale", [(2, 3, 1.0), (255, 3, 1.0), (257, 3, 1.0), (513, 3, 1.0), (1500, 2, 1.0),
+                                         (300, 3, 1e-60), (300, 3, 1e60), (130, 2, 1e-3)])
+def test_direct_shapes(n, dim, scale, soft):
+    rng = np.random.default_rng(n)
+    pos, m = rng.random((n, dim)) * scale, rng.random(n)
+    targets = np.array([0, n - 1, n // 2])
+    a, p = _direct(pos, m, targets, soft, 0.0)
+    with fmmgpu.Context(dim=dim) as c:
+        some, some_p = c.direct(pos, m, targets=targets, soft_mode=soft, want_pot=True)
+        every = c.direct(pos, m, soft_mode=soft)
+    assert rel_l2(some, a) < 1e-12
+    assert rel_l2(some_p, p) < 1e-12
+    assert rel_l2(every[targets], a) < 1e-12
