@@ -99,140 +99,127 @@ struct ContractArgs {
   const int *slot_list;  // M2L: [batch][slot index] present slots, nslots_tab[batch] of them
   const int *nslots_tab;
   int cell0, K, KS, KP, dim, mode, slot_base, level_stride;
-  unsigned long long *pair_count;  // M2L: number of (target, source) pairs contracted
 };
 
-// Resolves the source cell of target `tgt` for slot s; returns -1 if absent.
-__device__ inline int contract_source(const ContractArgs &a, int tgt, int s, int cls, int level, int &tslot) {
+// M2L: resolves the source cell of target `tgt` for slot s; returns -1 if absent.
+__device__ inline int m2l_source(const ContractArgs &a, int tgt, int s, int cls) {
   const int nc = 1 << a.dim, ns = a.dim == 3 ? 27 : 9;
-  if (a.mode == MODE_M2L) {
-    int e = c_m2l_slots[a.dim - 2][cls][s];
-    tslot = (e & 511) + level * a.level_stride;
-    int P = a.cparent[tgt];
-    int Q = a.ccoll[(int64_t)P * ns + ((e >> 9) & 31)];
-    if (Q < 0) return -1;
-    if (a.fdirect && a.fdirect[e & 511]) return -1;  // not well separated: direct far field
-    int src = a.cchild[(int64_t)Q * nc + ((e >> 14) & 7)];
-    if (src >= 0 && a.direct_max > 0) {
-      long long nt = a.cpend[tgt] - a.cpbeg[tgt], nsrc = a.cpend[src] - a.cpbeg[src];
-      if (nt * nsrc <= a.direct_max) return -1;  // evaluated by the direct far field
-    }
-    return src;
-  } else if (a.mode == MODE_M2M) {
-    tslot = a.slot_base + s;
-    return a.cchild[(int64_t)tgt * nc + s];
-  } else {
-    tslot = a.slot_base + cls;
-    return a.cparent[tgt];
+  const int e = c_m2l_slots[a.dim - 2][cls][s];
+  const int P = a.cparent[tgt];
+  const int Q = a.ccoll[(int64_t)P * ns + ((e >> 9) & 31)];
+  if (Q < 0) return -1;
+  if (a.fdirect && a.fdirect[e & 511]) return -1;  // not well separated: direct far field
+  const int src = a.cchild[(int64_t)Q * nc + ((e >> 14) & 7)];
+  if (src >= 0 && a.direct_max > 0) {
+    const long long nt = a.cpend[tgt] - a.cpbeg[tgt], nsrc = a.cpend[src] - a.cpbeg[src];
+    if (nt * nsrc <= a.direct_max) return -1;  // evaluated by the direct far field
   }
+  return src;
 }
 
+// A block's 64 targets x (32 J) outputs: warp w takes targets 8 w .. 8 w + 7,
+// a lane the outputs lane + 32 j.  Per slot the operator and the gathered
+// source rows come by cp.async into one of NS buffers; four threads copy a
+// row, whose source index each loaded a slot earlier, so that the only wait of
+// a slot is one barrier.  Bound by FP32 multiply-adds (64 x 81 x 96 at p = 8:
+// 3.9 K cycles per slot and SM).  With the index looked up, shared and counted
+// inside the slot, two barriers and a scalar shared load per target and input
+// it took 10.7 K.
 template <int J, int NS>
 __global__ void __launch_bounds__(CT_THREADS) k_contract(ContractArgs a) {
   extern __shared__ __align__(16) float smem[];
   const int K = a.K, KS = a.KS, KP = a.KP;
   float *Ts = smem;                              // [NS][K][KP]
   float *Xs = Ts + (size_t)NS * K * KP;          // [NS][CT_TGT][KS]
-  int *s_src = (int *)(Xs + (size_t)NS * CT_TGT * KS);  // [NS][CT_TGT]
-  int *s_tslot = s_src + NS * CT_TGT;            // [NS]
-  int *s_any = s_tslot + NS;                     // [NS]
-  __shared__ int s_tgt[CT_TGT];
 
   const int4 b = a.batches[blockIdx.x];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cnt = b.y, level = b.z, cls = b.w;
-  if (tid < CT_TGT) s_tgt[tid] = tid < cnt ? (a.tlist ? a.tlist[b.x + tid] : b.x + tid) : -1;
-  __syncthreads();
-  const int nslots = a.mode == MODE_M2L ? (a.src_tab ? a.nslots_tab[blockIdx.x] : (a.dim == 3 ? 189 : 27))
-                                        : (a.mode == MODE_M2M ? (1 << a.dim) : 1);
+  const int nslots = a.mode == MODE_M2L ? a.nslots_tab[blockIdx.x] : (a.mode == MODE_M2M ? (1 << a.dim) : 1);
+  // (a batch may have no source at all: the lists keep a cell whose only large pairs are with its neighbours)
+  if (nslots == 0) return;
+  const size_t tab_base = (size_t)blockIdx.x * 189;
+  const int row = tid >> 2;  // the row this thread copies a quarter of
+  const int row_tgt = row < cnt ? (a.tlist ? a.tlist[b.x + row] : b.x + row) : -1;
 
-  unsigned long long npairs = 0;
   float acc[8][J];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
     for (int j = 0; j < J; ++j) acc[i][j] = 0.f;
 
-  const bool tabled = a.mode == MODE_M2L && a.src_tab;
-  const size_t tab_base = (size_t)blockIdx.x * 189;
-  auto prefetch = [&](int s, int buf) {
-    int src = -1, ts = 0;
-    if (tid < CT_TGT) {
-      int tg = s_tgt[tid];
-      if (tabled) {
-        const int slot = a.slot_list[tab_base + s];
-        const int e = c_m2l_slots[a.dim - 2][cls][slot];
-        ts = (e & 511) + level * a.level_stride;
-        src = a.src_tab[(tab_base + slot) * CT_TGT + tid];
-      } else if (tg >= 0) {
-        src = contract_source(a, tg, s, cls, level, ts);
-      }
-      s_src[buf * CT_TGT + tid] = src;
-      if (tid == 0 || src >= 0) s_tslot[buf] = ts;  // same for all targets of the batch
+  // operator slot and this row's source cell (-1: none) of slot s
+  auto source = [&](int s, int &ts) -> int {
+    if (a.mode == MODE_M2L) {
+      const int slot = a.slot_list[tab_base + s];
+      ts = (c_m2l_slots[a.dim - 2][cls][slot] & 511) + level * a.level_stride;
+      return a.src_tab[(tab_base + slot) * CT_TGT + row];
     }
-    int any = __syncthreads_count(src >= 0);
-    if (tid == 0) {
-      s_any[buf] = any;
-      npairs += any;
-    }
-    if (any) {
-      const float *T = a.tab + (size_t)s_tslot[buf] * K * KP;
-      float *Td = Ts + (size_t)buf * K * KP;
-      const int nT = K * KP / 4;
-      for (int c = tid; c < nT; c += CT_THREADS) cp_async16(Td + 4 * c, T + 4 * c, 16);
-      float *Xd = Xs + (size_t)buf * CT_TGT * KS;
-      const int cpr = KS / 4;
-      for (int c = tid; c < CT_TGT * cpr; c += CT_THREADS) {
-        int r = c / cpr, q = c % cpr;
-        int sr = s_src[buf * CT_TGT + r];
-        const float *g = sr >= 0 ? a.X + (size_t)(sr - a.cell0) * KS + 4 * q : a.X;
-        cp_async16(Xd + (size_t)r * KS + 4 * q, g, sr >= 0 ? 16 : 0);
-      }
-    }
+    ts = a.slot_base + (a.mode == MODE_M2M ? s : cls);
+    if (row_tgt < 0) return -1;
+    return a.mode == MODE_M2M ? a.cchild[((int64_t)row_tgt << a.dim) + s] : a.cparent[row_tgt];
+  };
+  auto prefetch = [&](int src, int ts, int buf) {
+    const float *T = a.tab + (size_t)ts * K * KP;
+    float *Td = Ts + (size_t)buf * K * KP;
+    const int nT = K * KP / 4;
+    for (int c = tid; c < nT; c += CT_THREADS) cp_async16(Td + 4 * c, T + 4 * c, 16);
+    float *Xd = Xs + ((size_t)buf * CT_TGT + row) * KS;
+    const float *g = a.X + (size_t)(src >= 0 ? src - a.cell0 : 0) * KS;
+    for (int q = tid & 3; q < KS / 4; q += 4) cp_async16(Xd + 4 * q, g + 4 * q, src >= 0 ? 16 : 0);
     cp_async_commit();
   };
 
-  // a batch may have no source at all (the lists keep a cell whose only large pairs are with its neighbours): then
-  // its slot list is empty and holds nothing to read
-  if (NS == 2 && nslots > 0) prefetch(0, 0);
+  int ts_nx, src_nx = source(0, ts_nx);
+  if (NS == 2) {
+    prefetch(src_nx, ts_nx, 0);
+    if (nslots > 1) src_nx = source(1, ts_nx);
+  }
   for (int s = 0; s < nslots; ++s) {
     const int buf = NS == 2 ? (s & 1) : 0;
     if (NS == 1) {
-      prefetch(s, 0);
-      cp_async_wait<0>();
-    } else {
-      if (s + 1 < nslots) {
-        prefetch(s + 1, (s + 1) & 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
+      if (s > 0) __syncthreads();  // everyone is done with the buffer
+      prefetch(src_nx, ts_nx, 0);
+      if (s + 1 < nslots) src_nx = source(s + 1, ts_nx);
     }
-    __syncthreads();
-    if (s_any[buf]) {
-      const float *Tb = Ts + (size_t)buf * K * KP;
-      const float *Xb = Xs + (size_t)buf * CT_TGT * KS + (size_t)(warp * 8) * KS;
-#pragma unroll 2
-      for (int k = 0; k < K; ++k) {
+    cp_async_wait<0>();
+    __syncthreads();  // slot s has landed for everyone; everyone is done with slot s - 1
+    if (NS == 2 && s + 1 < nslots) {
+      prefetch(src_nx, ts_nx, (s + 1) & 1);
+      if (s + 2 < nslots) src_nx = source(s + 2, ts_nx);
+    }
+    const float *Tb = Ts + (size_t)buf * K * KP;
+    const float *Xb = Xs + (size_t)buf * CT_TGT * KS + (size_t)(warp * 8) * KS;
+    // four inputs at a time: one 16-byte broadcast load per target; a row's columns K .. KS - 1 are zero, the
+    // operator has no such rows
+    auto inputs = [&](int k, int m) {
+      float av[8][4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4 *>(av[i]) = *reinterpret_cast<const float4 *>(Xb + i * KS + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (q >= m) break;
         float bv[J];
 #pragma unroll
-        for (int j = 0; j < J; ++j) bv[j] = Tb[(size_t)k * KP + lane + 32 * j];
+        for (int j = 0; j < J; ++j) bv[j] = Tb[(k + q) * KP + lane + 32 * j];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float av = Xb[(size_t)i * KS + k];
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-          for (int j = 0; j < J; ++j) acc[i][j] = fmaf(av, bv[j], acc[i][j]);
-        }
+          for (int j = 0; j < J; ++j) acc[i][j] = fmaf(av[i][q], bv[j], acc[i][j]);
       }
-    }
-    __syncthreads();
+    };
+    const int kf = K & ~3;
+#pragma unroll 2
+    for (int k = 0; k < kf; k += 4) inputs(k, 4);
+    if (kf < K) inputs(kf, K - kf);
   }
-  if (tid == 0 && a.pair_count && a.mode == MODE_M2L) atomicAdd(a.pair_count, npairs);
   // write out
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    int tg = s_tgt[warp * 8 + i];
-    if (tg < 0) continue;
+    const int r = warp * 8 + i;
+    if (r >= cnt) continue;
+    const int tg = a.tlist ? a.tlist[b.x + r] : b.x + r;
     float *y = a.Y + (size_t)(tg - a.cell0) * KS;
 #pragma unroll
     for (int j = 0; j < J; ++j) {
@@ -252,7 +239,7 @@ static void launch_contract_j(const ContractArgs &a, int nb, int stages, size_t 
 }
 
 static size_t contract_smem(int K, int KS, int KP, int NS) {
-  return sizeof(float) * ((size_t)NS * K * KP + (size_t)NS * CT_TGT * KS) + sizeof(int) * (NS * CT_TGT + 2 * NS) + 16;
+  return sizeof(float) * ((size_t)NS * K * KP + (size_t)NS * CT_TGT * KS);
 }
 
 static int launch_contract(const ContractArgs &a, int nb, cudaStream_t st, int64_t &launches) {
@@ -324,8 +311,8 @@ __global__ void k_m2l_sources(ContractArgs a, int tchunk, int *src_tab, int *slo
   unsigned long long ntc = 0;
   for (int e = tid; e < nsl * tchunk; e += blockDim.x) {
     const int slot = e / tchunk, t = e % tchunk;
-    int src = -1, ts;
-    if (s_tgt[t] >= 0) src = contract_source(a, s_tgt[t], slot, b.w, b.z, ts);
+    int src = -1;
+    if (s_tgt[t] >= 0) src = m2l_source(a, s_tgt[t], slot, b.w);
     src_tab[(base + slot) * tchunk + t] = src;
     if (src >= 0) {
       s_flag[slot] = 1;
@@ -1968,7 +1955,6 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   ca.KP = ops.KP;
   ca.dim = dim;
   ca.level_stride = dim == 2 ? 49 : 0;
-  ca.pair_count = ws.counters;
   CUDA_TRY(cudaMemsetAsync(ws.counters, 0, 8 * sizeof(unsigned long long), st));
   TcArgs ta{};
   ta.cchild = ws.cell_child;
@@ -2021,7 +2007,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     if (nbm > 0) {
       // few batches: more threads for each, so that the chains of loads overlap
       k_m2l_sources<<<nbm, nbm < 2 * 148 ? 1024 : 256, 0, st>>>(cm, tchunk, eb.m2l_src.ptr, eb.m2l_list.ptr, eb.m2l_nslots.ptr,
-                                         tc ? eb.m2l_tslot.ptr : nullptr, tc ? ws.counters : nullptr,
+                                         tc ? eb.m2l_tslot.ptr : nullptr, ws.counters,
                                          geometric ? eb.order_p16.ptr : nullptr, geometric ? eb.m2l_w.ptr : nullptr,
                                          ws.counters + 4, lact, msrc, cell0);
       ws.launches += 1;
