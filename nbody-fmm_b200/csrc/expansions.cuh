@@ -56,19 +56,18 @@ struct ExpBuffers {
                           // possible M2L pairs
   DevBuf<uint8_t> lkey;   // (level, class) list keys of those cells, two lists
   DevBuf<int4> batches;
-  DevBuf<uint32_t> cls_count;
+  DevBuf<uint32_t> zeros;  // counters of a pass that start at zero
   DevBuf<float4> lvl_off;  // particle offsets from their level-d ancestor's centre, levels 2..D-1
   DevBuf<uint8_t> lact;    // shortcuts, per cell: [0, ncell) M2L contributions, [ncell, 2 ncell) needs L,
                            // [2 ncell, 3 ncell) M2L source, [3 ncell, 4 ncell) how M is formed
   DevBuf<int> rows;        // shortcuts: class-grouped cells that need L2L, then the M2M rows
-  DevBuf<int> p2m_list;    // shortcuts: the cells whose multipole comes straight from their particles, then their count
+  DevBuf<int> p2m_list;    // shortcuts: the cells whose multipole comes straight from their particles
   DevBuf<int4> batches2;   // shortcuts: batches of the cells that need L2L, then of the M2M rows
   HostPinned<int4> hbatches, hbatches2;  // their host staging
   DevBuf<int> esrc;        // L2L shortcut: per leaf, the cell whose local expansion its particles evaluate
   DevBuf<uint8_t> elev;    //   and that cell's level
   DevBuf<int> m2l_src, m2l_list, m2l_nslots, m2l_tslot;  // per M2L batch: resolved sources and present slots
   DevBuf<uint16_t> tc_img;       // BF16 split operator images for the tensor-core translations
-  DevBuf<unsigned int> tc_work;  // zeroed work counters of the tensor-core launches
   DevBuf<uint8_t> order_p16;     // per M2L operator slot: padded width of its pair order
   DevBuf<uint8_t> fdirect;       // per offset (dx+3) + 7(dy+3) + 49(dz+3): not well separated (direct)
   DevBuf<uint8_t> m2l_w;         // per M2L batch and present slot: padded width of its order

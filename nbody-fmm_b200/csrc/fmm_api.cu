@@ -161,14 +161,13 @@ int fmm_destroy(fmm_ctx *c) {
   c->eb.lkey.release();
   c->eb.rows.release();
   c->eb.batches.release();
-  c->eb.cls_count.release();
+  c->eb.zeros.release();
   c->eb.lvl_off.release();
   c->eb.m2l_src.release();
   c->eb.m2l_list.release();
   c->eb.m2l_nslots.release();
   c->eb.m2l_tslot.release();
   c->eb.tc_img.release();
-  c->eb.tc_work.release();
   c->eb.order_p16.release();
   c->eb.fdirect.release();
   c->eb.m2l_split.release();
@@ -328,12 +327,14 @@ static int evaluate_device(fmm_ctx *c, int64_t n, const double *d_pos, const dou
 }
 
 static int finish(fmm_ctx *c, cudaStream_t st) {
+  HostBack &hb = *c->ws.host;
+  CUDA_TRY(cudaMemcpyAsync(&hb.err, c->ws.dev_err, sizeof(hb.err), cudaMemcpyDeviceToHost, st));
+  if (c->timing_pending)
+    CUDA_TRY(cudaMemcpyAsync(hb.counters, c->ws.counters, sizeof(hb.counters), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
-  unsigned int herr = 0;
-  CUDA_TRY(cudaMemcpy(&herr, c->ws.dev_err, sizeof(herr), cudaMemcpyDeviceToHost));
+  const unsigned int herr = hb.err;
   if (c->timing_pending) {
-    unsigned long long cnt[6] = {0, 0, 0, 0, 0, 0};
-    CUDA_TRY(cudaMemcpy(cnt, c->ws.counters, sizeof(cnt), cudaMemcpyDeviceToHost));
+    const unsigned long long *cnt = hb.counters;
     c->stats.m2l_pairs = (int64_t)cnt[0];
     c->stats.p2p_pairs = (int64_t)(cnt[1] + cnt[3]);
     c->stats.far_direct_pairs = (int64_t)cnt[3];

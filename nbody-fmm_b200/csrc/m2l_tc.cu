@@ -222,14 +222,15 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
   // to chunk_slots of its present slots (item = batch * chunks + run).
   const int chunks = a.mode == TC_M2L ? (TC_MAX_SLOTS + a.chunk_slots - 1) / a.chunk_slots : 1;
   // Thread 0 draws the item after the one it hands out, so that nobody waits
-  // for the counter.
-  int drawn = tid == 0 ? (int)atomicAdd(work, 1u) : 0;
+  // for the counter; the first item of a CTA is its own index.
+  int drawn = (int)blockIdx.x;
   auto load_meta = [&](int buf, int &tg, int &tgg) {
     tg = tgg = -1;
     while (true) {
       if (tid == 0) {
         s_grab = drawn;
-        if (drawn < nb * chunks) drawn = (int)atomicAdd(work, 1u);
+        if (drawn < nb * chunks)
+          drawn = (int)gridDim.x < nb * chunks ? (int)(gridDim.x + atomicAdd(work, 1u)) : nb * chunks;
       }
       __syncthreads();
       const int item = s_grab;
@@ -280,9 +281,17 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
     }
   };
 
+  // Launched while the kernel before it drains (tc_launch_p).  The M2L lists
+  // are its predecessor's work; the rows and batches of M2M and L2L and the
+  // operators are older (the predecessor itself waited for them), so only the
+  // expansions are waited for, below.
+  if (a.mode == TC_M2L) asm volatile("griddepcontrol.wait;" ::: "memory");
   int tg_cur, tgg_cur, tg_nxt, tgg_nxt;
   load_meta(0, tg_cur, tgg_cur);
-  if (s_n[0] == 0) return;
+  if (s_n[0] == 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the launches form a chain: none ends before its predecessor
+    return;
+  }
   load_meta(1, tg_nxt, tgg_nxt);
 
   if (warp == 8) {
@@ -501,7 +510,9 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
       __syncwarp();
       if (lane == 0) mbar_arrive(&s_a);
     };
-    fetch(s_w[0][0], src_of(0, 0, tgg_cur));
+    const int src0 = src_of(0, 0, tgg_cur);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    fetch(s_w[0][0], src0);
     while (true) {
       const int n = s_n[c];
       // the source index of the next slot to fetch
@@ -645,8 +656,20 @@ static int tc_launch_p(const TcArgs &a, int nb, unsigned int *work, cudaStream_t
   if (a.mode == TC_M2L && a.run_slots > 0) b.chunk_slots = std::min(a.run_slots, TC_MAX_SLOTS);
   const int chunks = a.mode == TC_M2L ? (TC_MAX_SLOTS + b.chunk_slots - 1) / b.chunk_slots : 1;
   const int grid = std::min(nb * chunks, per_sm * nsm);
-  k_tc_translate<P16><<<grid, TC_THREADS, sh, st>>>(b, nb, work);
-  return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
+  // programmatic launch: the set-up, the metadata and the first operator
+  // copies run while the kernel before it drains (a small system's M2M and
+  // L2L are a chain of launches of one work item per CTA)
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(TC_THREADS);
+  cfg.dynamicSmemBytes = sh;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_tc_translate<P16>, b, nb, work) == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;
 }
 
 __global__ void k_tc_split(const int *slot_list, const int *tslot_list, const uint8_t *slot_p16, const int *nslots,

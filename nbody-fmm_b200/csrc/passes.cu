@@ -1836,11 +1836,15 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   const bool tc = m2l_mode == FMM_M2L_TC && P16 <= TC_MAX_P16;
   const int tchunk = tc ? 128 : CT_TGT;
   const bool split96 = ops.img96 != nullptr;  // M2L tiles up to 96 wide run in a kernel of their own
+  // counters that start at zero, in one buffer: bucket sizes of the two list
+  // steps, work counters of the tensor-core launches, listed P2M cells
+  if (!eb.zeros.reserve(1024 + TC_MAX_LAUNCHES + 1)) return FMM_ERR_OUT_OF_MEMORY;
+  CUDA_TRY(cudaMemsetAsync(eb.zeros.ptr, 0, (1024 + TC_MAX_LAUNCHES + 1) * sizeof(uint32_t), st));
+  uint32_t *const cls_count = eb.zeros.ptr;
+  unsigned int *const tc_work = eb.zeros.ptr + 1024, *const p2m_count = tc_work + TC_MAX_LAUNCHES;
   int tc_k = 0;  // tensor-core launches so far (work counter index)
   if (tc && D >= 2) {
-    if (!eb.tc_work.reserve(TC_MAX_LAUNCHES)) return FMM_ERR_OUT_OF_MEMORY;
     if (2 * D + 2 > TC_MAX_LAUNCHES) return FMM_ERR_UNSUPPORTED;
-    CUDA_TRY(cudaMemsetAsync(eb.tc_work.ptr, 0, TC_MAX_LAUNCHES * sizeof(unsigned int), st));
   }
   const double emax = g.emax > 0 ? g.emax : 1.0;
   const double sD = std::ldexp(emax, -D);
@@ -1881,7 +1885,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     ntl = t.level_off[D] + t.level_count[D] - t.level_off[2];
     // lists: every cell (without the shortcuts), then the M2L targets
     const int nlist = shortcut ? 1 : 2;
-    if (!eb.tlist.reserve((size_t)nlist * ntl) || !eb.lkey.reserve((size_t)2 * ntl) || !eb.cls_count.reserve(512))
+    if (!eb.tlist.reserve((size_t)nlist * ntl) || !eb.lkey.reserve((size_t)2 * ntl))
       return FMM_ERR_OUT_OF_MEMORY;
     uint8_t *k_all = shortcut ? nullptr : eb.lkey.ptr, *k_m2l = eb.lkey.ptr + (shortcut ? 0 : ntl);
     const int cw = ntl < (1 << 20) ? 4 : 32;
@@ -1892,13 +1896,12 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
                                                          adaptive ? ws.aflag : nullptr, cell0);
     ws.launches += 1;
     // (the counts of the M2L list are read from 256 on)
-    CUDA_TRY(cudaMemsetAsync(eb.cls_count.ptr, 0, 512 * sizeof(uint32_t), st));
-    bucket_lists(ws, eb.lkey.ptr, nlist, ntl, lvo.off[2], eb.tlist.ptr, eb.cls_count.ptr + (shortcut ? 256 : 0), st);
+    bucket_lists(ws, eb.lkey.ptr, nlist, ntl, lvo.off[2], eb.tlist.ptr, cls_count + (shortcut ? 256 : 0), st);
     if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
     tl = eb.tlist.ptr;
     tl_m2l = eb.tlist.ptr + (shortcut ? 0 : ntl);
-    uint32_t hc[512];
-    CUDA_TRY(cudaMemcpyAsync(hc, eb.cls_count.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    const uint32_t *hc = ws.host->hist;
+    CUDA_TRY(cudaMemcpyAsync(ws.host->hist, cls_count, sizeof(ws.host->hist), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     const int ncls = 1 << dim;
     // batch count, then the table written straight into pinned staging
@@ -2031,11 +2034,10 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   if (shortcut) {
     const int first2 = t.level_off[2], leaf_first = t.level_off[D];
     k_needs_l<<<cdiv(ntl, TPB), TPB, 0, st>>>(lact, first2, ntl, ws.cell_parent, cell0, needs);
-    if (!eb.p2m_list.reserve((size_t)ntl + 1)) return FMM_ERR_OUT_OF_MEMORY;
-    CUDA_TRY(cudaMemsetAsync(eb.p2m_list.ptr + ntl, 0, sizeof(int), st));
+    if (!eb.p2m_list.reserve((size_t)ntl)) return FMM_ERR_OUT_OF_MEMORY;
     k_m_mode<<<cdiv(ntl, TPB), TPB, 0, st>>>(lact, msrc, first2, leaf_first, ntl, ws.cell_parent, ws.cell_pbeg,
                                              ws.cell_pend, cell0, P2M_DIRECT_MAX, mmode, eb.p2m_list.ptr,
-                                             reinterpret_cast<unsigned *>(eb.p2m_list.ptr + ntl));
+                                             p2m_count);
     ws.launches += 2;
     // L2L rows: levels 3..D; M2M rows: children at levels 3..D (tensor
     // cores) or the mode-2 parents at levels 2..D-1
@@ -2044,11 +2046,10 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     k_row_keys<<<cdiv(ntl, TPB), TPB, 0, st>>>(ws.cell_key, needs, mmode, ws.cell_parent, lvo, D, dim, cell0,
                                                tc ? 1 : 0, ntl, eb.lkey.ptr);
     ws.launches += 1;
-    CUDA_TRY(cudaMemsetAsync(eb.cls_count.ptr, 0, 512 * sizeof(uint32_t), st));
-    bucket_lists(ws, eb.lkey.ptr, 2, ntl, first2, eb.rows.ptr, eb.cls_count.ptr, st);
+    bucket_lists(ws, eb.lkey.ptr, 2, ntl, first2, eb.rows.ptr, cls_count + 512, st);
     if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
-    uint32_t hc[512];
-    CUDA_TRY(cudaMemcpyAsync(hc, eb.cls_count.ptr, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    const uint32_t *hc = ws.host->hist;
+    CUDA_TRY(cudaMemcpyAsync(ws.host->hist, cls_count + 512, sizeof(ws.host->hist), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     const int ncls = 1 << dim;
     size_t cnt_b = 0, nb2 = 0;
@@ -2110,7 +2111,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     pm.pbeg = ws.cell_pbeg;
     pm.pend = ws.cell_pend;
     pm.list = eb.p2m_list.ptr;
-    pm.count = reinterpret_cast<const unsigned *>(eb.p2m_list.ptr + ntl);
+    pm.count = p2m_count;
     pm.cell0 = cell0;
     pm.p = p;
     pm.K = ops.K;
@@ -2136,7 +2137,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     t2.X = eb.M.ptr;
     t2.Y = eb.M.ptr;
     const int nb = shortcut ? um_b1[d + 1] - um_b0[d + 1] : lvl_b1[d + 1] - lvl_b0[d + 1];
-    int rc = tc_launch(t2, nb, eb.tc_work.ptr + tc_k++, st, ws.launches);
+    int rc = tc_launch(t2, nb, tc_work + tc_k++, st, ws.launches);
     if (rc) return rc;
   }
   for (int d = D - 1; d >= 2 && !tc; --d) {  // cells of level d gather their children
@@ -2252,7 +2253,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
           lo.tslot_list = lo_t;
           lo.slot_p16 = lo_w;
           lo.nslots = lo_n;
-          rc = tc_launch(lo, nbm, eb.tc_work.ptr + tc_k++, st, ws.launches);
+          rc = tc_launch(lo, nbm, tc_work + tc_k++, st, ws.launches);
         }
         if (!rc) {
           TcArgs hi = t2;
@@ -2260,10 +2261,10 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
           hi.tslot_list = hi_t;
           hi.slot_p16 = hi_w;
           hi.nslots = hi_n;
-          rc = tc_launch(hi, nbm, eb.tc_work.ptr + tc_k++, st, ws.launches);
+          rc = tc_launch(hi, nbm, tc_work + tc_k++, st, ws.launches);
         }
       } else {
-        rc = tc_launch(t2, nbm, eb.tc_work.ptr + tc_k++, st, ws.launches);
+        rc = tc_launch(t2, nbm, tc_work + tc_k++, st, ws.launches);
       }
     } else {
       cm.src_tab = eb.m2l_src.ptr;
@@ -2284,7 +2285,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     t2.op_base = ops.off_l2l;
     t2.X = eb.L.ptr;
     t2.Y = eb.L.ptr;
-    int rc = tc_launch(t2, l2_b1[d] - l2_b0[d], eb.tc_work.ptr + tc_k++, st, ws.launches);
+    int rc = tc_launch(t2, l2_b1[d] - l2_b0[d], tc_work + tc_k++, st, ws.launches);
     if (rc) return rc;
   }
   for (int d = 3; d <= D && !tc; ++d) {
@@ -2301,7 +2302,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   // adaptive targets: the direct far field's targets per level and the
   // colleague-sum items, counted on the device and read back together
   // (timed with the downward pass)
-  std::vector<unsigned> ntgt;
+  const unsigned *const ntgt = ws.host->ntgt;
   uint32_t n_items = 0;
   const int cl_chunk = p2p_chunk > 0 ? p2p_chunk : CL_CHUNK_DEFAULT;
   if (adaptive) {
@@ -2319,8 +2320,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
                                                          ws.cell_pend, dim == 3 ? 27 : 9, cl_chunk, ccnt);
     exclusive_scan(ws, ccnt, coff, ncell, cnt + D + 1, st);
     ws.launches += D;
-    ntgt.assign(D + 2, 0u);
-    CUDA_TRY(cudaMemcpyAsync(ntgt.data(), cnt, sizeof(unsigned) * (D + 2), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(ws.host->ntgt, cnt, sizeof(unsigned) * (D + 2), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     n_items = ntgt[D + 1];
     if (!eb.citems.reserve((size_t)n_items + 1)) return FMM_ERR_OUT_OF_MEMORY;

@@ -17,6 +17,7 @@
 // or for leaves of more than 512 particles a second stable sort of the
 // depth-d keys in input order.
 #include <algorithm>
+#include <cstddef>
 #include <vector>
 
 #include "common.cuh"
@@ -757,9 +758,8 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   const int nbN = cdiv(n, TPB);
   const int nblv = cdiv(n, LV_TILE);
   if (!ws.reserve_particles(n) || !ws.blev.reserve((size_t)nblv * (Dmax + 1))) return FMM_ERR_OUT_OF_MEMORY;
-  uint32_t *lev = ws.scalars;  // cells, then the largest cell, of every level
-  CUDA_TRY(cudaMemsetAsync(ws.dev_err, 0, sizeof(unsigned int), st));
-  CUDA_TRY(cudaMemsetAsync(lev, 0, 2 * LV_MAX * sizeof(uint32_t), st));
+  uint32_t *lev = ws.lev;  // cells, then the largest cell, of every level
+  CUDA_TRY(cudaMemsetAsync(lev, 0, offsetof(TreeBack, ticket) - offsetof(TreeBack, lev), st));  // and the error word
   k_aabb<<<std::min(nbN, WS_AABB_BLOCKS), TPB, 0, st>>>(d_pos, d_mass, n, dim, ws.box_u64, ws.ticket, ws.geom,
                                                        ws.dev_err);
   k_keys<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, ws.geom, ws.keyA, ws.valA);
@@ -772,14 +772,14 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   ws.launches += 1;
   // the box, the finiteness check (keys of non-finite positions are clamped
   // into range, so what ran above is harmless) and the levels' sizes
-  uint32_t hlev[2 * LV_MAX];
-  unsigned int herr = 0;
-  CUDA_TRY(cudaMemcpyAsync(t.lo, ws.geom, 6 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaMemcpyAsync(&herr, ws.dev_err, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-  CUDA_TRY(cudaMemcpyAsync(hlev, lev, sizeof(hlev), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(cudaMemcpyAsync(&ws.host->tree, ws.bback.ptr, sizeof(TreeBack), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
-  if (herr & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
-  for (int d = 0; d < 3; ++d) t.hi[d] = t.lo[3 + d];
+  const uint32_t *hlev = ws.host->tree.lev;
+  if (ws.host->tree.err & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
+  for (int d = 0; d < 3; ++d) {
+    t.lo[d] = ws.host->tree.geom[d];
+    t.hi[d] = ws.host->tree.geom[3 + d];
+  }
 
   // depth loop, tree.cpp:43-69
   unsigned int max_n = (unsigned int)n;

@@ -49,6 +49,24 @@ struct DevBuf {
 // blocks of the bounding-box kernel
 static constexpr int WS_AABB_BLOCKS = 148 * 4;
 
+// What the host reads after the tree's first kernels, in one copy.
+struct TreeBack {
+  double geom[6];                        // box min, max
+  uint32_t lev[2 * (FMM_MAX_DEPTH + 1)]; // cells, then the largest cell, of every level
+  unsigned int err;                      // device error word of the pass
+  unsigned int ticket;                   // of the bounding-box kernel, zero between launches
+};
+// Page-locked landing place of a context's small reads (each read is waited
+// for before the next one into the same place): a copy into pageable memory
+// goes through the driver's staging and takes several microseconds more.
+struct HostBack {
+  TreeBack tree;
+  uint32_t hist[512];
+  unsigned int ntgt[FMM_MAX_DEPTH + 3];
+  unsigned long long counters[6];
+  unsigned int err;
+};
+
 struct Workspace {
   // per particle
   DevBuf<uint64_t> bkeyA, bkeyB, bkeyC;
@@ -66,9 +84,8 @@ struct Workspace {
   // misc
   DevBuf<uint32_t> bscan, bhist;
   DevBuf<unsigned long long> bbox;
-  DevBuf<double> bgeom;
-  DevBuf<uint32_t> bscalars;
-  DevBuf<unsigned int> berr;
+  DevBuf<TreeBack> bback;
+  HostBack *host = nullptr;
   DevBuf<unsigned long long> bcount;  // [0] M2L pairs, [1] near-field pairs, [2] M2L tiles, [3] direct far-field
                                       // pairs, [4] sum over M2L pairs of the target's particle count
 
@@ -82,24 +99,24 @@ struct Workspace {
   int *alist = nullptr;
   unsigned long long *box_u64 = nullptr;
   double *geom = nullptr;
-  uint32_t *scalars = nullptr;
-  unsigned int *ticket = nullptr;  // of the bounding-box kernel, zero between launches
+  uint32_t *lev = nullptr;
+  unsigned int *ticket = nullptr;
   unsigned int *dev_err = nullptr;
   unsigned long long *counters = nullptr;
   int64_t launches = 0;
   bool ok = true;
 
   bool init_small() {
-    ok &= bbox.reserve(6 * WS_AABB_BLOCKS) && bgeom.reserve(8) && bscalars.reserve(2 * (FMM_MAX_DEPTH + 1) + 1) &&
-          berr.reserve(4) && bcount.reserve(8);
+    ok &= bbox.reserve(6 * WS_AABB_BLOCKS) && bback.reserve(1) && bcount.reserve(8);
     if (!ok) return false;
-    ticket = bscalars.ptr + 2 * (FMM_MAX_DEPTH + 1);
-    ok &= cudaMemset(ticket, 0, sizeof(unsigned int)) == cudaSuccess;
+    ok &= cudaHostAlloc((void **)&host, sizeof(HostBack), cudaHostAllocDefault) == cudaSuccess;
+    ok &= cudaMemset(bback.ptr, 0, sizeof(TreeBack)) == cudaSuccess;
     counters = bcount.ptr;
     box_u64 = bbox.ptr;
-    geom = bgeom.ptr;
-    scalars = bscalars.ptr;
-    dev_err = berr.ptr;
+    geom = bback.ptr->geom;
+    lev = bback.ptr->lev;
+    dev_err = &bback.ptr->err;
+    ticket = &bback.ptr->ticket;
     return ok;
   }
   bool reserve_particles(int64_t n) {
@@ -148,7 +165,9 @@ struct Workspace {
     bleaf_of.release(); bpart.release(); bpart_lo.release(); bfar.release();
     bcell_key.release(); bcell_pbeg.release(); bcell_pend.release(); bcell_parent.release();
     bcell_child.release(); bcell_coll.release(); baflag.release(); balist.release();
-    bscan.release(); bhist.release(); bbox.release(); bgeom.release(); bscalars.release(); berr.release(); bcount.release();
+    bscan.release(); bhist.release(); bbox.release(); bback.release(); bcount.release();
+    if (host) cudaFreeHost(host);
+    host = nullptr;
   }
 };
 
@@ -164,7 +183,7 @@ struct TreeState {
   int dim = 3;
   int64_t n = 0;
   int depth = 0;
-  double lo[6] = {0, 0, 0, 0, 0, 0};  // lo[0..2] box min (lo[3..5] scratch)
+  double lo[3] = {0, 0, 0};
   double hi[3] = {0, 0, 0};
   std::vector<int> level_count, level_off;
   std::vector<int> level_max;  // particles of the largest cell of each level
