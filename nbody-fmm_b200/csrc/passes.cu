@@ -101,17 +101,17 @@ struct ContractArgs {
   int cell0, K, KS, KP, dim, mode, slot_base, level_stride;
 };
 
-// M2L: resolves the source cell of target `tgt` for slot s; returns -1 if absent.
-__device__ inline int m2l_source(const ContractArgs &a, int tgt, int s, int cls) {
+// M2L: the source cell of slot s of a target with nt particles and parent P;
+// -1 if absent.
+__device__ inline int m2l_source(const ContractArgs &a, int P, int nt, int s, int cls) {
   const int nc = 1 << a.dim, ns = a.dim == 3 ? 27 : 9;
   const int e = c_m2l_slots[a.dim - 2][cls][s];
-  const int P = a.cparent[tgt];
   const int Q = a.ccoll[(int64_t)P * ns + ((e >> 9) & 31)];
   if (Q < 0) return -1;
   if (a.fdirect && a.fdirect[e & 511]) return -1;  // not well separated: direct far field
   const int src = a.cchild[(int64_t)Q * nc + ((e >> 14) & 7)];
   if (src >= 0 && a.direct_max > 0) {
-    const long long nt = a.cpend[tgt] - a.cpbeg[tgt], nsrc = a.cpend[src] - a.cpbeg[src];
+    const long long nsrc = a.cpend[src] - a.cpbeg[src];
     if (nt * nsrc <= a.direct_max) return -1;  // evaluated by the direct far field
   }
   return src;
@@ -293,13 +293,18 @@ __global__ void k_m2l_sources(ContractArgs a, int tchunk, int *src_tab, int *slo
                               uint8_t *slot_p16, unsigned long long *nt_sum, uint8_t *lact, uint8_t *msrc,
                               int cell0) {
   __shared__ int s_flag[189];
-  __shared__ int s_tgt[128];
+  __shared__ int s_tgt[128], s_par[128], s_np[128];  // targets, their parents and sizes
   __shared__ int s_cnt;
   __shared__ unsigned long long s_nt;
   const int4 b = a.batches[blockIdx.x];
   const int tid = threadIdx.x;
   const int nsl = a.dim == 3 ? 189 : 27;
-  if (tid < tchunk) s_tgt[tid] = tid < b.y ? a.tlist[b.x + tid] : -1;
+  if (tid < tchunk) {
+    const int t = tid < b.y ? a.tlist[b.x + tid] : -1;
+    s_tgt[tid] = t;
+    s_par[tid] = t >= 0 ? a.cparent[t] : 0;
+    s_np[tid] = t >= 0 ? a.cpend[t] - a.cpbeg[t] : 0;
+  }
   for (int i = tid; i < 189; i += blockDim.x) s_flag[i] = 0;
   if (tid == 0) {
     s_cnt = 0;
@@ -312,12 +317,12 @@ __global__ void k_m2l_sources(ContractArgs a, int tchunk, int *src_tab, int *slo
   for (int e = tid; e < nsl * tchunk; e += blockDim.x) {
     const int slot = e / tchunk, t = e % tchunk;
     int src = -1;
-    if (s_tgt[t] >= 0) src = m2l_source(a, s_tgt[t], slot, b.w);
+    if (s_tgt[t] >= 0) src = m2l_source(a, s_par[t], s_np[t], slot, b.w);
     src_tab[(base + slot) * tchunk + t] = src;
     if (src >= 0) {
       s_flag[slot] = 1;
       ++cnt;
-      ntc += (unsigned long long)(a.cpend[s_tgt[t]] - a.cpbeg[s_tgt[t]]);
+      ntc += (unsigned long long)s_np[t];
       if (lact) lact[s_tgt[t] - cell0] = 1;
       if (msrc) msrc[src - cell0] = 1;
     }
@@ -1456,11 +1461,18 @@ __global__ void k_class_keys(const uint64_t *ckey, const int *cpbeg, const int *
 // of them needed.  mode 0: not formed.
 static constexpr int P2M_DIRECT_MAX = 64;
 
+//
+// It also marks (needs) every ancestor-or-self at levels >= 2 of the cells
+// with M2L contributions (lact): the cells whose local expansion is needed
+// below them.
 __global__ void k_m_mode(const uint8_t *lact, const uint8_t *msrc, int first2, int leaf_first, int count,
                          const int *parent, const int *pbeg, const int *pend, int cell0, int tmax, uint8_t *mode,
-                         int *list1, unsigned *count1) {
+                         int *list1, unsigned *count1, uint8_t *needs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   const int c = first2 + i;
+  if (i < count && lact[c - cell0])
+    for (int a = c; a >= first2 && !needs[a - cell0]; a = parent[a])  // stops where another walk already passed
+      needs[a - cell0] = 1;
   int md = 0;
   if (i < count) {
     int a = c;
@@ -1706,19 +1718,6 @@ static int launch_p2m_list(const P2MListArgs &pm, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------ L2L shortcut
-// Marks every ancestor-or-self at levels >= 2 of the cells with M2L
-// contributions (lact): the cells whose local expansion is needed below.
-__global__ void k_needs_l(const uint8_t *lact, int first2, int count, const int *parent, int cell0, uint8_t *needs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  int c = first2 + i;
-  if (!lact[c - cell0]) return;
-  while (c >= first2 && !needs[c - cell0]) {  // stops where another walk already passed
-    needs[c - cell0] = 1;
-    c = parent[c];
-  }
-}
-
 // Per leaf: its deepest ancestor-or-self with a needed local expansion.
 __global__ void k_leaf_esrc(int leaf_first, int nleaves, int D, int first2, const int *parent, const uint8_t *needs,
                             int cell0, int *esrc, uint8_t *elev) {
@@ -2033,12 +2032,11 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   std::vector<int> l2_b0(lvl_b0), l2_b1(lvl_b1), um_b0(D + 2, 0), um_b1(D + 2, 0);
   if (shortcut) {
     const int first2 = t.level_off[2], leaf_first = t.level_off[D];
-    k_needs_l<<<cdiv(ntl, TPB), TPB, 0, st>>>(lact, first2, ntl, ws.cell_parent, cell0, needs);
     if (!eb.p2m_list.reserve((size_t)ntl)) return FMM_ERR_OUT_OF_MEMORY;
     k_m_mode<<<cdiv(ntl, TPB), TPB, 0, st>>>(lact, msrc, first2, leaf_first, ntl, ws.cell_parent, ws.cell_pbeg,
                                              ws.cell_pend, cell0, P2M_DIRECT_MAX, mmode, eb.p2m_list.ptr,
-                                             p2m_count);
-    ws.launches += 2;
+                                             p2m_count, needs);
+    ws.launches += 1;
     // L2L rows: levels 3..D; M2M rows: children at levels 3..D (tensor
     // cores) or the mode-2 parents at levels 2..D-1
     const int m_lo = tc ? 3 : 2, m_hi = tc ? D : D - 1;

@@ -235,11 +235,118 @@ __global__ void __launch_bounds__(RS_BLOCK) k_radix_scatter(const uint64_t *kin,
   }
 }
 
+// The whole sort of up to 32,768 items in one launch: a cluster of up to 8
+// CTAs, one tile of 256 RR items each, goes through the digits with two
+// cluster barriers per digit (histograms out, items moved) instead of two
+// launches; the tiles' histograms and the ping-pong buffers are in global
+// memory (L2).  A warp takes 32 RR consecutive items: one count of its items
+// per digit, then their places round by round; the rounds are a chain, so RR
+// is the smallest that eight CTAs hold the items with.
+static constexpr int RC_MAX_CLUSTER = 8;
+
+__device__ inline void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int RC_ROUNDS>
+__global__ void __launch_bounds__(RS_BLOCK) k_sort_cluster(uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb, int n,
+                                                           int bits, uint32_t *hist) {
+  __shared__ uint32_t s_warp[RS_BLOCK / 32];
+  __shared__ uint32_t s_cnt[RS_BLOCK / 32][256];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nb = gridDim.x;
+  const int base = blockIdx.x * RS_BLOCK * RC_ROUNDS + warp * 32 * RC_ROUNDS;
+  for (int shift = 0; shift < bits; shift += 8) {
+    uint64_t key[RC_ROUNDS];
+    uint32_t val[RC_ROUNDS];
+    for (int b = lane; b < 256; b += 32) s_cnt[warp][b] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const int i = base + r * 32 + lane;
+      key[r] = i < n ? __ldcg(ka + i) : 0ull;  // (written by other SMs in the digit before)
+      val[r] = i < n ? __ldcg(va + i) : 0u;
+    }
+    // items past the end take digit 256 + lane (no peers, counted nowhere)
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const bool in = base + r * 32 + lane < n;
+      const uint32_t d = in ? (uint32_t)(key[r] >> shift) & 255u : 256u + lane;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      if (in && lane == __ffs(peers) - 1) s_cnt[warp][d] += (uint32_t)__popc(peers);
+      __syncwarp();
+    }
+    __syncthreads();
+    uint32_t mine = 0;
+    for (int w = 0; w < RS_BLOCK / 32; ++w) mine += s_cnt[w][tid];
+    __stcg(hist + blockIdx.x * 256 + tid, mine);
+    cluster_sync();
+    uint32_t all = 0, before = 0, total;
+    for (int b = 0; b < nb; ++b) {
+      const uint32_t v = __ldcg(hist + b * 256 + tid);
+      if (b < (int)blockIdx.x) before += v;
+      all += v;
+    }
+    uint32_t run = block_excl_scan(all, s_warp, total) + before;
+    for (int w = 0; w < RS_BLOCK / 32; ++w) {
+      const uint32_t c = s_cnt[w][tid];
+      s_cnt[w][tid] = run;  // where the warp's items of this digit start
+      run += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RC_ROUNDS; ++r) {
+      const bool in = base + r * 32 + lane < n;
+      const uint32_t d = in ? (uint32_t)(key[r] >> shift) & 255u : 256u + lane;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t at = in ? s_cnt[warp][d] : 0u;
+      __syncwarp();
+      if (in) {
+        const uint32_t pos = at + __popc(peers & ((1u << lane) - 1u));
+        __stcg(kb + pos, key[r]);
+        __stcg(vb + pos, val[r]);
+        if (lane == __ffs(peers) - 1) s_cnt[warp][d] = at + (uint32_t)__popc(peers);
+      }
+      __syncwarp();
+    }
+    cluster_sync();
+    uint64_t *kt = ka;
+    ka = kb;
+    kb = kt;
+    uint32_t *vt = va;
+    va = vb;
+    vb = vt;
+  }
+}
+
 // Sorts (keys, vals) by the low `bits` bits of the key, stably; the result
 // ends in (keys, vals) (the buffers are ping-ponged with the alternates).
 void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
                 int bits, cudaStream_t st) {
   if (n <= 1 || bits <= 0) return;
+  if (n <= (int64_t)RS_BLOCK * 16 * RC_MAX_CLUSTER) {
+    int rounds = 2, nc = 1;
+    while ((int64_t)RS_BLOCK * rounds * RC_MAX_CLUSTER < n) rounds *= 2;
+    while ((int64_t)RS_BLOCK * rounds * nc < n) nc *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nc);
+    cfg.blockDim = dim3(RS_BLOCK);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)nc;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    auto kern = rounds == 2 ? k_sort_cluster<2> : rounds == 4 ? k_sort_cluster<4> : rounds == 8 ? k_sort_cluster<8>
+                                                                                              : k_sort_cluster<16>;
+    cudaLaunchKernelEx(&cfg, kern, keys, vals, keys_alt, vals_alt, (int)n, bits, ws.radix_hist(nc));
+    ws.launches += 1;
+    if (((bits + 7) / 8) & 1) {
+      std::swap(keys, keys_alt);
+      std::swap(vals, vals_alt);
+    }
+    return;
+  }
   int nb = (int)((n + RS_TILE - 1) / RS_TILE);
   uint32_t *hist = ws.radix_hist(nb);
   const bool by_tile = nb <= RS_FUSED_TILES;
@@ -547,7 +654,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_level_scan(uint32_t *blockcnt, i
 __global__ void __launch_bounds__(LV_BLOCK) k_make_cells(const uint64_t *keys, int64_t n, int dim, int Dmax, int D,
                                                          int nb, const uint32_t *blockoff, LevelOffsets lo,
                                                          uint64_t *ckey, int *cpbeg, int *cpend, int *cparent,
-                                                         int *cchild, int *leaf_of) {
+                                                         int *cchild, int *ccoll, int *leaf_of) {
   __shared__ uint32_t s_wc[LV_MAX][LV_BLOCK / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // a warp takes 32 LV_ROUNDS consecutive particles
@@ -567,6 +674,9 @@ __global__ void __launch_bounds__(LV_BLOCK) k_make_cells(const uint64_t *keys, i
     if (lane == 0) s_wc[d][warp] = (uint32_t)c;
   }
   __syncthreads();
+  const int ns = dim == 3 ? 27 : 9;
+  if (blockIdx.x == 0 && (int)threadIdx.x < ns)  // the root's only colleague is itself
+    ccoll[(int64_t)lo.off[0] * ns + threadIdx.x] = (int)threadIdx.x == ns / 2 ? lo.off[0] : -1;
   int up[LV_ROUNDS];  // the particle's cell one level up
 #pragma unroll
   for (int r = 0; r < LV_ROUNDS; ++r) up[r] = -1;
@@ -696,14 +806,6 @@ __global__ void k_colleagues_targets(const uint64_t *ckey, const int *cparent, c
   }
 }
 
-__global__ void k_root_colleague(int *ccoll, int root, int dim) {
-  if (threadIdx.x == 0) {
-    int ns = dim == 3 ? 27 : 9;
-    for (int s = 0; s < ns; ++s) ccoll[(int64_t)root * ns + s] = -1;
-    ccoll[(int64_t)root * ns + ns / 2] = root;
-  }
-}
-
 // Gathers particles into leaf order: the offset from the leaf's geometric
 // centre split into FP32 hi + lo parts (x - c = hi + lo to ~48 bits), and the
 // FP32 mass, used by P2M, L2P (hi only) and P2P (hi and lo).
@@ -814,7 +916,7 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   CUDA_TRY(cudaMemsetAsync(ws.cell_child, 0xff, sizeof(int) * (size_t)cells * nc, st));
   k_level_scan<<<D + 1, SCAN_BLOCK, 0, st>>>(ws.blev.ptr, nblv);
   k_make_cells<<<nblv, LV_BLOCK, 0, st>>>(kA, n, dim, Dmax, D, nblv, ws.blev.ptr, lo, ws.cell_key, ws.cell_pbeg,
-                                          ws.cell_pend, ws.cell_parent, ws.cell_child, ws.leaf_of);
+                                          ws.cell_pend, ws.cell_parent, ws.cell_child, ws.cell_coll, ws.leaf_of);
   ws.launches += 2;
   // final order: each leaf's particles in input order (tree.cpp:62-66).  The
   // Dmax order already groups the leaves; with leaves of at most
@@ -844,8 +946,6 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
     aflag = ws.aflag;
   }
   // colleagues, top-down
-  k_root_colleague<<<1, 32, 0, st>>>(ws.cell_coll, 0, dim);
-  ws.launches += 1;
   for (int d = 1; d <= D; ++d) {
     if (aflag)  // adaptive targets are 3D only
       k_colleagues_targets<3><<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(
