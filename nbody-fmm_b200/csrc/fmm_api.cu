@@ -50,6 +50,9 @@ struct fmm_ctx {
   fmm_stats stats;
   cudaEvent_t ev[7] = {};  // pass boundaries; ev[6] ends the direct far field
   bool timing_pending = false;
+  bool phase_times = true;  // record the phase events of a pass (not where nobody can ask for them: eight events
+                            // and their queries are a tenth of a small pass's driver calls)
+  bool times_recorded = false;
   bool have_tree = false;
 };
 
@@ -220,7 +223,8 @@ static int64_t direct_threshold(const fmm_config &c) {
 static int pass(fmm_ctx *c, int64_t n, const double *d_pos, const double *d_mass, double *d_acc, double *d_pot,
                 cudaStream_t st, const OrderOpts &oo, bool want64) {
   const int dim = c->cfg.dim;
-  CUDA_TRY(cudaEventRecord(c->ev[0], st));
+  cudaEvent_t *const ev = c->phase_times ? c->ev : nullptr;
+  if (ev) CUDA_TRY(cudaEventRecord(ev[0], st));
   int rc = build_tree(c->ws, c->tree, d_pos, d_mass, n, dim, c->cfg.leaf_cap, st, c->cfg.adaptive_leaf);
   if (rc) return rc;
   if (!c->ws.ok) return FMM_ERR_OUT_OF_MEMORY;
@@ -245,7 +249,7 @@ static int pass(fmm_ctx *c, int64_t n, const double *d_pos, const double *d_mass
   c->stats.judge_rel_l2 = jr;
   c->stats.order_fallbacks = fb;
   rc = run_fmm_passes(c->ws, c->tree, c->ops, c->eb, d_pos, d_mass, c->cfg.p, c->cfg.eps2, c->cfg.G, g, d_acc, d_pot,
-                      c->cfg.m2l_mode, direct_threshold(c->cfg), oo, st, c->stats, c->ev, c->cfg.adaptive_leaf,
+                      c->cfg.m2l_mode, direct_threshold(c->cfg), oo, st, c->stats, ev, c->cfg.adaptive_leaf,
                       c->cfg.p2p_chunk, c->cfg.m2l_run);
   c->stats.direct_max = direct_threshold(c->cfg);
   if (rc) return rc;
@@ -254,6 +258,7 @@ static int pass(fmm_ctx *c, int64_t n, const double *d_pos, const double *d_mass
   c->stats.n_levels = c->tree.depth + 1;
   c->stats.n_leaves = c->tree.level_count[c->tree.depth];
   c->timing_pending = true;
+  c->times_recorded = c->phase_times;
   return FMM_OK;
 }
 
@@ -340,6 +345,10 @@ static int finish(fmm_ctx *c, cudaStream_t st) {
     c->stats.far_direct_pairs = (int64_t)cnt[3];
     c->stats.m2l_tiles = (int64_t)cnt[2];
     c->stats.m2l_width_sum = (int64_t)cnt[5];
+    c->timing_pending = false;
+  }
+  if (c->times_recorded) {
+    c->times_recorded = false;
     float ms[5] = {0, 0, 0, 0, 0};
     for (int i = 0; i < 5; ++i) cudaEventElapsedTime(&ms[i], c->ev[i], c->ev[i + 1]);
     c->stats.ms_tree = ms[0];
@@ -353,7 +362,6 @@ static int finish(fmm_ctx *c, cudaStream_t st) {
     float tot = 0;
     cudaEventElapsedTime(&tot, c->ev[0], c->ev[5]);
     c->stats.ms_total = tot;
-    c->timing_pending = false;
   }
   if (herr & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
   if (herr & FMM_DEV_ERR_NONFINITE_OUTPUT) return FMM_ERR_NONFINITE_OUTPUT;
@@ -387,6 +395,7 @@ int fmm_evaluate_batched(fmm_ctx *c, int32_t nsys, const int64_t *offsets, const
     fmm_ctx *w = nullptr;
     int rc = fmm_create(&wc, &w);
     if (rc) return rc;
+    w->phase_times = false;
     c->workers.push_back(w);
   }
   const int dim = c->cfg.dim;
@@ -624,7 +633,20 @@ static int integrate(fmm_ctx *c, int32_t method, double dt, int32_t steps, int64
   CUDA_TRY(cudaMemcpyAsync(c->d_vel.ptr, vel, sizeof(double) * nd, cudaMemcpyHostToDevice, c->stream));
   double *x = c->d_pos.ptr, *v = c->d_vel.ptr, *a = c->d_acc.ptr;
   cudaStream_t st = c->stream;
+  // SE steps without frames: the error word stays up from pass to pass and is
+  // read with the next pass's box, so that only the last step is waited for;
+  // phase times are those of the last pass
+  const bool carry = method == FMM_INT_SYMPLECTIC_EULER && !frames;
+  struct Restore {
+    fmm_ctx *c;
+    ~Restore() {
+      c->ws.keep_err = false;
+      c->phase_times = true;
+    }
+  } restore{c};
   for (int s = 0; s < steps; ++s) {
+    c->ws.keep_err = carry && s > 0;
+    c->phase_times = !carry || s == steps - 1;
     if (frames && s % every == 0) {  // no acceleration before the first step: zeros
       rc = fmm_frames_write_device(frames, n, x, v, s ? a : nullptr, c->d_mass.ptr, step0 + s, t0 + s * dt, st);
       if (rc) return rc;
@@ -650,6 +672,7 @@ static int integrate(fmm_ctx *c, int32_t method, double dt, int32_t steps, int64
       if (rc) return rc;
       rk4_final(x, v, a, vs, c->d_asum.ptr, c->d_vsum.ptr, nd, dt, st, c->ws.launches);
     }
+    if (carry && s < steps - 1) continue;
     rc = finish(c, st);
     if (rc) return rc;
   }

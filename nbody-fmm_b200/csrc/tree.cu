@@ -861,7 +861,8 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   const int nblv = cdiv(n, LV_TILE);
   if (!ws.reserve_particles(n) || !ws.blev.reserve((size_t)nblv * (Dmax + 1))) return FMM_ERR_OUT_OF_MEMORY;
   uint32_t *lev = ws.lev;  // cells, then the largest cell, of every level
-  CUDA_TRY(cudaMemsetAsync(lev, 0, offsetof(TreeBack, ticket) - offsetof(TreeBack, lev), st));  // and the error word
+  const size_t cleared = ws.keep_err ? offsetof(TreeBack, err) : offsetof(TreeBack, ticket);  // with the error word
+  CUDA_TRY(cudaMemsetAsync(lev, 0, cleared - offsetof(TreeBack, lev), st));
   k_aabb<<<std::min(nbN, WS_AABB_BLOCKS), TPB, 0, st>>>(d_pos, d_mass, n, dim, ws.box_u64, ws.ticket, ws.geom,
                                                        ws.dev_err);
   k_keys<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, ws.geom, ws.keyA, ws.valA);
@@ -877,7 +878,10 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   CUDA_TRY(cudaMemcpyAsync(&ws.host->tree, ws.bback.ptr, sizeof(TreeBack), cudaMemcpyDeviceToHost, st));
   CUDA_TRY(cudaStreamSynchronize(st));
   const uint32_t *hlev = ws.host->tree.lev;
-  if (ws.host->tree.err & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
+  const unsigned int herr = ws.host->tree.err;
+  if (ws.keep_err && (herr & FMM_DEV_ERR_NONFINITE_OUTPUT)) return FMM_ERR_NONFINITE_OUTPUT;  // of the pass before
+  if (ws.keep_err && (herr & FMM_DEV_ERR_TIMEOUT)) return FMM_ERR_TIMEOUT;
+  if (herr & FMM_DEV_ERR_NONFINITE_INPUT) return FMM_ERR_NONFINITE_INPUT;
   for (int d = 0; d < 3; ++d) {
     t.lo[d] = ws.host->tree.geom[d];
     t.hi[d] = ws.host->tree.geom[3 + d];

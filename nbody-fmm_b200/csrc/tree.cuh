@@ -105,6 +105,7 @@ struct Workspace {
   unsigned long long *counters = nullptr;
   int64_t launches = 0;
   bool ok = true;
+  bool keep_err = false;  // build_tree leaves the error word of the pass before up and reports it
 
   bool init_small() {
     ok &= bbox.reserve(6 * WS_AABB_BLOCKS) && bback.reserve(1) && bcount.reserve(8);

@@ -94,3 +94,23 @@ def test_direct_shapes(n, dim, scale, soft):
     assert rel_l2(some, a) < 1e-12
     assert rel_l2(some_p, p) < 1e-12
     assert rel_l2(every[targets], a) < 1e-12
+
+
+@pytest.mark.parametrize("method", [fmmgpu.FMM_INT_SYMPLECTIC_EULER, fmmgpu.FMM_INT_RK4])
+@pytest.mark.parametrize("steps", [1, 2, 5])
+def test_integrate_reports_nonfinite_forces(method, steps):
+    """Coincident particles in the first step's pass: the call reports the
+    non-finite output whether or not it waits for every step, and the context
+    works on."""
+    pos, m = workloads.uniform_cube(400, seed=3)
+    bad = pos.copy()
+    bad[7] = bad[11]
+    with fmmgpu.Context(dim=3, p=4, leaf_cap=16) as c:
+        with pytest.raises(fmmgpu.FmmError) as e:
+            c.integrate(method, 1e-3, steps, bad, 0 * bad, m)
+        want = fmmgpu.FMM_ERR_NONFINITE_OUTPUT if method == fmmgpu.FMM_INT_SYMPLECTIC_EULER else None
+        assert e.value.code in (want, fmmgpu.FMM_ERR_NONFINITE_INPUT) if want is None else e.value.code == want
+        acc = c.evaluate(pos, m)
+        assert np.all(np.isfinite(acc))
+        x, v, a = c.integrate(method, 1e-3, steps, pos, 0 * pos, m)
+        assert np.all(np.isfinite(x)) and np.all(np.isfinite(a))
