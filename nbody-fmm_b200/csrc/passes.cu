@@ -908,16 +908,17 @@ __device__ void colleague_targets(const P2PArgs &a, const double *xs, float4 *fa
   for (int g0 = 0; g0 < groups; g0 += gpr) {
     const int gi = g0 + lane / Gl, sub = lane % Gl;
     const bool live = gi < groups;
-    float thx[R], tlx[R], thy[R], tly[R], thz[R], tlz[R], ax[R], ay[R], az[R], ph[R];
+    float2 tx[R], ty[R], tz[R];  // hi, lo
+    float ax[R], ay[R], az[R], ph[R];
     int me[R];  // the target's particle index (target 0's for the lanes' padding)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int ti = gi * R + r;
       me[r] = tb + (live && ti < nt ? ti : 0);
-      split_hi_lo(xs[DIM * (size_t)me[r]] - cc.ox, thx[r], tlx[r]);
-      split_hi_lo(xs[DIM * (size_t)me[r] + 1] - cc.oy, thy[r], tly[r]);
-      thz[r] = tlz[r] = 0.f;
-      if (DIM == 3) split_hi_lo(xs[DIM * (size_t)me[r] + 2] - cc.oz, thz[r], tlz[r]);
+      split_hi_lo(xs[DIM * (size_t)me[r]] - cc.ox, tx[r].x, tx[r].y);
+      split_hi_lo(xs[DIM * (size_t)me[r] + 1] - cc.oy, ty[r].x, ty[r].y);
+      tz[r] = make_float2(0.f, 0.f);
+      if (DIM == 3) split_hi_lo(xs[DIM * (size_t)me[r] + 2] - cc.oz, tz[r].x, tz[r].y);
       ax[r] = ay[r] = az[r] = ph[r] = 0.f;
     }
     for (int fb = cc.f0; fb < cc.f1; fb += 32) {
@@ -935,8 +936,8 @@ __device__ void colleague_targets(const P2PArgs &a, const double *xs, float4 *fa
         split_hi_lo(xs[DIM * (size_t)j] - cc.ox, hx, lx);
         split_hi_lo(xs[DIM * (size_t)j + 1] - cc.oy, hy, ly);
         if (DIM == 3) split_hi_lo(xs[DIM * (size_t)j + 2] - cc.oz, hz, lz);
-        s_hi[lane] = make_float4(hx, hy, hz, a.part[j].w);
-        s_lo[lane] = make_float4(lx, ly, lz, __int_as_float(j));
+        s_hi[lane] = make_float4(-hx, -lx, -hy, -ly);
+        s_lo[lane] = make_float4(-hz, -lz, a.part[j].w, __int_as_float(j));
       }
       __syncwarp();
       const int cnt = min(32, cc.f1 - fb);
@@ -947,10 +948,9 @@ __device__ void colleague_targets(const P2PArgs &a, const double *xs, float4 *fa
 #pragma unroll
           for (int r = 0; r < R; ++r) {
             if (j == me[r]) continue;
-            const float rx = (thx[r] - q.x) + (tlx[r] - ql.x);
-            const float ry = (thy[r] - q.y) + (tly[r] - ql.y);
-            const float rz = (thz[r] - q.z) + (tlz[r] - ql.z);
-            pair_acc<DIM, false, POT>(rx, ry, rz, q.w, a.eps2, ax[r], ay[r], az[r], ph[r]);
+            const float2 dx = __fadd2_rn(tx[r], make_float2(q.x, q.y)), dy = __fadd2_rn(ty[r], make_float2(q.z, q.w)),
+                         dz = __fadd2_rn(tz[r], make_float2(ql.x, ql.y));
+            pair_acc<DIM, false, POT>(dx.x + dx.y, dy.x + dy.y, dz.x + dz.y, ql.z, a.eps2, ax[r], ay[r], az[r], ph[r]);
           }
         }
       } else {
@@ -958,10 +958,9 @@ __device__ void colleague_targets(const P2PArgs &a, const double *xs, float4 *fa
           const float4 q = s_hi[k], ql = s_lo[k];
 #pragma unroll
           for (int r = 0; r < R; ++r) {
-            const float rx = (thx[r] - q.x) + (tlx[r] - ql.x);
-            const float ry = (thy[r] - q.y) + (tly[r] - ql.y);
-            const float rz = (thz[r] - q.z) + (tlz[r] - ql.z);
-            pair_acc<DIM, false, POT>(rx, ry, rz, q.w, a.eps2, ax[r], ay[r], az[r], ph[r]);
+            const float2 dx = __fadd2_rn(tx[r], make_float2(q.x, q.y)), dy = __fadd2_rn(ty[r], make_float2(q.z, q.w)),
+                         dz = __fadd2_rn(tz[r], make_float2(ql.x, ql.y));
+            pair_acc<DIM, false, POT>(dx.x + dx.y, dy.x + dy.y, dz.x + dz.y, ql.z, a.eps2, ax[r], ay[r], az[r], ph[r]);
           }
         }
       }
@@ -1276,10 +1275,11 @@ __device__ __noinline__ void direct_split(const DirectArgs &a, const float4 *off
 }
 
 template <int DIM, bool POT, bool LIST, bool SPLIT>
-__global__ void __launch_bounds__(256, 4) k_direct_far(DirectArgs a) {
+__global__ void __launch_bounds__(256, DIM == 3 ? 4 : 6) k_direct_far(DirectArgs a) {
   constexpr int NS = DIM == 3 ? 27 : 9, NC = 1 << DIM, NCAND = NS * NC, NR = (NCAND + 31) / 32;
-  __shared__ float4 s_cell_all[8][189];
-  __shared__ int s_pref_all[8][190];
+  constexpr int NSRC = DIM == 3 ? 189 : 27;  // interaction-list offsets
+  __shared__ float4 s_cell_all[8][NSRC];
+  __shared__ int s_pref_all[8][NSRC + 1];
   __shared__ float4 s_stage_all[8][32];
   __shared__ int s_dir_all[8][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
