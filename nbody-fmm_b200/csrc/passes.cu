@@ -621,6 +621,7 @@ __device__ inline void red_add4(float4 *p, float x, float y, float z, float w) {
 
 struct P2PArgs {
   int leaf_first, nleaves, depth;
+  int parts, chunk;  // k_p2p: warps per leaf, taking `chunk` of its targets at a time in turn
   const int *pbeg, *pend, *coll, *parent, *child, *leaf_of;
   const uint64_t *ckey;
   const float4 *part, *part_lo, *far;
@@ -800,10 +801,12 @@ __global__ void __launch_bounds__(256, 4) k_p2p(P2PArgs a) {
   __shared__ int2 s_cell_all[8][NS];
   __shared__ int s_pref_all[8][NS + 1];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int part = a.parts > 1 ? (int)(w % a.parts) : 0, wl = (int)(a.parts > 1 ? w / a.parts : w);
   if (wl >= a.nleaves) return;
   const int g = a.leaf_first + wl;
-  const int tb = a.pbeg[g], nt = a.pend[g] - tb;
+  const int lb = a.pbeg[g], le = a.pend[g];
+  if (part > 0 && (int64_t)part * a.chunk >= le - lb) return;
   const int C = lane < NS ? a.coll[(int64_t)g * NS + lane] : -1;
   const int cb = C >= 0 ? a.pbeg[C] : 0, cn = C >= 0 ? a.pend[C] - cb : 0;
   int x = cn;
@@ -825,16 +828,20 @@ __global__ void __launch_bounds__(256, 4) k_p2p(P2PArgs a) {
   const float2 h[3] = {make_float2((float)a.hx, (float)(a.hx - (double)(float)a.hx)),
                        make_float2((float)a.hy, (float)(a.hy - (double)(float)a.hy)),
                        make_float2((float)a.hz, (float)(a.hz - (double)(float)a.hz))};
-  int Gl = 1;
-  bool bad;
-  switch (best_shape(nt, Gl)) {
-    case 1: bad = near_targets<1, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
-    case 2: bad = near_targets<2, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
-    case 3: bad = near_targets<3, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
-    default: bad = near_targets<4, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+  bool bad = false;
+  for (int64_t t0 = lb + (int64_t)part * a.chunk; t0 < le; t0 += (int64_t)a.parts * a.chunk) {
+    const int tb = (int)t0, nt = min(a.chunk, le - tb);
+    int Gl = 1;
+    switch (best_shape(nt, Gl)) {
+      case 1: bad |= near_targets<1, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+      case 2: bad |= near_targets<2, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+      case 3: bad |= near_targets<3, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+      default: bad |= near_targets<4, DIM, POT>(a, tb, nt, Gl, nl, h, s_hi_all[wib], s_lo_all[wib], lane); break;
+    }
   }
   if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(a.err, FMM_DEV_ERR_NONFINITE_OUTPUT);
-  if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * (total - 1)));
+  if (lane == 0 && a.pair_count && part == 0)
+    atomicAdd(a.pair_count, (unsigned long long)((long long)(le - lb) * (total - 1)));
 }
 
 // The 2D near field of small leaves: eight lanes per leaf, each with every
@@ -2678,7 +2685,15 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   pa.pot = d_pot;
   pa.err = ws.dev_err;
   pa.pair_count = ws.counters + 1;
-  const int pgrid = cdiv((int64_t)pa.nleaves * 32, TPB);
+  // one warp per leaf, or in systems of few leaves (where a full leaf's warp
+  // outlasts the kernel) one per 16 targets
+  pa.parts = 1;
+  pa.chunk = t.level_max[D];
+  if (pa.nleaves <= 65536 && t.level_max[D] > 32) {
+    pa.chunk = 16;
+    pa.parts = std::min(cdiv(t.level_max[D], pa.chunk), 16);
+  }
+  const int pgrid = cdiv((int64_t)pa.nleaves * pa.parts * 32, TPB);
   if (adaptive) {
     // every particle lies in exactly one adaptive leaf: its colleague sums
     // add into far, then every particle's output is written
