@@ -784,18 +784,20 @@ __global__ void k_adaptive_flags(const int *pbeg, const int *pend, const int *pa
 // With adaptive targets (aflag set) only target cells get a row: nothing
 // reads the row of a cell that is no target (their parents' rows serve the
 // targets, and a target's parent is a target).
-__global__ void k_colleagues(const uint64_t *ckey, const int *cparent, const int *cchild, int *ccoll, int base,
-                             int count, int dim, const uint8_t *aflag, int cell0) {
-  // blocks of 8 cells x ns slots, one thread per (cell, slot): consecutive
-  // threads write consecutive slots
-  const int nc = 1 << dim, ns = dim == 3 ? 27 : 9;
-  const int ci = blockIdx.x * 8 + (int)threadIdx.x / ns, s = (int)threadIdx.x % ns;
+template <int DIM>
+__global__ void __launch_bounds__(256) k_colleagues(const uint64_t *ckey, const int *cparent, const int *cchild,
+                                                    int *ccoll, int base, int count) {
+  // one thread per (cell, slot): consecutive threads write consecutive slots.  (Blocks of 8 cells' slots, 72
+  // threads in 2D, spent their time on the launch of blocks: 728 us for the 7.3 M cells of a 4M disk.)
+  constexpr int NC = 1 << DIM, NS = DIM == 3 ? 27 : 9;
+  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int ci = (int)(idx / NS), s = (int)(idx % NS);
   if (ci >= count) return;
   const int c = base + ci;
-  if (aflag && !(aflag[c - cell0] & 1)) return;
-  const int b = (int)(ckey[c] & (uint64_t)(nc - 1));
+  const int b = (int)(ckey[c] & (uint64_t)(NC - 1));
   int pslot = 0, child = 0, mul = 1;
-  for (int a = 0; a < dim; ++a) {
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
     const int delta = (s / mul) % 3 - 1;
     const int v = ((b >> a) & 1) + delta;  // in [-1, 2]
     const int f = (v + 2) / 2 - 1;        // floor(v / 2)
@@ -803,8 +805,8 @@ __global__ void k_colleagues(const uint64_t *ckey, const int *cparent, const int
     child |= (v - 2 * f) << a;
     mul *= 3;
   }
-  const int Q = ccoll[(int64_t)cparent[c] * ns + pslot];
-  ccoll[(int64_t)c * ns + s] = Q >= 0 ? cchild[(int64_t)Q * nc + child] : -1;
+  const int Q = ccoll[(int64_t)cparent[c] * NS + pslot];
+  ccoll[(int64_t)c * NS + s] = Q >= 0 ? cchild[(int64_t)Q * NC + child] : -1;
 }
 
 // The same rows with adaptive targets, one thread per cell: most cells of the
@@ -987,9 +989,8 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
       k_colleagues_targets<3><<<cdiv(t.level_count[d], TPB), TPB, 0, st>>>(
           ws.cell_key, ws.cell_parent, ws.cell_child, ws.cell_coll, t.level_off[d], t.level_count[d], aflag, t.cell0);
     else
-      k_colleagues<<<cdiv(t.level_count[d], 8), 8 * ns, 0, st>>>(ws.cell_key, ws.cell_parent, ws.cell_child,
-                                                                  ws.cell_coll, t.level_off[d], t.level_count[d], dim,
-                                                                  nullptr, t.cell0);
+      (dim == 3 ? k_colleagues<3> : k_colleagues<2>)<<<cdiv((int64_t)t.level_count[d] * ns, 256), 256, 0, st>>>(
+          ws.cell_key, ws.cell_parent, ws.cell_child, ws.cell_coll, t.level_off[d], t.level_count[d]);
     ws.launches += 1;
   }
   // particles in leaf order
