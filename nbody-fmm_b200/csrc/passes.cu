@@ -2601,6 +2601,7 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     k_colleague_count<<<cdiv(ncell, TPB), TPB, 0, st>>>(ws.alist, acount, ncell, ws.cell_coll, ws.cell_pbeg,
                                                          ws.cell_pend, dim == 3 ? 27 : 9, cl_chunk, ccnt);
     exclusive_scan(ws, ccnt, coff, ncell, cnt + D + 1, st);
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
     ws.launches += D;
     CUDA_TRY(cudaMemcpyAsync(ws.host->ntgt, cnt, sizeof(unsigned) * (D + 2), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));

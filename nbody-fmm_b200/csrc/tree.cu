@@ -116,6 +116,7 @@ void exclusive_scan(Workspace &ws, const uint32_t *in, uint32_t *out, int64_t n,
                     cudaStream_t st) {
   int nb = (int)std::max<int64_t>(1, (n + SCAN_TILE - 1) / SCAN_TILE);
   uint32_t *sums = ws.scan_tmp(nb);
+  if (!ws.ok) return;  // out of memory: the caller looks at ws.ok
   // k_scan_reduce uses a strided tile layout and k_scan_apply a blocked one;
   // both cover the same SCAN_TILE elements per block, so the sums agree.
   // Up to 2048 blocks (4M elements) adding the sums up in every block is
@@ -337,9 +338,11 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    uint32_t *chist = ws.radix_hist(nc);
+    if (!ws.ok) return;
     auto kern = rounds == 2 ? k_sort_cluster<2> : rounds == 4 ? k_sort_cluster<4> : rounds == 8 ? k_sort_cluster<8>
                                                                                               : k_sort_cluster<16>;
-    cudaLaunchKernelEx(&cfg, kern, keys, vals, keys_alt, vals_alt, (int)n, bits, ws.radix_hist(nc));
+    cudaLaunchKernelEx(&cfg, kern, keys, vals, keys_alt, vals_alt, (int)n, bits, chist);
     ws.launches += 1;
     if (((bits + 7) / 8) & 1) {
       std::swap(keys, keys_alt);
@@ -349,10 +352,12 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
   }
   int nb = (int)((n + RS_TILE - 1) / RS_TILE);
   uint32_t *hist = ws.radix_hist(nb);
+  if (!ws.ok) return;
   const bool by_tile = nb <= RS_FUSED_TILES;
   for (int shift = 0; shift < bits; shift += 8) {
     k_radix_hist<<<nb, RS_BLOCK, 0, st>>>(keys, n, shift, hist, nb, by_tile);
     if (!by_tile) exclusive_scan(ws, hist, hist, (int64_t)256 * nb, nullptr, st);
+    if (!ws.ok) return;
     k_radix_scatter<<<nb, RS_BLOCK, 0, st>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, nb, by_tile);
     ws.launches += 2;
     std::swap(keys, keys_alt);
@@ -449,9 +454,11 @@ void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int 
   const int nb = (int)std::max<int64_t>(1, (n + RS_TILE - 1) / RS_TILE);
   const bool by_tile = nb <= RS_FUSED_TILES;
   uint32_t *hist = ws.radix_hist(nlist * nb);
+  if (!ws.ok) return;
   const dim3 grid(nb, nlist);
   k_bucket_hist<<<grid, RS_BLOCK, 0, st>>>(keys, n, hist, nb, by_tile, counts);
   if (!by_tile) exclusive_scan(ws, hist, hist, (int64_t)256 * nb * nlist, nullptr, st);
+  if (!ws.ok) return;
   k_bucket_scatter<<<grid, RS_BLOCK, 0, st>>>(keys, n, hist, nb, by_tile, first, out);
   ws.launches += 2;
 }
@@ -905,6 +912,7 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   uint64_t *kA = ws.keyA, *kB = ws.keyB;
   uint32_t *vA = ws.valA, *vB = ws.valB;
   radix_sort(ws, kA, vA, kB, vB, n, dim * Dmax, st);
+  if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
   k_levels<<<nblv, LV_BLOCK, 0, st>>>(kA, n, dim, Dmax, nblv, ws.blev.ptr, lev);
   ws.launches += 1;
   // the box, the finiteness check (keys of non-finite positions are clamped
@@ -970,6 +978,7 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
     k_leafkeys_input<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, D, ws.geom, ws.keyC, ws.valC);
     ws.launches += 1;
     radix_sort(ws, lk, pv, lkAlt, pvAlt, n, dim * D, st);
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
   }
   t.d_perm = pv;
   // adaptive targets (3D trees of depth >= 3, as the force pass runs them):
