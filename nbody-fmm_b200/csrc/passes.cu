@@ -1425,11 +1425,12 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 4 : 6) k_direct_far(DirectArgs
   __shared__ float4 s_stage_all[8][32];
   __shared__ int s_dir_all[8][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int wl = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  // (64 bits: a flattened box with a dense clump has more than 2^27 warps, 2^32 threads)
+  const int64_t wl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (wl >= a.w0[a.nlev]) return;
   int lv = a.nlev - 1;  // deep levels, which hold most of the warps, first
   while (wl < a.w0[lv]) --lv;
-  int ci = wl - a.w0[lv], part = 0;
+  int ci = (int)(wl - a.w0[lv]), part = 0;
   const int parts = SPLIT ? a.parts[lv] : 1;
   if (SPLIT && parts > 1) {
     part = ci % parts;
