@@ -17,7 +17,9 @@ static constexpr int DS_THREADS = 256, DS_R = 2, DS_TARGETS = DS_THREADS * DS_R;
 // reciprocal square root, of r^2 (r^2 + 1e-4)^2, while that product stays
 // well inside the FP64 range (r^2 in [2^-300, 2^300), tested on the exponent
 // bits; outside, the two divisions and the square root), and nothing is
-// computed for a potential that is not asked for.
+// computed for a potential that is not asked for.  The mass is the last
+// factor of both, so that a force that leaves the range does not take a
+// potential with it that is still inside.
 template <int DIM, int SOFT, bool POT>
 __device__ __forceinline__ void direct_pair(double r2, double w, double eps2, double &f, double &pw) {
   if (DIM == 3) {
@@ -25,8 +27,9 @@ __device__ __forceinline__ void direct_pair(double r2, double w, double eps2, do
       const double s = r2 + 1.0e-4;
       const unsigned ex = (unsigned)__double2hiint(r2) >> 20;
       if (ex - 723u < 600u) {
-        f = w * rsqrt(r2 * s * s);
-        if (POT) pw = f * s;
+        const double g = rsqrt(r2 * s * s);
+        f = w * g;
+        if (POT) pw = w * (g * s);
       } else {
         const double r = sqrt(r2);
         f = w / (s * r);

@@ -96,6 +96,20 @@ def test_direct_shapes(n, dim, scale, soft):
     assert rel_l2(every[targets], a) < 1e-12
 
 
+# NaiveUpdate's softening with masses at which the force turns subnormal or leaves the FP64 range, the potential not
+@pytest.mark.parametrize("scale,mass", [(1e40, 1e-200), (1e-44, 2e261)])
+def test_direct_potential_beyond_the_force_range(scale, mass):
+    rng = np.random.default_rng(2)
+    pos, m = rng.random((30, 3)) * scale, (0.5 + rng.random(30)) * mass
+    targets = np.arange(30)
+    with np.errstate(all="ignore"):
+        _, want = _direct(pos, m, targets, fmmgpu.FMM_SOFT_NAIVE_REF, 0.0)
+    with fmmgpu.Context(dim=3) as c:
+        _, pot = c.direct(pos, m, soft_mode=fmmgpu.FMM_SOFT_NAIVE_REF, want_pot=True)
+    unit = mass / scale  # (the norm's squares would leave the range themselves)
+    assert rel_l2(pot / unit, want / unit) < 1e-12
+
+
 @pytest.mark.parametrize("method", [fmmgpu.FMM_INT_SYMPLECTIC_EULER, fmmgpu.FMM_INT_RK4])
 @pytest.mark.parametrize("steps", [1, 2, 5])
 def test_integrate_reports_nonfinite_forces(method, steps):
