@@ -444,7 +444,7 @@ int fmm_evaluate_batched(fmm_ctx *c, int32_t nsys, const int64_t *offsets, const
     c->stats.n_leaves += x.n_leaves;
   }
   c->stats.ms_total = wall;
-  c->timing_pending = false;
+  c->timing_pending = c->times_recorded = false;  // of a pass before this call: its statistics are replaced
   return err.load();
 }
 

@@ -57,3 +57,23 @@ def test_batched_rejects_bad_offsets():
         with pytest.raises(fmmgpu.FmmError) as e:
             c.evaluate_batched(np.array([0, 5, 3], np.int64), None, None, None)
         assert e.value.code == fmmgpu.FMM_ERR_INVALID_ARGUMENT
+
+
+def test_batched_statistics_stay_when_the_host_waits():
+    """The context's statistics are those of the batched call, also after a
+    wait for the context, where a pass that nobody waited for came before."""
+    torch = pytest.importorskip("torch")
+    dev = torch.device("cuda", 0)
+    sizes = [700, 900]
+    pos, mass = _ensemble(sizes, 60)
+    off = np.r_[0, np.cumsum(sizes)].astype(np.int64)
+    d_pos, d_m = torch.from_numpy(pos).to(dev), torch.from_numpy(mass).to(dev)
+    d_acc = torch.empty_like(d_pos)
+    torch.cuda.synchronize()
+    with fmmgpu.Context(dim=3, p=4, leaf_cap=32, m2l_mode=fmmgpu.FMM_M2L_TC) as c:
+        c.evaluate_device(700, d_pos.data_ptr(), d_m.data_ptr(), d_acc.data_ptr())
+        c.evaluate_batched(off, d_pos.data_ptr(), d_m.data_ptr(), d_acc.data_ptr(), workers=1)
+        before = c.stats()
+        c.synchronize()
+        after = c.stats()
+    assert before == after
