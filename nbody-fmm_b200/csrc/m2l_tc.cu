@@ -47,9 +47,9 @@
 // Shared-memory operands use the K-major layout without swizzle: 8-row x
 // 16-byte core matrices, rows of a core matrix contiguous, 8-row groups
 // SBO = 128 B apart and 16-byte K chunks LBO apart.  Every wait on an
-// mbarrier gives up after about a second; the kernel then flags the device
-// error word, drains its copies (again with a limit), releases its TMEM and
-// returns.
+// mbarrier gives up after about a second; the kernel then issues nothing more,
+// flags the device error word, waits for its MMAs and copies in flight (again
+// with a limit), releases its TMEM and returns.
 #include <algorithm>
 #include <mutex>
 
@@ -181,8 +181,9 @@ __device__ inline void tc_fence_after() { asm volatile("tcgen05.fence::after_thr
 //
 // Barriers: s_a (the workers have written A and read D), s_full / s_mma (an
 // operator copy has landed in a buffer / its MMAs are done), s_done (the
-// slot's MMAs are done).  A wait that gives up makes its thread skip the rest of the
-// batch; all threads meet at the batch's end and leave together.
+// slot's MMAs are done), s_drain (after a wait that gave up: all MMAs issued are
+// done).  A wait that gives up makes its thread skip the rest of the batch; all
+// threads meet at the batch's end and leave together.
 static constexpr int TC_WORKERS = 256, TC_THREADS = TC_WORKERS + 64, TC_NBUF = 4;
 
 // CTAs per SM: two where shared memory and TMEM (512 columns) hold them, at
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
   extern __shared__ __align__(1024) uint8_t smem[];
   uint16_t *As = (uint16_t *)smem;  // 3 splits
   uint16_t *Bs = As + 3 * ASPLIT;   // TC_NBUF buffers
-  __shared__ __align__(8) uint64_t s_full[TC_NBUF], s_mma[TC_NBUF], s_a, s_done;
+  __shared__ __align__(8) uint64_t s_full[TC_NBUF], s_mma[TC_NBUF], s_a, s_done, s_drain;
   __shared__ uint32_t s_tmem;
   __shared__ short s_slot[2][TC_MAX_SLOTS], s_op[2][TC_MAX_SLOTS];  // 16-bit: two 96-wide CTAs fit an SM
   __shared__ uint8_t s_w[2][TC_MAX_SLOTS];  // padded width of each slot's order
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
     }
     mbar_init(&s_a, TC_WORKERS / 32);
     mbar_init(&s_done, 1);
+    mbar_init(&s_drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   tc_fence_before();
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
             (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(w >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
 #pragma unroll
         for (int s = 2; s >= 0; --s)
-          for (int h = 0; h < np; ++h, ++g) {
+          for (int h = 0; h < np && ok; ++h, ++g) {
             if (!mbar_wait(&s_full[g % TC_NBUF], (g / TC_NBUF) & 1)) {
               ok = false;
               break;
@@ -434,6 +436,12 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
       ok = __syncthreads_and(ok);
       if (!ok) {
         if (!mine) atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
+        // what was issued may still be writing D, in columns that are freed below
+        if (lead) {
+          mma_commit(&s_drain);
+          mbar_wait(&s_drain, 0);
+        }
+        __syncwarp();
         break;
       }
       if (s_n[c ^ 1] == 0) break;
