@@ -321,9 +321,11 @@ __global__ void __launch_bounds__(RS_BLOCK) k_sort_cluster(uint64_t *ka, uint32_
 
 // Sorts (keys, vals) by the low `bits` bits of the key, stably; the result
 // ends in (keys, vals) (the buffers are ping-ponged with the alternates).
-void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
-                int bits, cudaStream_t st) {
-  if (n <= 1 || bits <= 0) return;
+// A cluster launch can be refused for want of resources: nothing may then go
+// on, since the unsorted values would be used as indices.
+int radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
+               int bits, cudaStream_t st) {
+  if (n <= 1 || bits <= 0) return FMM_OK;
   if (n <= (int64_t)RS_BLOCK * 16 * RC_MAX_CLUSTER) {
     int rounds = 2, nc = 1;
     while ((int64_t)RS_BLOCK * rounds * RC_MAX_CLUSTER < n) rounds *= 2;
@@ -339,30 +341,31 @@ void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys
     cfg.attrs = at;
     cfg.numAttrs = 1;
     uint32_t *chist = ws.radix_hist(nc);
-    if (!ws.ok) return;
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
     auto kern = rounds == 2 ? k_sort_cluster<2> : rounds == 4 ? k_sort_cluster<4> : rounds == 8 ? k_sort_cluster<8>
                                                                                               : k_sort_cluster<16>;
-    cudaLaunchKernelEx(&cfg, kern, keys, vals, keys_alt, vals_alt, (int)n, bits, chist);
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, keys, vals, keys_alt, vals_alt, (int)n, bits, chist));
     ws.launches += 1;
     if (((bits + 7) / 8) & 1) {
       std::swap(keys, keys_alt);
       std::swap(vals, vals_alt);
     }
-    return;
+    return FMM_OK;
   }
   int nb = (int)((n + RS_TILE - 1) / RS_TILE);
   uint32_t *hist = ws.radix_hist(nb);
-  if (!ws.ok) return;
+  if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
   const bool by_tile = nb <= RS_FUSED_TILES;
   for (int shift = 0; shift < bits; shift += 8) {
     k_radix_hist<<<nb, RS_BLOCK, 0, st>>>(keys, n, shift, hist, nb, by_tile);
     if (!by_tile) exclusive_scan(ws, hist, hist, (int64_t)256 * nb, nullptr, st);
-    if (!ws.ok) return;
+    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
     k_radix_scatter<<<nb, RS_BLOCK, 0, st>>>(keys, vals, keys_alt, vals_alt, n, shift, hist, nb, by_tile);
     ws.launches += 2;
     std::swap(keys, keys_alt);
     std::swap(vals, vals_alt);
   }
+  return FMM_OK;
 }
 
 // ------------------------------------------------------------ bucket lists
@@ -911,8 +914,8 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   // sort all particles by their Dmax key
   uint64_t *kA = ws.keyA, *kB = ws.keyB;
   uint32_t *vA = ws.valA, *vB = ws.valB;
-  radix_sort(ws, kA, vA, kB, vB, n, dim * Dmax, st);
-  if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
+  int rc = radix_sort(ws, kA, vA, kB, vB, n, dim * Dmax, st);
+  if (rc) return rc;
   k_levels<<<nblv, LV_BLOCK, 0, st>>>(kA, n, dim, Dmax, nblv, ws.blev.ptr, lev);
   ws.launches += 1;
   // the box, the finiteness check (keys of non-finite positions are clamped
@@ -977,8 +980,8 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
     uint32_t *pvAlt = ws.valA;
     k_leafkeys_input<<<nbN, TPB, 0, st>>>(d_pos, n, dim, Dmax, D, ws.geom, ws.keyC, ws.valC);
     ws.launches += 1;
-    radix_sort(ws, lk, pv, lkAlt, pvAlt, n, dim * D, st);
-    if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
+    rc = radix_sort(ws, lk, pv, lkAlt, pvAlt, n, dim * D, st);
+    if (rc) return rc;
   }
   t.d_perm = pv;
   // adaptive targets (3D trees of depth >= 3, as the force pass runs them):
@@ -986,7 +989,7 @@ int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d
   const uint8_t *aflag = nullptr;
   if (adaptive_leaf > 0 && dim == 3 && D >= 3) {
     if (!ws.reserve_adaptive(t.n_cells)) return FMM_ERR_OUT_OF_MEMORY;
-    int rc = launch_adaptive_flags(ws, t, adaptive_leaf, ws.aflag, ws.alist, st);
+    rc = launch_adaptive_flags(ws, t, adaptive_leaf, ws.aflag, ws.alist, st);
     if (rc) return rc;
     ws.launches += 1;
     t.adaptive_leaf = adaptive_leaf;

@@ -197,8 +197,8 @@ struct TreeState {
 
 void exclusive_scan(Workspace &ws, const uint32_t *in, uint32_t *out, int64_t n, uint32_t *total_dev,
                     cudaStream_t st);
-void radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
-                int bits, cudaStream_t st);
+int radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_alt, uint32_t *&vals_alt, int64_t n,
+               int bits, cudaStream_t st);
 void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int first, int *out, uint32_t *counts,
                   cudaStream_t st);
 int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d_mass, int64_t n, int dim,

@@ -28,6 +28,21 @@ def test_tree_at_tile_edges(oracle, n, dim):
         np.testing.assert_array_equal(a, b)
 
 
+# the one-launch sort: 1 to 8 blocks of 2, 4, 8 or 16 items per thread, up to 32,768 items
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("n", [512, 513, 4096, 4097, 8192, 8193, 16384, 16385, 32768, 32769])
+def test_tree_at_sort_edges(oracle, n, dim):
+    gen = workloads.plummer if dim == 3 else workloads.disk_clumps_2d
+    pos = gen(n, seed=32)[0]
+    want = oracle.tree(pos, 16, with_pairs=False)
+    with fmmgpu.Context(dim=dim, leaf_cap=16) as c:
+        got = c.tree(pos, with_pairs=False)
+    for k in ("depth", "leaf_keys", "leaf_start", "perm"):
+        np.testing.assert_array_equal(got[k], want[k])
+    for a, b in zip(got["level_keys"], want["level_keys"]):
+        np.testing.assert_array_equal(a, b)
+
+
 def test_tree_with_many_equal_keys(oracle):
     """More than 512 particles with one key at the maximum depth (the leaf
     order by a sort) next to single ones, and runs across tiles."""
