@@ -62,6 +62,7 @@ struct ExpBuffers {
                            // [2 ncell, 3 ncell) M2L source, [3 ncell, 4 ncell) how M is formed
   DevBuf<int> rows;        // shortcuts: class-grouped cells that need L2L, then the M2M rows
   DevBuf<int> p2m_list;    // shortcuts: the cells whose multipole comes straight from their particles
+  DevBuf<int2> fitems;     // boxes not near a cube: far-field targets of large cells, (cell, part) items
   DevBuf<int4> batches2;   // shortcuts: batches of the cells that need L2L, then of the M2M rows
   HostPinned<int4> hbatches, hbatches2;  // their host staging
   DevBuf<int> esrc;        // L2L shortcut: per leaf, the cell whose local expansion its particles evaluate

@@ -180,6 +180,7 @@ int fmm_destroy(fmm_ctx *c) {
   c->eb.elev.release();
   c->eb.p2m_list.release();
   c->eb.ftl.release();
+  c->eb.fitems.release();
   c->eb.xs.release();
   c->eb.ccnt.release();
   c->eb.citems.release();

@@ -1230,12 +1230,16 @@ static constexpr int DF_MAX_LEVELS = 33;
 
 struct DirectArgs {
   // levels of the launch, coarse first: warps [w0[k], w0[k+1]) take the
-  // cells first[k] + (warp - w0[k]) / parts[k], or with a target list
-  // (k_direct_far's LIST) the cells tlist[first[k] + (warp - w0[k]) / parts[k]];
-  // the parts of a cell take its targets `chunk` at a time in turn
-  int nlev, chunk;
-  int parts[DF_MAX_LEVELS];
+  // cells first[k] + (warp - w0[k]), or with a target list (k_direct_far's
+  // LIST) the cells tlist[first[k] + (warp - w0[k])]
+  int nlev;
   int first[DF_MAX_LEVELS], w0[DF_MAX_LEVELS + 1];
+  // k_direct_far's SPLIT: warp w takes item w of *nitems, (cell, part): the
+  // part'th `chunk` targets of the cell
+  int chunk;
+  const int2 *items;
+  const uint32_t *nitems;
+  int cell[DF_MAX_LEVELS];           // first cell of each level
   const float4 *off[DF_MAX_LEVELS];  // particle offsets from their level-d ancestor's centre
   float h[DF_MAX_LEVELS][3];         // level-d cell size
   const int *pbeg, *pend, *coll, *parent, *child;
@@ -1258,8 +1262,15 @@ struct DirectArgs {
 //
 // With offsets that are not well separated (a box that is not near a cube)
 // whole pairs of coarse cells are summed, and with one warp per cell the
-// kernel waited for a few warps with thousands of targets: there a cell's
-// targets are spread over parts[k] warps.
+// kernel waited for a few warps with thousands of targets: there (SPLIT) every
+// `chunk` targets of a cell are an item of a list in the order of the cells, a
+// warp each.  (As many warps for every cell of a level as for its largest left
+// 94 to 99.8 % of them empty where a box holds a clump: a flattened halo of
+// 60,000 particles with half of them in one cell on ten levels 36.9 ms, now 1.3;
+// a flattened sphere of 2^20 35.5, now 24.1.)  The items come in runs of one
+// cell, whose warps read the same sources; in the order in which atomics drew
+// them that sphere took 42 ms.  Three blocks per SM: at four the loops over
+// thousands of sources spill (32 ms).
 //
 // Per kept source cell si the warp keeps s_pref[si] (its first position in
 // the concatenation; every cell non-empty) and s_cell[si] = (shift c_S - c_T,
@@ -1408,16 +1419,8 @@ __device__ __forceinline__ void direct_targets(const DirectArgs &a, const float4
   }
 }
 
-// The same for a part of a large cell's targets, out of line (the kernel's own
-// copy keeps its registers).
-template <int DIM, bool POT>
-__device__ __noinline__ void direct_split(const DirectArgs &a, const float4 *off, int tb, int nt, const float4 *s_cell,
-                                          const int *s_pref, int nsrc, int lane, float4 *stage) {
-  direct_targets<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, stage);
-}
-
 template <int DIM, bool POT, bool LIST, bool SPLIT>
-__global__ void __launch_bounds__(256, DIM == 3 ? 4 : 6) k_direct_far(DirectArgs a) {
+__global__ void __launch_bounds__(256, SPLIT ? 3 : DIM == 3 ? 4 : 6) k_direct_far(DirectArgs a) {
   constexpr int NS = DIM == 3 ? 27 : 9, NC = 1 << DIM, NCAND = NS * NC, NR = (NCAND + 31) / 32;
   constexpr int NSRC = DIM == 3 ? 189 : 27;  // interaction-list offsets
   __shared__ float4 s_cell_all[8][NSRC];
@@ -1425,21 +1428,23 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 4 : 6) k_direct_far(DirectArgs
   __shared__ float4 s_stage_all[8][32];
   __shared__ int s_dir_all[8][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  // (64 bits: a flattened box with a dense clump has more than 2^27 warps, 2^32 threads)
   const int64_t wl = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (wl >= a.w0[a.nlev]) return;
   int lv = a.nlev - 1;  // deep levels, which hold most of the warps, first
-  while (wl < a.w0[lv]) --lv;
-  int ci = (int)(wl - a.w0[lv]), part = 0;
-  const int parts = SPLIT ? a.parts[lv] : 1;
-  if (SPLIT && parts > 1) {
-    part = ci % parts;
-    ci /= parts;
+  int T, part = 0;
+  if (SPLIT) {
+    if (wl >= *a.nitems) return;
+    const int2 it = a.items[wl];
+    T = it.x;
+    part = it.y;
+    while (T < a.cell[lv]) --lv;
+  } else {
+    if (wl >= a.w0[a.nlev]) return;
+    while (wl < a.w0[lv]) --lv;
+    const int ci = a.first[lv] + (int)(wl - a.w0[lv]);
+    T = LIST ? a.tlist[ci] : ci;
   }
-  const int T = LIST ? a.tlist[a.first[lv] + ci] : a.first[lv] + ci;
   int tb = a.pbeg[T], nt = a.pend[T] - tb;
   if ((long long)nt > a.direct_max && !a.any_fdirect) return;
-  if (SPLIT && part > 0 && (long long)part * a.chunk >= nt) return;
   const float4 *off = a.off[lv];
   float4 *s_cell = s_cell_all[wib];
   int *s_pref = s_pref_all[wib];
@@ -1507,17 +1512,12 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 4 : 6) k_direct_far(DirectArgs
   }
   __syncwarp();
   if (nsrc == 0) return;
-  if (!SPLIT || parts == 1) {
-    if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
-    direct_targets<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, s_stage_all[wib]);
-    return;
+  if (SPLIT) {
+    tb += part * a.chunk;
+    nt = min(a.chunk, nt - part * a.chunk);
   }
-  const int tend = tb + nt;
-  for (tb += part * a.chunk; tb < tend; tb += parts * a.chunk) {
-    nt = min(a.chunk, tend - tb);
-    if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
-    direct_split<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, s_stage_all[wib]);
-  }
+  if (lane == 0 && a.pair_count) atomicAdd(a.pair_count, (unsigned long long)((long long)nt * ptotal));
+  direct_targets<DIM, POT>(a, off, tb, nt, s_cell, s_pref, nsrc, lane, s_stage_all[wib]);
 }
 
 // The 2D far field with small thresholds, eight lanes per target cell.  A 2D
@@ -2110,11 +2110,13 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   const int tchunk = tc ? 128 : CT_TGT;
   const bool split96 = ops.img96 != nullptr;  // M2L tiles up to 96 wide run in a kernel of their own
   // counters that start at zero, in one buffer: bucket sizes of the two list
-  // steps, work counters of the tensor-core launches, listed P2M cells
-  if (!eb.zeros.reserve(1024 + TC_MAX_LAUNCHES + 1)) return FMM_ERR_OUT_OF_MEMORY;
-  CUDA_TRY(cudaMemsetAsync(eb.zeros.ptr, 0, (1024 + TC_MAX_LAUNCHES + 1) * sizeof(uint32_t), st));
+  // steps, work counters of the tensor-core launches, listed P2M cells, items
+  // of the far field
+  if (!eb.zeros.reserve(1024 + TC_MAX_LAUNCHES + 2)) return FMM_ERR_OUT_OF_MEMORY;
+  CUDA_TRY(cudaMemsetAsync(eb.zeros.ptr, 0, (1024 + TC_MAX_LAUNCHES + 2) * sizeof(uint32_t), st));
   uint32_t *const cls_count = eb.zeros.ptr;
-  unsigned int *const tc_work = eb.zeros.ptr + 1024, *const p2m_count = tc_work + TC_MAX_LAUNCHES;
+  unsigned int *const tc_work = eb.zeros.ptr + 1024, *const p2m_count = tc_work + TC_MAX_LAUNCHES,
+               *const far_items = p2m_count + 1;
   int tc_k = 0;  // tensor-core launches so far (work counter index)
   if (tc && D >= 2) {
     if (2 * D + 2 > TC_MAX_LAUNCHES) return FMM_ERR_UNSUPPORTED;
@@ -2646,8 +2648,10 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     // a few thousand warps, up to the 128 of four targets per lane
     da.chunk = n < (1 << 17) ? 32 : n < (1 << 19) ? 64 : 128;
     int64_t nw = 0;
+    int64_t nitems = 0;  // a bound on the items: a level's last parts, then n / chunk full ones
     for (int d = 2; d <= D; ++d) {
       const int k = da.nlev++;
+      da.cell[k] = t.level_off[d];
       const double invd = std::ldexp(1.0, -d);
       da.first[k] = adaptive ? t.level_off[d] - t.level_off[2] : t.level_off[d];
       da.w0[k] = (int)nw;
@@ -2656,12 +2660,19 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
       da.h[k][1] = (float)(g.ext[1] * invd);
       da.h[k][2] = (float)(g.ext[2] * invd);
       const int64_t nc = adaptive ? (int64_t)ntgt[d] : (int64_t)t.level_count[d];
-      const int64_t most = std::max<int64_t>(1, (1 << 25) / std::max<int64_t>(nc, 1));
-      da.parts[k] = any_fdirect ? (int)std::min<int64_t>(cdiv(t.level_max[d], da.chunk), most) : 1;
-      nw += nc * da.parts[k];
+      nw += nc;
+      nitems += nc + std::min(n / da.chunk, nc * ((t.level_max[d] - 1) / da.chunk));
     }
     da.w0[da.nlev] = (int)nw;
-    const int64_t grid = cdiv(nw * 32, TPB);
+    if (any_fdirect) {
+      if (!eb.fitems.reserve((size_t)nitems)) return FMM_ERR_OUT_OF_MEMORY;
+      split_items(ws, adaptive ? ws.aflag : nullptr, cell0, t.level_off[2], t.level_off[D + 1] - t.level_off[2],
+                  da.chunk, eb.fitems.ptr, far_items, st);
+      if (!ws.ok) return FMM_ERR_OUT_OF_MEMORY;
+    }
+    da.items = eb.fitems.ptr;
+    da.nitems = far_items;
+    const int64_t grid = cdiv((any_fdirect ? nitems : nw) * 32, TPB);
     auto pick = [&](auto plain, auto split) { return any_fdirect ? split : plain; };
     void (*kern)(DirectArgs);
     if (adaptive)

@@ -466,6 +466,71 @@ void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int 
   ws.launches += 2;
 }
 
+// ------------------------------------------------------------- split items
+// Parts of at most `chunk` particles of cell first + i, 0 past the end and for
+// a cell without bit 0 of its flag (flag null: every cell).
+__device__ inline uint32_t cell_parts(const uint8_t *flag, int cell0, int first, int64_t i, int64_t count,
+                                      const int *pbeg, const int *pend, int chunk) {
+  const int64_t g = first + i;
+  if (i >= count || (flag && !(flag[g - cell0] & 1))) return 0;
+  return (uint32_t)((pend[g] - pbeg[g] + (int64_t)chunk - 1) / chunk);
+}
+
+__global__ void k_split_reduce(const uint8_t *flag, int cell0, int first, int64_t count, const int *pbeg,
+                               const int *pend, int chunk, uint32_t *sums) {
+  __shared__ uint32_t s_warp[SCAN_BLOCK / 32];
+  uint32_t s = 0, total;
+  for (int q = 0; q < SCAN_ITEMS; ++q)
+    s += cell_parts(flag, cell0, first, (int64_t)blockIdx.x * SCAN_TILE + q * SCAN_BLOCK + threadIdx.x, count, pbeg,
+                    pend, chunk);
+  block_excl_scan(s, s_warp, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+// A thread takes SCAN_ITEMS consecutive cells; cells of more than two parts
+// are written by the whole warp.
+__global__ void k_split_fill(const uint8_t *flag, int cell0, int first, int64_t count, const int *pbeg,
+                             const int *pend, int chunk, const uint32_t *sums, int2 *items, uint32_t *nitems) {
+  __shared__ uint32_t s_warp[SCAN_BLOCK / 32];
+  const int lane = threadIdx.x & 31;
+  uint32_t t = 0, before, total, v[SCAN_ITEMS], s = 0;
+  for (int k = threadIdx.x; k < (int)blockIdx.x; k += SCAN_BLOCK) t += sums[k];
+  block_excl_scan(t, s_warp, before);
+  const int64_t i0 = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+#pragma unroll
+  for (int q = 0; q < SCAN_ITEMS; ++q) s += v[q] = cell_parts(flag, cell0, first, i0 + q, count, pbeg, pend, chunk);
+  uint32_t at = block_excl_scan(s, s_warp, total) + before;
+#pragma unroll
+  for (int q = 0; q < SCAN_ITEMS; ++q) {
+    const int g = (int)(first + i0 + q);
+    if (v[q] >= 1 && v[q] <= 2) items[at] = make_int2(g, 0);
+    if (v[q] == 2) items[at + 1] = make_int2(g, 1);
+    for (unsigned m = __ballot_sync(0xffffffffu, v[q] > 2); m; m &= m - 1) {
+      const int b = __ffs(m) - 1, gb = __shfl_sync(0xffffffffu, g, b);
+      const uint32_t cb = __shfl_sync(0xffffffffu, v[q], b), ab = __shfl_sync(0xffffffffu, at, b);
+      for (uint32_t k = lane; k < cb; k += 32) items[ab + k] = make_int2(gb, (int)k);
+    }
+    at += v[q];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *nitems = before + total;
+}
+
+// The list of (cell, part) of the cells [first, first + count), parts of at
+// most `chunk` particles, in the order of the cells; *nitems its length.  The
+// counts are formed again for the second launch instead of stored, and up to
+// 2048 cells take one launch: small systems are bound by launches.
+void split_items(Workspace &ws, const uint8_t *flag, int cell0, int first, int64_t count, int chunk, int2 *items,
+                 uint32_t *nitems, cudaStream_t st) {
+  const int nb = (int)std::max<int64_t>(1, (count + SCAN_TILE - 1) / SCAN_TILE);
+  uint32_t *sums = ws.scan_tmp(nb);
+  if (!ws.ok) return;
+  if (nb > 1)
+    k_split_reduce<<<nb, SCAN_BLOCK, 0, st>>>(flag, cell0, first, count, ws.cell_pbeg, ws.cell_pend, chunk, sums);
+  k_split_fill<<<nb, SCAN_BLOCK, 0, st>>>(flag, cell0, first, count, ws.cell_pbeg, ws.cell_pend, chunk, sums, items,
+                                          nitems);
+  ws.launches += nb > 1 ? 2 : 1;
+}
+
 // ------------------------------------------------------------ tree kernels
 // AABB (tree.cpp:20-30) plus a finiteness check of positions and masses.
 // Every block writes its box to part[block][6]; the last one to finish (a

@@ -201,6 +201,8 @@ int radix_sort(Workspace &ws, uint64_t *&keys, uint32_t *&vals, uint64_t *&keys_
                int bits, cudaStream_t st);
 void bucket_lists(Workspace &ws, const uint8_t *keys, int nlist, int64_t n, int first, int *out, uint32_t *counts,
                   cudaStream_t st);
+void split_items(Workspace &ws, const uint8_t *flag, int cell0, int first, int64_t count, int chunk, int2 *items,
+                 uint32_t *nitems, cudaStream_t st);
 int build_tree(Workspace &ws, TreeState &t, const double *d_pos, const double *d_mass, int64_t n, int dim,
                int threshold, cudaStream_t st, int adaptive_leaf = 0);
 // Adaptive-target flags of every cell of a built tree into flag[0 .. n_cells)

@@ -56,7 +56,7 @@ def test_tree_with_many_equal_keys(oracle):
         np.testing.assert_array_equal(got[k], want[k])
 
 
-# boxes far from a cube: whole cell pairs are summed directly, large cells by several warps (32, 64 or 128 targets each)
+# boxes far from a cube: whole cell pairs are summed directly, large cells by several warps (32 targets each)
 # (adaptive targets need a tree of depth 3: from 6000 particles)
 @pytest.mark.parametrize("n,adaptive", [(700, 0), (6000, 0), (20000, 0), (6000, 32), (20000, 32)])
 @pytest.mark.parametrize("stretch", [(1.0, 0.7, 1.0), (1.0, 0.45, 0.6)])
@@ -166,3 +166,48 @@ def test_clump_in_flat_halo(oracle):
     want = oracle.fmm(pos, m, 6, 64, direct_max=128)
     assert rel_l2(acc[n // 2:], want[n // 2:]) < 1e-6
     assert rel_l2(acc[: n // 2], want[: n // 2]) < 1e-6
+
+
+def test_clump_in_flat_halo_launches_no_empty_warps():
+    """The far field of such a box costs what its pairs cost: here at least
+    2e11 pairs/s (a fifth of the rate in boxes without a clump) after 1 ms,
+    where warps for every cell as for the largest took 37 ms."""
+    n = 60000
+    pos, m = _clump_in_flat_halo(n, 1e-4)
+    with fmmgpu.Context(dim=3, p=8, leaf_cap=64, m2l_mode=fmmgpu.FMM_M2L_TC) as c:
+        ms = []
+        for _ in range(4):
+            c.evaluate(pos, m)
+            st = c.stats()
+            ms.append(st["ms_far_direct"])
+    assert min(ms) < 1.0 + st["far_direct_pairs"] / 2e11 * 1e3
+
+
+# 64 and 128 targets per warp, lists of one, a few and hundreds of tiles of 2048 cells (p = 8 truncates to 2e-5 to 6e-5
+# here, in FP64 as well)
+@pytest.mark.parametrize("n,adaptive", [((1 << 17) + 1, 0), ((1 << 19) + 1, 0), ((1 << 19) + 1, 32)])
+def test_flattened_sphere_against_direct(oracle, n, adaptive):
+    pos, m = workloads.plummer(n, seed=8)
+    pos = pos * np.array([1.0, 1.0, 0.8])
+    with fmmgpu.Context(dim=3, p=8, leaf_cap=64, m2l_mode=fmmgpu.FMM_M2L_TC, adaptive_leaf=adaptive) as c:
+        acc, pot = c.evaluate(pos, m, want_pot=True)
+    some = np.random.default_rng(1).choice(n, 300, replace=False)
+    want, want_pot = oracle.direct(pos, m, targets=some, want_pot=True)
+    assert rel_l2(acc[some], want) < 1e-4
+    assert rel_l2(pot[some], want_pot) < 1e-4
+
+
+@pytest.mark.parametrize("clump", [0.0, 0.5])
+@pytest.mark.parametrize("n", [100, 3000, 9000])
+def test_elongated_box_2d(oracle, n, clump):
+    rng = np.random.default_rng(n)
+    pos = rng.random((n, 2)) * np.array([1.0, 0.4])
+    k = int(clump * n)
+    pos[:k] = np.array([0.3, 0.12]) + 1e-3 * rng.normal(size=(k, 2))
+    m = np.full(n, 1.0 / n)
+    with fmmgpu.Context(dim=2, p=10, leaf_cap=16, direct_max=64, m2l_mode=fmmgpu.FMM_M2L_TC) as c:
+        acc, pot = c.evaluate(pos, m, want_pot=True)
+    want, want_pot = oracle.fmm(pos, m, 10, 16, direct_max=64, want_pot=True)
+    assert rel_l2(acc[k:], want[k:]) < 1e-6
+    assert rel_l2(acc, want) < 1e-6
+    assert rel_l2(pot, want_pot) < 1e-6
