@@ -111,6 +111,52 @@ def test_direct_shapes(n, dim, scale, soft):
     assert rel_l2(every[targets], a) < 1e-12
 
 
+# one or two targets per thread: around 256 and 512 targets, idle warps, blocks of 512 targets before and after there
+# are 800 (every target checked where there are few, else the ends of the blocks)
+@pytest.mark.parametrize("n,nt,dim", [(3000, 1, 3), (3000, 33, 3), (3000, 256, 3), (3000, 257, 3), (450000, 385, 3),
+                                      (450000, 384, 3), (120000, 1920, 2), (14000, 14000, 3), (15000, 15000, 3)])
+@pytest.mark.parametrize("soft", [fmmgpu.FMM_SOFT_PLUMMER, fmmgpu.FMM_SOFT_NAIVE_REF])
+def test_direct_target_blocks(n, nt, dim, soft):
+    rng = np.random.default_rng(nt)
+    pos, m = rng.random((n, dim)), rng.random(n)
+    targets = rng.permutation(n)[:nt]
+    look = np.unique(np.clip(np.r_[np.arange(0, nt, max(1, nt // 16)), np.arange(0, nt + 1, 256) - 1, nt - 1], 0, nt - 1))
+    a, p = _direct(pos, m, targets[look], soft, 0.0)
+    with fmmgpu.Context(dim=dim) as c:
+        acc, pot = c.direct(pos, m, targets=targets, soft_mode=soft, want_pot=True)
+        plain = c.direct(pos, m, targets=targets, soft_mode=soft)
+    assert rel_l2(acc[look], a) < 1e-12
+    assert rel_l2(pot[look], p) < 1e-12
+    assert rel_l2(plain, acc) < 1e-12
+
+
+def test_direct_of_few_targets_takes_less_than_of_many():
+    """One target, 256 and 512 of 2^20 particles: idle threads cost nothing,
+    so 256 take at most three quarters of the time of 512, and one at most
+    half (the idle halves of blocks of 512 took as long as full ones)."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 20
+    g = torch.Generator(device="cuda").manual_seed(3)
+    pos = torch.rand(n, 3, generator=g, device="cuda", dtype=torch.float64)
+    mass = torch.full((n,), 1.0 / n, device="cuda", dtype=torch.float64)
+    acc = torch.empty(512, 3, device="cuda", dtype=torch.float64)
+    stream = torch.cuda.Stream()
+    ms = {}
+    with fmmgpu.Context(dim=3) as c, torch.cuda.stream(stream):
+        for nt in (1, 256, 512):
+            times = []
+            for _ in range(8):
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record()
+                c.direct_device(n, pos.data_ptr(), mass.data_ptr(), nt, None, acc.data_ptr(), stream=stream.cuda_stream)
+                e1.record()
+                torch.cuda.synchronize()
+                times.append(e0.elapsed_time(e1))
+            ms[nt] = min(times)
+    assert ms[256] < 0.75 * ms[512]
+    assert ms[1] < 0.5 * ms[512]
+
+
 # NaiveUpdate's softening with masses at which the force turns subnormal or leaves the FP64 range, the potential not
 @pytest.mark.parametrize("scale,mass", [(1e40, 1e-200), (1e-44, 2e261)])
 def test_direct_potential_beyond_the_force_range(scale, mass):
