@@ -918,8 +918,21 @@ __device__ __forceinline__ bool near2d_targets(const P2PArgs &a, int tb, int nt,
   return bad;
 }
 
-// Particles per leaf up to which a 2D leaf gets an octet.
-static constexpr int NEAR2D_SMALL = 4;
+// The mean leaf up to which 2D leaves may get octets: 300,000 particles of a
+// disk at 5.8 per leaf 0.077 ms with octets and 0.112 with warps, at 15 per
+// leaf (200,000) 0.112 and 0.105.
+static constexpr int SMALL2D_MEAN = 8;
+
+// Whether the leaves of a 2D near field get octets.  An octet is busy with its
+// leaf of m particles for a time that grows as m^2, so that a full leaf may
+// outlast all others: octets gained with leaves / m^2 = 33 (200,000 particles
+// in clumps, m = 56, 0.097 against 0.122 ms with warps), 159 and 340 (2M, m =
+// 57, 0.69 against 1.16) and lost at 21 (300,000, m = 84, 1.41 against 0.35),
+// 19 (20,000, m = 25, 0.112 against 0.034) and 14.  At least 32 m^2 leaves also
+// keep a warp's pair count within 32 bits.
+static bool near2d_octets(int64_t n, int64_t nleaves, int64_t largest) {
+  return n <= SMALL2D_MEAN * nleaves && 32 * largest * largest <= nleaves;
+}
 
 template <bool POT>
 __global__ void __launch_bounds__(256) k_p2p2d_small(P2PArgs a) {
@@ -2742,8 +2755,8 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     }
     k_far_output<3><<<cdiv(n, TPB), TPB, 0, st>>>(ws.far, t.d_perm, n, G, d_acc, d_pot, ws.dev_err);
     ws.launches += 3;
-  } else if (dim == 2 && n <= (int64_t)NEAR2D_SMALL * pa.nleaves && t.level_max[D] <= 4096) {
-    // (4M clumped disk, 1.6 particles per leaf: 2.05 -> 0.81 ms; a pair count fits 32 bits)
+  } else if (dim == 2 && near2d_octets(n, pa.nleaves, t.level_max[D])) {
+    // (4M clumped disk, 1.6 particles per leaf: 2.05 -> 0.81 ms)
     (want_pot ? k_p2p2d_small<true> : k_p2p2d_small<false>)<<<cdiv((int64_t)pa.nleaves * 8, TPB), TPB, 0, st>>>(pa);
   } else if (dim == 3) {
     if (want_pot) k_p2p<3, true><<<pgrid, TPB, 0, st>>>(pa);

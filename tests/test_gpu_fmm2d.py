@@ -112,3 +112,40 @@ def test_c3_full_size_error_vs_direct():
     ref = d_ref.cpu().numpy()
     assert st["m2l_tiles"] > 0  # the tensor-core M2L ran
     assert rel_l2(a, ref) < 1e-6
+
+
+def _clump_in_disk(n, k, sigma, seed):
+    """k of n particles in a clump, the others uniform in the unit disk."""
+    pos = workloads.uniform_disk_2d(n, seed=seed)[0]
+    pos[:k] = np.array([0.21, 0.13]) + sigma * np.random.default_rng(seed).normal(size=(k, 2))
+    return pos, np.full(n, 1.0 / n)
+
+
+# means of about 2 and of 8 and more particles per leaf; the fullest leaf against the number of leaves on either side
+# of 32 m^2; leaves of more than 16 x 16 targets
+@pytest.mark.parametrize("n,k,sigma,T", [(3000, 0, 1.0, 4), (3000, 0, 1.0, 16), (3000, 0, 1.0, 64), (20000, 0, 1.0, 16),
+                                         (6000, 3000, 1e-3, 8), (6000, 3000, 1e-3, 64), (6000, 3000, 1e-3, 400)])
+def test_near_field_with_small_and_full_leaves(oracle, n, k, sigma, T):
+    pos, m = _clump_in_disk(n, k, sigma, 5)
+    with fmmgpu.Context(dim=2, p=12, leaf_cap=T, direct_max=20) as c:
+        a, ph = c.evaluate(pos, m, want_pot=True)
+        b = c.evaluate(pos, m)
+    g, po = oracle.fmm(pos, m, 12, T, want_pot=True, direct_max=20)
+    assert rel_l2(a, g) < 1e-6
+    assert rel_l2(a[k:], g[k:]) < 1e-6
+    assert rel_l2(ph, po) < 1e-6
+    assert rel_l2(b, g) < 1e-6
+
+
+def test_full_leaves_do_not_outlast_the_near_field():
+    """A clump whose leaves are full among leaves of one or two particles: a
+    near-field pair takes no longer than 5e-11 s after 0.3 ms (with octets on
+    leaves of up to 700 particles it was 13 ms for 2e7 pairs)."""
+    pos, m = _clump_in_disk(20000, 10000, 1e-3, 6)
+    with fmmgpu.Context(dim=2, p=10, leaf_cap=700) as c:
+        ms = []
+        for _ in range(4):
+            c.evaluate(pos, m)
+            st = c.stats()
+            ms.append(st["ms_p2p"] - st["ms_far_direct"])
+    assert min(ms) < 0.3 + (st["p2p_pairs"] - st["far_direct_pairs"]) * 5e-8
