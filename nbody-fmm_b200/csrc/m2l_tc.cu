@@ -136,7 +136,7 @@ __device__ inline void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
 }
 
-// One lane of a converged warp.
+// One lane of a converged warp, the same one each time.
 __device__ inline bool elect_one() {
   uint32_t p;
   asm volatile(
@@ -388,47 +388,48 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
           mma_bf16(tmem, ad + (uint32_t)(ks * 2 * (int)LBO_A >> 4), bd + (uint32_t)(ks * 2 * (int)LBO_B >> 4), idesc,
                    first && ks == 0 ? 0u : 1u);
     };
+    // The products of one slot of width w; false, with nothing more issued, as
+    // soon as a wait for a copy gives up.
+    auto issue = [&](int w) -> bool {
+      const int np = (w + KH - 1) / KH;
+      const uint32_t idesc =
+          (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(w >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+#pragma unroll
+      for (int s = 2; s >= 0; --s)
+        for (int h = 0; h < np; ++h, ++g) {
+          if (!mbar_wait(&s_full[g % TC_NBUF], (g / TC_NBUF) & 1)) return false;
+          const int nk = min(w - h * KH, KH) / 16;
+          if (s == 2) {
+            mma_steps(0, h, g, nk, idesc, h == 0);
+            mma_commit(&s_mma[g % TC_NBUF]);
+          } else if (s == 1) {
+            mma_steps(1, h, g, nk, idesc, false);
+            mma_steps(0, h, g, nk, idesc, false);
+            mma_commit(&s_mma[g % TC_NBUF]);
+          } else {
+            mma_steps(2, h, g, nk, idesc, false);
+            mma_steps(1, h, g, nk, idesc, false);
+            if (h == np - 1) {  // the largest product (x1 y1) last, over all parts (np <= TC_NBUF: all resident)
+              for (int q = 0; q < np; ++q) {
+                const uint32_t gq = g - (uint32_t)(np - 1 - q);
+                mma_steps(0, q, gq, min(w - q * KH, KH) / 16, idesc, false);
+                mma_commit(&s_mma[gq % TC_NBUF]);
+              }
+              mma_commit(&s_done);
+            }
+          }
+        }
+      return true;
+    };
     const bool lead = elect_one();
     while (true) {
       const int n = s_n[c];
       // one thread waits and issues, without a warp-wide step in between
       for (int j = 0; lead && j < n && ok; ++j) {
-        if (!mbar_wait(&s_a, (sidx + (uint32_t)j) & 1)) {
-          ok = false;
-          break;
-        }
+        ok = mbar_wait(&s_a, (sidx + (uint32_t)j) & 1);
+        if (!ok) break;
         tc_fence_after();
-        const int w = s_w[c][j], np = (w + KH - 1) / KH;
-        const uint32_t idesc =
-            (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(w >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
-#pragma unroll
-        for (int s = 2; s >= 0; --s)
-          for (int h = 0; h < np && ok; ++h, ++g) {
-            if (!mbar_wait(&s_full[g % TC_NBUF], (g / TC_NBUF) & 1)) {
-              ok = false;
-              break;
-            }
-            const int nk = min(w - h * KH, KH) / 16;
-            if (s == 2) {
-              mma_steps(0, h, g, nk, idesc, h == 0);
-              mma_commit(&s_mma[g % TC_NBUF]);
-            } else if (s == 1) {
-              mma_steps(1, h, g, nk, idesc, false);
-              mma_steps(0, h, g, nk, idesc, false);
-              mma_commit(&s_mma[g % TC_NBUF]);
-            } else {
-              mma_steps(2, h, g, nk, idesc, false);
-              mma_steps(1, h, g, nk, idesc, false);
-              if (h == np - 1) {  // the largest product (x1 y1) last, over all parts (np <= TC_NBUF: all resident)
-                for (int q = 0; q < np; ++q) {
-                  const uint32_t gq = g - (uint32_t)(np - 1 - q);
-                  mma_steps(0, q, gq, min(w - q * KH, KH) / 16, idesc, false);
-                  mma_commit(&s_mma[gq % TC_NBUF]);
-                }
-                mma_commit(&s_done);
-              }
-            }
-          }
+        ok = issue(s_w[c][j]);
       }
       __syncwarp();
       sidx += (uint32_t)n;
@@ -436,12 +437,6 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
       ok = __syncthreads_and(ok);
       if (!ok) {
         if (!mine) atomicOr(a.err, FMM_DEV_ERR_TIMEOUT);
-        // what was issued may still be writing D, in columns that are freed below
-        if (lead) {
-          mma_commit(&s_drain);
-          mbar_wait(&s_drain, 0);
-        }
-        __syncwarp();
         break;
       }
       if (s_n[c ^ 1] == 0) break;
@@ -603,6 +598,16 @@ __global__ void __launch_bounds__(TC_THREADS, tc_per_sm(P16)) k_tc_translate(TcA
 
   tc_fence_before();
   __syncthreads();
+  // After a wait that gave up, what was issued may still be writing D: it is
+  // waited for before the columns are freed (by the same elected thread; here
+  // and not where the issuing warp leaves its loop, which cost the M2L 2 %).
+  if (warp == 8 && !ok) {
+    if (elect_one()) {
+      mma_commit(&s_drain);
+      mbar_wait(&s_drain, 0);
+    }
+    __syncwarp();
+  }
   if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS));
 }
 
