@@ -1543,6 +1543,16 @@ __global__ void __launch_bounds__(256, SPLIT ? 3 : DIM == 3 ? 4 : 6) k_direct_fa
 // lane takes every eighth of them for up to four targets in registers.
 static constexpr long long FAR2D_MAX = 256;
 
+// Whether a 2D far field takes octets: with leaves of few particles in the
+// mean (in larger ones hardly a pair is kept: 23 per leaf 0.030 ms with octets
+// and 0.017 with warps), and enough cells, since an octet is busy four times as
+// long as a warp with the up to 27 direct_max pairs of a cell (direct_max 256:
+// 69,000 cells 0.122 and 0.214 ms, 3,500 cells 0.042 and 0.019; direct_max 17:
+// 14,000 cells 0.021 and 0.034, 2,600 cells 0.017 and 0.011).
+static bool far2d_octets(int64_t n, int64_t nleaves, int64_t ncells, int64_t direct_max) {
+  return direct_max <= FAR2D_MAX && n <= SMALL2D_MEAN * nleaves && ncells >= 256 * direct_max;
+}
+
 template <int R, bool POT>
 __device__ __forceinline__ void far2d_targets(const DirectArgs &a, const float4 *off, int tb, int nt, int t0,
                                               const float4 *s_cell, const int *s_pref, int total, int sub) {
@@ -2697,8 +2707,8 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
     else
       kern = want_pot ? pick(k_direct_far<2, true, false, false>, k_direct_far<2, true, false, true>)
                       : pick(k_direct_far<2, false, false, false>, k_direct_far<2, false, false, true>);
-    // small thresholds in 2D: eight lanes per cell (4M clumped disk, threshold 43: 6.9 -> 2.8 ms)
-    const bool octets = dim == 2 && !any_fdirect && direct_max <= FAR2D_MAX;
+    // (4M clumped disk, threshold 43: 6.9 -> 2.8 ms)
+    const bool octets = dim == 2 && !any_fdirect && far2d_octets(n, t.level_count[D], nw, direct_max);
     if (octets) (want_pot ? k_direct_far2d<true> : k_direct_far2d<false>)<<<cdiv(nw * 8, TPB), TPB, 0, st>>>(da);
     else if (grid > 0) kern<<<(unsigned)grid, TPB, 0, st>>>(da);
     ws.launches += 1;

@@ -137,6 +137,19 @@ def test_near_field_with_small_and_full_leaves(oracle, n, k, sigma, T):
     assert rel_l2(b, g) < 1e-6
 
 
+# the far field by warps and by octets: thresholds up to and above 256, few and many cells for the threshold, small and
+# larger leaves
+@pytest.mark.parametrize("n,T,dm", [(800, 4, 8), (6000, 4, 8), (6000, 4, 17), (6000, 4, 64), (20000, 4, 256),
+                                    (20000, 4, 257), (50000, 4, 256), (20000, 64, 40)])
+def test_far_field_thresholds(oracle, n, T, dm):
+    pos, m = _clump_in_disk(n, n // 4, 2e-2, 7)
+    with fmmgpu.Context(dim=2, p=10, leaf_cap=T, direct_max=dm, m2l_mode=fmmgpu.FMM_M2L_TC) as c:
+        a, ph = c.evaluate(pos, m, want_pot=True)
+    g, po = oracle.fmm(pos, m, 10, T, want_pot=True, direct_max=dm)
+    assert rel_l2(a, g) < 1e-6
+    assert rel_l2(ph, po) < 1e-6
+
+
 def test_full_leaves_do_not_outlast_the_near_field():
     """A clump whose leaves are full among leaves of one or two particles: a
     near-field pair takes no longer than 5e-11 s after 0.3 ms (with octets on
