@@ -853,6 +853,22 @@ __global__ void __launch_bounds__(256, 4) k_p2p(P2PArgs a) {
     atomicAdd(a.pair_count, (unsigned long long)((long long)(le - lb) * (total - 1)));
 }
 
+// Whether k_p2p's leaves are split over several warps of 16 targets: where the
+// fullest leaf holds more than 32 particles, m, and m^2 is above twice the
+// pairs of the mean leaf, (n / leaves)^2, times the leaves that one of the 4736
+// warps at a time goes through.  Measured m^2 over that, without and with the
+// split: 2.6 (300,000 uniform, 73 per leaf) 1.27 and 1.04 ms, 22 (20,000, 39
+// per leaf) 0.19 and 0.09, 315 (a sphere of 300,000 with up to 300 per leaf)
+// 4.05 and 1.00; 0.6 (2^20 uniform, 30 per leaf) 1.36 and 1.55, 1.4 (a 2D disk,
+// 23 per leaf) 0.14 and 0.17.  A split leaf's other warps exist for every leaf
+// and are mostly empty, so only up to 65,536 leaves (300,000 of up to 300 per
+// leaf 2.16 and 2.35 ms, 570,000 of up to 128 1.20 and 2.11).
+static bool near_split(int64_t n, int64_t nleaves, int64_t largest) {
+  const double mean = (double)n / (double)nleaves;
+  return nleaves <= 65536 && largest > 32 &&
+         (double)largest * (double)largest > 2.0 * mean * mean * (double)nleaves / 4736.0;
+}
+
 // The 2D near field of small leaves: eight lanes per leaf, each with every
 // eighth source for up to four targets in registers.  A leaf of one or two
 // particles has about 15 sources, half of which a warp's lanes have nothing
@@ -2741,11 +2757,11 @@ int run_fmm_passes(Workspace &ws, TreeState &t, OpTables &ops, ExpBuffers &eb, c
   pa.pot = d_pot;
   pa.err = ws.dev_err;
   pa.pair_count = ws.counters + 1;
-  // one warp per leaf, or in systems of few leaves (where a full leaf's warp
-  // outlasts the kernel) one per 16 targets
+  // one warp per leaf, or where the fullest leaf's warp outlasts the kernel one
+  // per 16 targets
   pa.parts = 1;
   pa.chunk = t.level_max[D];
-  if (pa.nleaves <= 65536 && t.level_max[D] > 32) {
+  if (near_split(n, pa.nleaves, t.level_max[D])) {
     pa.chunk = 16;
     pa.parts = std::min(cdiv(t.level_max[D], pa.chunk), 16);
   }

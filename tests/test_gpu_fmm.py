@@ -321,3 +321,34 @@ def test_m2l_batch_without_sources(oracle, p):
     with fmmgpu.Context(dim=3, p=p, leaf_cap=64, direct_max=262) as c:
         acc = c.evaluate(pos, mass)
     assert rel_l2(acc, oracle.fmm(pos, mass, p, 64, direct_max=262)) < 1e-6
+
+
+# leaves split over warps of 16 targets (more than 32 particles in the fullest, few leaves), the warps of the first 256
+# targets taking more than one turn, and leaves of up to 32 by one warp each
+@pytest.mark.parametrize("n,k,T", [(3000, 1500, 400), (3000, 2000, 100), (3000, 2000, 24), (3000, 0, 300), (600, 0, 600)])
+def test_near_field_of_full_leaves(oracle, n, k, T):
+    pos, m = workloads.uniform_cube(n, seed=9)
+    pos[:k] = np.array([0.31, 0.42, 0.17]) + 1e-3 * np.random.default_rng(9).normal(size=(k, 3))
+    with fmmgpu.Context(dim=3, p=6, leaf_cap=T, direct_max=20) as c:
+        acc, pot = c.evaluate(pos, m, want_pot=True)
+        plain = c.evaluate(pos, m)
+    want, want_pot = oracle.fmm(pos, m, 6, T, direct_max=20, want_pot=True)
+    assert rel_l2(acc, want) < 1e-6
+    assert rel_l2(plain, want) < 1e-6
+    assert rel_l2(pot, want_pot) < 1e-6
+
+
+@pytest.mark.parametrize("n", [100000, 140000])
+def test_near_field_around_65536_leaves(oracle, n):
+    """Half of the particles in a clump whose leaves hold up to 57 and 81,
+    below and above the number of leaves up to which full leaves are split:
+    the clump's forces against the FP64 direct sum at sampled targets (their
+    p = 8 truncation is below 2e-5)."""
+    pos, m = workloads.uniform_cube(n, seed=10)
+    pos[: n // 2] = 0.37 + 1e-3 * np.random.default_rng(10).normal(size=(n // 2, 3))
+    with fmmgpu.Context(dim=3, p=8, leaf_cap=100, m2l_mode=fmmgpu.FMM_M2L_TC) as c:
+        acc = c.evaluate(pos, m)
+        leaves = c.stats()["n_leaves"]
+    assert (leaves > 65536) == (n > 130000)
+    some = np.arange(0, n // 2, n // 400)
+    assert rel_l2(acc[some], oracle.direct(pos, m, targets=some)) < 1e-4
