@@ -705,6 +705,14 @@ def run_reference(args, world, rank):
         return
     import multiprocessing as mp
 
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle
+
+    if not os.path.exists(oracle.REF_SO):
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "oracle/_ref/libref.so is not built (make -C oracle ref, where the "
+                                         "reference's sources are)"}), flush=True)
+        return
     cores = os.cpu_count() or 1
     ctx = mp.get_context("spawn")
     n, p, leaf = REF_SAMPLE_N, args.p, args.leaf

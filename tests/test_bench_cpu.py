@@ -36,3 +36,20 @@ def test_reference_arm_prints_one_contract_line(workload):
     assert ("2D" in line["config"]["workload"]) == (workload == "disk2d")
     # the reference's own force error on its sample is stated beside its speed
     assert cb["reference_force_rel_l2"] > 0
+
+
+def test_reference_arm_says_that_it_is_unavailable(monkeypatch, capsys, tmp_path):
+    """Where the reference is not built the arm prints one line that says so
+    and ends normally."""
+    sys.path.insert(0, ROOT)
+    import bench
+    import oracle
+
+    monkeypatch.setattr(oracle, "REF_SO", str(tmp_path / "libref.so"))
+    for rank, lines in ((0, 1), (1, 0)):
+        bench.run_reference(None, 2, rank)
+        out = capsys.readouterr().out.splitlines()
+        assert len(out) == lines
+    bench.run_reference(None, 1, 0)
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and "not built" in line["unavailable"] and set(line) == {"impl", "unavailable"}
