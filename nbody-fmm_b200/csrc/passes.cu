@@ -1564,7 +1564,9 @@ static constexpr long long FAR2D_MAX = 256;
 // and 0.017 with warps), and enough cells, since an octet is busy four times as
 // long as a warp with the up to 27 direct_max pairs of a cell (direct_max 256:
 // 69,000 cells 0.122 and 0.214 ms, 3,500 cells 0.042 and 0.019; direct_max 17:
-// 14,000 cells 0.021 and 0.034, 2,600 cells 0.017 and 0.011).
+// 14,000 cells 0.021 and 0.034, 2,600 cells 0.017 and 0.011).  Thresholds above
+// FAR2D_MAX, which nothing sets by itself in 2D, stay with the warps: octets
+// still gain a little at 512, lose at 1024 with full leaves and at 4096.
 static bool far2d_octets(int64_t n, int64_t nleaves, int64_t ncells, int64_t direct_max) {
   return direct_max <= FAR2D_MAX && n <= SMALL2D_MEAN * nleaves && ncells >= 256 * direct_max;
 }
