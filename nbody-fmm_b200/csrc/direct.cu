@@ -47,48 +47,42 @@ __device__ __forceinline__ void direct_pair(double r2, double w, double eps2, do
   }
 }
 
-// A thread sums R targets (DS_THREADS apart) over the block's share of the
-// sources, staged DS_THREADS at a time: four pairs of one target unrolled, or
-// two pairs of two targets, so that independent chains fill the FP64 pipe's
-// latency.  The test for j == i runs only in the stages that hold one of the
-// warp's own targets; a warp without targets only stages.
-template <int DIM, int SOFT, bool POT, int R>
+// A thread sums one target over the block's share of the sources, staged
+// DS_THREADS at a time, four pairs unrolled to fill the FP64 pipe's latency.
+// (Two targets per thread, two pairs unrolled: all pairs of 20,011 particles
+// 0.70 against 0.60 ms with NaiveUpdate's softening and 0.62 against 0.56 with
+// Plummer's, 4096 targets of 2^20 6.4 against 6.0 ms, and idle threads in every
+// call whose targets are no multiple of 512: 256 of 2^20 0.74 against 0.40.)
+// The test for j == i runs only in the stages that hold one of the warp's own
+// targets; a warp without targets only stages.
+template <int DIM, int SOFT, bool POT>
 __global__ void __launch_bounds__(DS_THREADS) k_direct(const double *pos, const double *mass, int64_t n,
                                                        const int64_t *targets, int64_t nt, double eps2, int64_t chunk,
                                                        double G, double *acc, double *pot) {
   __shared__ double4 sp[DS_THREADS];
-  double x[R][3], a[R][3], ph[R];
-  int64_t me[R];
+  const int64_t ti = (int64_t)blockIdx.x * DS_THREADS + threadIdx.x;
+  const int64_t me = ti < nt ? (targets ? targets[ti] : ti) : -1;
+  double x[3], a[3], ph = 0.0;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t ti = (int64_t)blockIdx.x * (R * DS_THREADS) + r * DS_THREADS + threadIdx.x;
-    me[r] = ti < nt ? (targets ? targets[ti] : ti) : -1;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      x[r][k] = me[r] >= 0 && k < DIM ? pos[me[r] * DIM + k] : 0.0;
-      a[r][k] = 0.0;
-    }
-    ph[r] = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    x[k] = me >= 0 && k < DIM ? pos[me * DIM + k] : 0.0;
+    a[k] = 0.0;
   }
-  const bool busy = __any_sync(0xffffffffu, me[0] >= 0);  // (no second target without a first)
+  const bool busy = __any_sync(0xffffffffu, me >= 0);
   const int64_t j0 = (int64_t)blockIdx.y * chunk, j1 = min(n, j0 + chunk);
-  constexpr int U = 4 / R;
   auto sum = [&](int cnt, int64_t jb, bool own) {
-#pragma unroll U
+#pragma unroll 4
     for (int k = 0; k < cnt; ++k) {
       const double4 q = sp[k];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (own && jb + k == me[r]) continue;
-        const double dx = x[r][0] - q.x, dy = x[r][1] - q.y, dz = DIM == 3 ? x[r][2] - q.z : 0.0;
-        const double r2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
-        double f, pw = 0.0;
-        direct_pair<DIM, SOFT, POT>(r2, q.w, eps2, f, pw);
-        a[r][0] -= f * dx;
-        a[r][1] -= f * dy;
-        if (DIM == 3) a[r][2] -= f * dz;
-        if (POT) ph[r] += pw;
-      }
+      if (own && jb + k == me) continue;
+      const double dx = x[0] - q.x, dy = x[1] - q.y, dz = DIM == 3 ? x[2] - q.z : 0.0;
+      const double r2 = DIM == 3 ? dx * dx + dy * dy + dz * dz : dx * dx + dy * dy;
+      double f, pw = 0.0;
+      direct_pair<DIM, SOFT, POT>(r2, q.w, eps2, f, pw);
+      a[0] -= f * dx;
+      a[1] -= f * dy;
+      if (DIM == 3) a[2] -= f * dz;
+      if (POT) ph += pw;
     }
   };
   for (int64_t jb = j0; jb < j1; jb += DS_THREADS) {
@@ -97,47 +91,29 @@ __global__ void __launch_bounds__(DS_THREADS) k_direct(const double *pos, const 
       sp[threadIdx.x] = make_double4(pos[j * DIM], pos[j * DIM + 1], DIM == 3 ? pos[j * DIM + 2] : 0.0, mass[j]);
     __syncthreads();
     const int cnt = (int)min((int64_t)DS_THREADS, j1 - jb);
-    bool mine = false;
-#pragma unroll
-    for (int r = 0; r < R; ++r) mine |= me[r] >= jb && me[r] < jb + DS_THREADS;
-    if (__any_sync(0xffffffffu, mine)) sum(cnt, jb, true);
-    else if (R == 2 || busy) sum(cnt, jb, false);
+    if (__any_sync(0xffffffffu, me >= jb && me < jb + DS_THREADS)) sum(cnt, jb, true);
+    else if (busy) sum(cnt, jb, false);
     __syncthreads();
   }
+  if (ti >= nt) return;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int64_t ti = (int64_t)blockIdx.x * (R * DS_THREADS) + r * DS_THREADS + threadIdx.x;
-    if (ti >= nt) continue;
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) {
-      if (gridDim.y == 1) acc[ti * DIM + k] = G * a[r][k];
-      else atomicAdd(&acc[ti * DIM + k], G * a[r][k]);
-    }
-    if (POT) {
-      if (gridDim.y == 1) pot[ti] = G * ph[r];
-      else atomicAdd(&pot[ti], G * ph[r]);
-    }
+  for (int k = 0; k < DIM; ++k) {
+    if (gridDim.y == 1) acc[ti * DIM + k] = G * a[k];
+    else atomicAdd(&acc[ti * DIM + k], G * a[k]);
+  }
+  if (POT) {
+    if (gridDim.y == 1) pot[ti] = G * ph;
+    else atomicAdd(&pot[ti], G * ph);
   }
 }
 
 int direct_sum(const double *d_pos, const double *d_mass, int64_t n, const int64_t *d_targets, int64_t nt, int dim,
                double eps2, int soft_mode, double G, double *d_acc, double *d_pot, cudaStream_t st, int64_t &launches) {
   if (nt <= 0 || n <= 0) return FMM_OK;
-  // Two targets per thread where blocks of 512 targets fill the chip even so,
-  // that is from 800 of them with shares of two stages (10,000 targets of
-  // 2^20: 16.3 ms with one, 15.0 with two), and the last of few blocks is not
-  // much emptier than the others (768 targets: 1.22 against 1.45 ms); else one
-  // (256 targets of 2^20 0.40 against 0.74 ms, all pairs of 2000 0.09 against
-  // 0.14).
-  // NaiveUpdate's 3D form has enough to do per pair with one, four unrolled:
-  // all pairs of 100,000 14.7 ms against 16.1 with two.
-  const int64_t bx2 = (nt + 2 * DS_THREADS - 1) / (2 * DS_THREADS), last = nt - (bx2 - 1) * 2 * DS_THREADS;
-  const int64_t shares = (n + 2 * DS_THREADS - 1) / (2 * DS_THREADS);
-  const bool naive = soft_mode == FMM_SOFT_NAIVE_REF;
-  const bool two = !(naive && dim == 3) && bx2 * shares >= 800 && (bx2 >= 8 || last > 384);
-  const int64_t bx = two ? bx2 : (nt + DS_THREADS - 1) / DS_THREADS;
-  // source shares for about eight blocks per SM (three run at a time), of at least two stages
-  const int64_t by = std::max<int64_t>(1, std::min<int64_t>({(148 * 8 + bx - 1) / bx, shares, 65535}));
+  const int64_t bx = (nt + DS_THREADS - 1) / DS_THREADS;
+  // source shares for about 16 blocks per SM, of at least two stages (shorter shares also round less)
+  const int64_t by = std::max<int64_t>(
+      1, std::min<int64_t>({(148 * 16 + bx - 1) / bx, (n + 2 * DS_THREADS - 1) / (2 * DS_THREADS), 65535}));
   const int64_t chunk = (n + by - 1) / by;
   if (by > 1) {
     cudaMemsetAsync(d_acc, 0, sizeof(double) * nt * dim, st);
@@ -147,18 +123,14 @@ int direct_sum(const double *d_pos, const double *d_mass, int64_t n, const int64
   auto run = [&](auto kern) {
     kern<<<grid, DS_THREADS, 0, st>>>(d_pos, d_mass, n, d_targets, nt, eps2, chunk, G, d_acc, d_pot);
   };
-  auto pick = [&](auto one, auto both) { run(two ? both : one); };
+  const bool naive = soft_mode == FMM_SOFT_NAIVE_REF;
   constexpr int P = FMM_SOFT_PLUMMER, N = FMM_SOFT_NAIVE_REF;
   if (dim == 3) {
-    if (naive) d_pot ? run(k_direct<3, N, true, 1>) : run(k_direct<3, N, false, 1>);
-    else if (d_pot) pick(k_direct<3, P, true, 1>, k_direct<3, P, true, 2>);
-    else pick(k_direct<3, P, false, 1>, k_direct<3, P, false, 2>);
-  } else if (naive) {
-    if (d_pot) pick(k_direct<2, N, true, 1>, k_direct<2, N, true, 2>);
-    else pick(k_direct<2, N, false, 1>, k_direct<2, N, false, 2>);
+    if (d_pot) naive ? run(k_direct<3, N, true>) : run(k_direct<3, P, true>);
+    else naive ? run(k_direct<3, N, false>) : run(k_direct<3, P, false>);
   } else {
-    if (d_pot) pick(k_direct<2, P, true, 1>, k_direct<2, P, true, 2>);
-    else pick(k_direct<2, P, false, 1>, k_direct<2, P, false, 2>);
+    if (d_pot) naive ? run(k_direct<2, N, true>) : run(k_direct<2, P, true>);
+    else naive ? run(k_direct<2, N, false>) : run(k_direct<2, P, false>);
   }
   launches += 1;
   return cudaGetLastError() == cudaSuccess ? FMM_OK : FMM_ERR_CUDA;

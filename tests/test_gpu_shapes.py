@@ -111,8 +111,8 @@ def test_direct_shapes(n, dim, scale, soft):
     assert rel_l2(every[targets], a) < 1e-12
 
 
-# one or two targets per thread: around 256 and 512 targets, idle warps, blocks of 512 targets before and after there
-# are 800 (every target checked where there are few, else the ends of the blocks)
+# blocks of 256 targets, full, with idle warps and with idle threads, over one and many shares of the sources (every
+# target checked where there are few, else the ends of the blocks)
 @pytest.mark.parametrize("n,nt,dim", [(3000, 1, 3), (3000, 33, 3), (3000, 256, 3), (3000, 257, 3), (450000, 385, 3),
                                       (450000, 384, 3), (120000, 1920, 2), (14000, 14000, 3), (15000, 15000, 3)])
 @pytest.mark.parametrize("soft", [fmmgpu.FMM_SOFT_PLUMMER, fmmgpu.FMM_SOFT_NAIVE_REF])
